@@ -198,11 +198,14 @@ typedef struct vkg_gemm_args {
   int32_t split_k;           /* K cut into slices: each slice's partial tile goes to
                                 `workspace` and a second kernel adds the slices in order
                                 (deterministic).  Plain fp32 epilogue, unbatched only.
-                                0 = library decides (splits only if a workspace is given),
                                 1 = never, n > 1 = exactly n slices.
-                                -1: as many slices as a rule of M, N, K alone says, whatever
-                                tiles are chosen: the order a sum is taken in then stays the
-                                same when the library's time model changes. */
+                                0 = as many as a rule of M, N, K and of what this block asks
+                                for itself (tile_n, cta_pair, max_ctas) says, so that the order
+                                a sum is taken in depends on nothing else: not on the tiles
+                                that are chosen, the SM limit or the size of the workspace, as
+                                long as that holds vkg_gemm_workspace_bytes (with less, as many
+                                slices as fit; without one, 1).
+                                -1 = the same rule as if tile_n, cta_pair and max_ctas were 0. */
   void* workspace;           /* scratch for the slices: slices * M * N floats */
   int64_t workspace_bytes;
   int32_t causal;            /* attention shortcuts for square (T x T) causal operands:
@@ -226,6 +229,9 @@ typedef struct vkg_gemm_args {
 } vkg_gemm_args;
 
 int64_t vkg_gemm_colsum_scratch_floats(int M, int N);
+/* Bytes of workspace that the slices of this call need (`workspace` itself is not looked at); 0
+ * when K stays whole. */
+int64_t vkg_gemm_workspace_bytes(const vkg_gemm_args* args);
 
 /* Many independent plain GEMMs (fp32 output, unbatched, no epilogue extras) in ONE launch: the
  * dW = X^T dY of every Linear of a model (autograd.py:217-219, transformer.py:97-98), which

@@ -2,6 +2,7 @@
 the unique-id rendezvous between two processes, and a world-size-2 data-parallel step
 over gloo checked against the single-process oracle."""
 
+import ctypes as C
 import multiprocessing as mp
 import os
 import socket
@@ -235,3 +236,56 @@ def test_host_wait_reports_an_asynchronous_communicator_error_before_the_deadlin
     rc, aborted, msg = _wait_selftest(-1, 3, 30.0)
     assert rc != 0 and aborted == 1 and "asynchronous error" in msg
     assert time.perf_counter() - t0 < 5.0
+
+
+def _slices(M, N, K):
+    """The rule of M, N and K by which a GEMM's K is cut, restated: the cheapest of up to 8 slices
+    (16 where the partial sums fit 1 MB), of waves of tiles on 148 SMs plus the reduction."""
+    up = lambda a, b: -(-a // b)
+    kbs, out = up(K, 64), 4 * M * N
+    most = min(max((1 << 20) // out, 8), 16)
+
+    def best(bm, slots, widths):
+        times = []
+        for bn in widths:
+            kb_us = {256: 0.41, 192: 0.36}.get(bn, 0.33)
+            for sp in range(1, most + 1):
+                if sp == 1 or kbs // sp >= 4:
+                    waves = up(up(M, bm) * up(N, bn) * sp, slots)
+                    times.append((waves * (up(kbs, sp) * kb_us + 4.4 * bn / 256)
+                                  + ((sp + 1) * out / 4e6 + 4.0 if sp > 1 else 0.0), len(times), sp))
+        return min(times)[2]
+    if M > 128 and N >= 128:
+        pairs = best(256, 74, [256])
+        if pairs > 1 or 10 * up(M, 256) * up(N, 256) >= 60 * 74:
+            return pairs
+        if N % 192 == 0 and N <= 768 and K >= 1536 and up(M, 256) * (N // 192) >= 74:
+            return best(256, 74, [192])
+    return best(128, 148, [bn for bn in (256, 192, 128, 64) if bn <= up(N, 64) * 64 or bn == 64])
+
+
+def test_slices_of_k_follow_the_shape_alone():
+    """The order a sum is taken in is a rule of M, N and K: not of the workspace at hand, nor of
+    anything a device is set to (there is none here).  What a caller insists on is taken."""
+    import random
+    from vkgrad_b200 import _lib
+    lib, rng, cut = _lib.load(), random.Random(5), 0
+    shapes = [(416, 496, 6976), (512, 512, 1800), (256, 768, 50304), (64, 64, 16384), (768, 768, 8192),
+              (1024, 4096, 16384), (8, 8, 8), (128, 128, 512)]
+    shapes += [(rng.randint(1, 4096), 8 * rng.randint(1, 512), int(2 ** rng.uniform(3, 15))) for _ in range(300)]
+    for M, N, K in shapes:
+        a = _lib.GemmArgs(M=M, N=N, K=K, ldc=N, C=1 << 20, c_dtype=_lib.F32, nb0=1, nb1=1)
+        got = []
+        for split, ws in ((0, 0), (0, 1 << 40), (-1, 0), (-1, 4 * M * N)):
+            a.split_k, a.workspace, a.workspace_bytes = split, 1 << 21 if ws else None, ws
+            got.append(lib.vkg_gemm_workspace_bytes(C.byref(a)))
+        want = _slices(M, N, K)
+        assert got == [4 * M * N * want if want > 1 else 0] * 4, (M, N, K)
+        cut += want > 1
+        a.split_k = 1
+        assert lib.vkg_gemm_workspace_bytes(C.byref(a)) == 0
+        a.split_k = 3
+        assert lib.vkg_gemm_workspace_bytes(C.byref(a)) == 12 * M * N
+        a.bias = 1 << 20           # an epilogue: K stays whole
+        assert lib.vkg_gemm_workspace_bytes(C.byref(a)) == 0
+    assert 30 < cut < len(shapes) - 30

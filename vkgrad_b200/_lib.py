@@ -90,6 +90,7 @@ _SIGNATURES = {
     "vkg_gemm": (i32, [vp, C.POINTER(GemmArgs)]),
     "vkg_gemm_run": (i32, [vp, C.POINTER(GemmArgs), i32, C.POINTER(C.c_double)]),
     "vkg_gemm_colsum_scratch_floats": (i64, [i32, i32]),
+    "vkg_gemm_workspace_bytes": (i64, [C.POINTER(GemmArgs)]),
     "vkg_selftest_wait_timeout": (i32, [vp, i64]),
     "vkg_gemm_group_table_bytes": (i64, [i32]),
     "vkg_gemm_group_prepare": (i32, [vp, C.POINTER(GemmArgs), i32, vp, i32, C.POINTER(i32)]),

@@ -1238,12 +1238,10 @@ int make_out_map(vkg_device* dev, CUtensorMap* map, const void* ptr, int dtype, 
 // ---- which tiles ---------------------------------------------------------------------------
 //
 // A launch is planned with a time model over its candidates: 128-row tiles of one CTA and 256-row
-// tiles of a CTA pair, 64 to 256 columns wide, K whole or in up to eight slices (few tiles and a
-// long K: the dW shapes).  Its constants were fitted to 208 shapes (M to 50272, N and K alike,
-// aligned and ragged, the three transpositions, every epilogue of a training step; launches in a
-// graph on B200, operands warm): the choice costs 0.3 % over the best candidate on average and 11 %
-// at worst, where the model before it (one k-block cost per width, measured before the issue loop
-// was rewritten; pairs from six waves on; slices whenever they looked even) cost 3.4 % and 56 %.
+// tiles of a CTA pair, 64 to 256 columns wide.  How many slices K is cut into is not the model's to
+// choose (k_slices): it is part of the result.  Its constants were fitted to 208 shapes (M to 50272,
+// N and K alike, aligned and ragged, the three transpositions, every epilogue of a training step;
+// launches in a graph on B200, operands warm).
 //
 // Per k-block (64 of K), microseconds by tile width 64 / 128 / 192 / 256.  A CTA pulls its operands
 // through an L2 port of 64 bytes a cycle; K-major operands go a little faster than MN-major ones.
@@ -1259,11 +1257,9 @@ constexpr double PL_PAIR = 1.29;       // a pair's barriers and its later start
 constexpr double PL_IDLE = 0.81;       // k-block cost with one CTA busy, of that with all
 constexpr double PL_WAVE = 0.95;       // per further wave
 constexpr double PL_OVERLAP = 1.42;    // epilogue beside a main loop, of the epilogue alone
-constexpr double PL_SLICE = 1.41, PL_SLICE_BYTES = 1.04e7;   // the reduction: launch, bytes per us
 constexpr double PL_RAGGED[2] = {0.387, 0.138};   // operand rows off the 128-byte lines: single, pair
 constexpr double PL_HOT[2] = {0.293, 0.064};      // the clock under sustained load: single, pair
 constexpr double PL_HOT_FLOPS = 3.5e10;
-constexpr double PL_SLICE_GAIN = 0.9;  // slices have to gain this much: they change the sum's order
 
 struct Tiles {
   bool pair;
@@ -1292,50 +1288,62 @@ double tiles_us(const vkg_gemm_args* a, bool pair, int bn, int split, int batch,
   const double epi = PL_EPI + (pair ? PL_PAIR : 0.0) + PL_EPI_COL * bn * (0.5 + 0.125 * out);
   const double main_loop = kbs * tk;
   const long long waves = (tiles + slots - 1) / slots;
-  double t = PL_LAUNCH + main_loop + epi +
-             (waves - 1) * (main_loop + PL_WAVE > epi * PL_OVERLAP ? main_loop + PL_WAVE : epi * PL_OVERLAP);
-  if (split > 1) t += PL_SLICE + (split + 1) * M * N * 4.0 / PL_SLICE_BYTES;
-  return t;
+  return PL_LAUNCH + main_loop + epi +
+         (waves - 1) * (main_loop + PL_WAVE > epi * PL_OVERLAP ? main_loop + PL_WAVE : epi * PL_OVERLAP);
 }
 
-// single / pair: whether such tiles may be used; force_bn, force_split: 0 = free.
-Tiles choose_tiles(vkg_device* dev, const vkg_gemm_args* a, bool single, bool pair, int force_bn, bool may_split,
-                   int force_split) {
+// single / pair: whether such tiles may be used; force_bn: 0 = free; split: slices of K.
+Tiles choose_tiles(vkg_device* dev, const vkg_gemm_args* a, bool single, bool pair, int force_bn, int split) {
   const int batch = (a->nb0 > 0 ? a->nb0 : 1) * (a->nb1 > 0 ? a->nb1 : 1);
-  const int num_kb = (a->K + BK - 1) / BK, n_round = ((a->N + 63) / 64) * 64;
+  const int n_round = ((a->N + 63) / 64) * 64;
   const int ctas = a->max_ctas > 0 ? a->max_ctas : vkg_persistent_ctas(dev);
-  Tiles best = {false, 64, 1, -1.0};
-  double whole = -1.0;          // best time with K whole
-  for (int sp = force_split > 0 ? force_split : 1; sp <= (force_split > 0 ? force_split : 8); ++sp) {
-    if (force_split == 0 && sp > 1 && (!may_split || num_kb / sp < 4)) continue;
-    if (sp > 1 && (int64_t)sp * a->M * a->N * 4 > a->workspace_bytes) continue;
-    for (int kind = 0; kind < 2; ++kind) {
-      if (kind ? !pair : !single) continue;
-      for (int bn = kind ? 192 : 64; bn <= 256; bn += 64) {
-        if (force_bn ? bn != force_bn : bn > n_round && bn != 64) continue;
-        if (kind && !force_bn && a->cta_pair <= 0 && bn == 192 && !dev->pair192) continue;
-        const int slots = kind ? ctas / 2 : ctas;
-        if (slots < 1) continue;
-        const double us = tiles_us(a, kind != 0, bn, sp, batch, slots);
-        if (kind && bn == 256 && sp == 1 && a->cta_pair <= 0 && dev->pair_min_waves_x10 > 0) {
-          const long long tiles = (long long)((a->M + 2 * BM - 1) / (2 * BM)) * ((a->N + bn - 1) / bn) * batch;
-          if (10 * tiles < (long long)dev->pair_min_waves_x10 * slots) continue;
-        }
-        if (best.us < 0 || us < best.us * (sp > 1 && best.split == 1 && whole > 0 ? PL_SLICE_GAIN : 1.0))
-          best = {kind != 0, bn, sp, us};
-        if (sp == 1 && (whole < 0 || us < whole)) whole = us;
+  Tiles best = {false, 64, split, -1.0};
+  for (int kind = 0; kind < 2; ++kind) {
+    if (kind ? !pair : !single) continue;
+    for (int bn = kind ? 192 : 64; bn <= 256; bn += 64) {
+      if (force_bn ? bn != force_bn : bn > n_round && bn != 64) continue;
+      if (kind && !force_bn && a->cta_pair <= 0 && bn == 192 && !dev->pair192) continue;
+      const int slots = kind ? ctas / 2 : ctas;
+      if (slots < 1) continue;
+      const double us = tiles_us(a, kind != 0, bn, split, batch, slots);
+      if (kind && bn == 256 && split == 1 && a->cta_pair <= 0 && dev->pair_min_waves_x10 > 0) {
+        const long long tiles = (long long)((a->M + 2 * BM - 1) / (2 * BM)) * ((a->N + bn - 1) / bn) * batch;
+        if (10 * tiles < (long long)dev->pair_min_waves_x10 * slots) continue;
       }
+      if (best.us < 0 || us < best.us) best = {kind != 0, bn, split, us};
     }
   }
   return best;
 }
 
-// Slices of K by a rule that does not follow the time model above (split_k = -1).  Slices change the
-// order of a sum by about 1e-5, and where that sum is a gradient on its way into fp16 without a loss
-// scale, subnormals make 3e-3 of it in the weight gradients below.  The rule: few 256-column pair
-// tiles, or few single ones, are cut while that shortens the waves by more than the reduction costs.
-int fixed_slices(vkg_device* dev, const vkg_gemm_args* a) {
+// Whether an output is one that slices of K can be added up into: fp32, not batched, nothing in the
+// epilogue.
+bool plain_output(const vkg_gemm_args* a) {
+  const int batch = (a->nb0 > 0 ? a->nb0 : 1) * (a->nb1 > 0 ? a->nb1 : 1);
+  return !a->bias && !a->pre && !a->act && !a->dact_z && !a->residual && !a->C2 && !a->colsum &&
+         a->c_dtype == VKG_F32 && (a->alpha == 0.0f || a->alpha == 1.0f) && batch == 1 && a->causal == 0 &&
+         a->N % 4 == 0 && a->ldc % 4 == 0 && ((uintptr_t)a->C & 15) == 0;
+}
+
+// Whether K may be cut into slices that a second launch adds up.
+bool may_split(const vkg_gemm_args* a) {
+  return plain_output(a) && a->workspace && ((uintptr_t)a->workspace & 15) == 0;
+}
+
+// Slices of K where the caller leaves them to the library: a rule of M, N, K and the tiles the caller
+// insists on.  Nothing else may enter it -- not the time model above, not how many SMs a launch is
+// held to, not how large a workspace happens to be: slices change the order of a sum, by 1e-6 of the
+// result, and a training step whose fp16 gradients are subnormals, for want of a loss scale, makes
+// 2e-3 of that in its second step (512-wide model, 1800 rows: the head's dW).  The rule: few
+// 256-column pair tiles, or few single ones, are cut while that shortens the waves of a full B200 by
+// more than the reduction costs, by the k-block and epilogue times of an early version of the kernel.
+// At most 8 slices, or 16 where the partial sums are small.
+constexpr int SLICE_SMS = 148;
+constexpr int64_t SLICE_SMALL_BYTES = 1 << 20;
+int k_slices(const vkg_gemm_args* a) {
   const int num_kb = (a->K + BK - 1) / BK, n_round = ((a->N + 63) / 64) * 64;
+  const int64_t out_bytes = (int64_t)a->M * a->N * 4, small = SLICE_SMALL_BYTES / out_bytes;
+  const int most = small < 8 ? 8 : small > 16 ? 16 : (int)small;
   const auto slices = [&](int bm, int slots, int only_bn) {
     double best = -1.0;
     int got = 1;
@@ -1343,11 +1351,11 @@ int fixed_slices(vkg_device* dev, const vkg_gemm_args* a) {
       if (only_bn ? bn != only_bn : bn > n_round && bn != 64) continue;
       const long long tiles = (long long)((a->M + bm - 1) / bm) * ((a->N + bn - 1) / bn);
       const double t_kb = bn == 256 ? 0.41 : bn == 192 ? 0.36 : 0.33;
-      for (int sp = 1; sp <= 16; ++sp) {
-        if (sp > 1 && (num_kb / sp < 4 || (int64_t)sp * a->M * a->N * 4 > a->workspace_bytes)) break;
+      for (int sp = 1; sp <= most; ++sp) {
+        if (sp > 1 && num_kb / sp < 4) break;
         const long long waves = (tiles * sp + slots - 1) / slots;
         double t = waves * ((num_kb + sp - 1) / sp * t_kb + 4.4 * bn / 256.0);
-        if (sp > 1) t += (double)(sp + 1) * a->M * a->N * 4.0 / 4.0e6 + 4.0;
+        if (sp > 1) t += (double)(sp + 1) * out_bytes / 4.0e6 + 4.0;
         if (best < 0 || t < best) {
           best = t;
           got = sp;
@@ -1356,16 +1364,18 @@ int fixed_slices(vkg_device* dev, const vkg_gemm_args* a) {
     }
     return got;
   };
-  const int ctas = vkg_persistent_ctas(dev);
-  if (a->M > BM && a->N >= PAIR_BN / 2) {
+  const bool any = a->split_k < 0;      // -1: as if the tiles were the library's to choose
+  const int tile_n = any ? 0 : a->tile_n, pair = any ? 0 : a->cta_pair;
+  if (pair >= 0 && a->M > BM && a->N >= PAIR_BN / 2 && (tile_n == 0 || tile_n == 192 || tile_n == PAIR_BN) &&
+      (any || a->max_ctas == 0)) {
     const long long rows = (a->M + 2 * BM - 1) / (2 * BM);
-    const int sp = slices(2 * BM, ctas / 2, 256);
-    if (sp > 1) return sp;
-    if (10 * rows * ((a->N + 255) / 256) >= 60ll * (ctas / 2)) return 1;
-    if (a->N % 192 == 0 && a->N <= 4 * 192 && a->K >= 1536 && rows * (a->N / 192) >= ctas / 2)
-      return slices(2 * BM, ctas / 2, 192);
+    const int slots = SLICE_SMS / 2;
+    if (pair > 0 || slices(2 * BM, slots, PAIR_BN) > 1 || 10 * rows * ((a->N + 255) / 256) >= 60ll * slots)
+      return slices(2 * BM, slots, tile_n == 192 ? 192 : PAIR_BN);
+    if (tile_n == 0 && a->N % 192 == 0 && a->N <= 4 * 192 && a->K >= 1536 && rows * (a->N / 192) >= slots)
+      return slices(2 * BM, slots, 192);
   }
-  return slices(BM, ctas, 0);
+  return slices(BM, SLICE_SMS, tile_n);
 }
 
 // One width for all problems of a grouped launch, from the same costs: waves of all their tiles
@@ -1407,15 +1417,6 @@ struct Problem {
   bool vec;
   long long total_tiles;
 };
-
-// Whether K may be cut into slices that a second launch adds up.
-bool may_split(const vkg_gemm_args* a) {
-  const int batch = (a->nb0 > 0 ? a->nb0 : 1) * (a->nb1 > 0 ? a->nb1 : 1);
-  const bool plain_f32 = !a->bias && !a->pre && !a->act && !a->dact_z && !a->residual && !a->C2 && !a->colsum &&
-                         a->c_dtype == VKG_F32 && (a->alpha == 0.0f || a->alpha == 1.0f);
-  return plain_f32 && batch == 1 && a->causal == 0 && a->workspace && a->N % 4 == 0 && a->ldc % 4 == 0 &&
-         (((uintptr_t)a->C | (uintptr_t)a->workspace) & 15) == 0;
-}
 
 // The arguments' own conditions, before anything is planned from them.
 int check_args(const vkg_gemm_args* a) {
@@ -1621,6 +1622,12 @@ extern "C" int64_t vkg_gemm_colsum_scratch_floats(int M, int N) {
   return (int64_t)4 * 2 * ((M + 2 * BM - 1) / (2 * BM)) * N;
 }
 
+extern "C" int64_t vkg_gemm_workspace_bytes(const vkg_gemm_args* a) {
+  if (!a || a->M <= 0 || a->N <= 0 || a->K <= 0 || !plain_output(a)) return 0;
+  const int split = a->split_k > 0 ? a->split_k : k_slices(a);
+  return split > 1 ? (int64_t)split * a->M * a->N * 4 : 0;
+}
+
 extern "C" int vkg_selftest_wait_timeout(vkg_device* dev, int64_t budget_cycles) {
   if (vkg_bind(dev)) return 1;
   VKG_REQUIRE(budget_cycles > 0 && budget_cycles <= 100000000ll,
@@ -1732,12 +1739,13 @@ int make_plan(vkg_device* dev, const vkg_gemm_args* a, GemmPlan* out) {
                        (a->tile_n == 0 || a->tile_n == PAIR_BN || a->tile_n == 192) && a->max_ctas == 0 &&
                        a->cta_pair >= 0;
   const bool pair_only = pair_ok && a->cta_pair > 0;
-  // a caller who asks for pairs compares bits with the other kernel: K is then cut only when asked
-  const Tiles t = choose_tiles(dev, a, !pair_only, pair_ok, pair_only && a->tile_n == 0 ? PAIR_BN : a->tile_n,
-                               may_split(a) && a->split_k != 1 && !pair_only,
-                               a->split_k >= 0 ? a->split_k : may_split(a) ? fixed_slices(dev, a) : 1);
-  VKG_REQUIRE(t.us >= 0, "gemm: split_k workspace too small (%lld bytes for %d slices of %d x %d)",
-              (long long)a->workspace_bytes, a->split_k, a->M, a->N);
+  // the rule's slices, or as many of them as the workspace holds
+  int split = a->split_k > 0 ? a->split_k : may_split(a) ? k_slices(a) : 1;
+  if (a->split_k <= 0)
+    while (split > 1 && (int64_t)split * a->M * a->N * 4 > a->workspace_bytes) --split;
+  const Tiles t = choose_tiles(dev, a, !pair_only, pair_ok, pair_only && a->tile_n == 0 ? PAIR_BN : a->tile_n, split);
+  VKG_REQUIRE(t.us >= 0, "gemm: no tile of %d columns for %d x %d x %d on %d CTAs", a->tile_n, a->M, a->N, a->K,
+              a->max_ctas);
   const bool use_pair = t.pair;
   if (build_problem(dev, a, &q, use_pair, t.bn, t.split)) return 1;
   if (use_pair) {

@@ -99,10 +99,11 @@ def _gemm_args(dev, a, b, c, m, n, k, trans_a=False, trans_b=False,
     plain = (bias is None and pre is None and dact_z is None and residual is None and c2 is None
              and act == ACT_NONE and c_dtype == F32 and alpha == 1.0)
     if split_k != 1 and plain and nb0 * nb1 == 1 and m * n * 4 <= SPLIT_K_MAX_TILE_BYTES:
-        # few output tiles, long K (the dW shapes): give the library room to split K
-        ws = dev.scratch((int(split_k) if split_k > 1 else 8) * m * n * 4)
-        args.workspace = ws.dptr
-        args.workspace_bytes = ws.size
+        # few output tiles, long K (the dW shapes): room for the slices of K the library cuts
+        need = dev.lib.vkg_gemm_workspace_bytes(C.byref(args))
+        if need:
+            ws = dev.scratch(need)
+            args.workspace, args.workspace_bytes = ws.dptr, ws.size
     return args
 
 

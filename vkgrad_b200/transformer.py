@@ -185,7 +185,7 @@ class Dense:
                     self._colsum_scratch = c.buf(dev.lib.vkg_gemm_colsum_scratch_floats(R, I) * 4)
                 cs = self._colsum_scratch
             gemm(dev, dy16, self.W.w16, dx, R, I, O, trans_b=True, graph=graph, c_dtype=dx_dtype,
-                 split_k=-1, dact_z=dact_z, dact=dact, colsum=dx_colsum, colsum_scratch=cs, name=f"{self.name}.dX")
+                 dact_z=dact_z, dact=dact, colsum=dx_colsum, colsum_scratch=cs, name=f"{self.name}.dX")
         if not bias_grad_done:
             c.col_sum(dy16, self.b.g32, O, R, graph=graph)
         return dx if need_dx else None
@@ -559,8 +559,7 @@ class GPT:
         c.launch(gh, lambda: _check(lib.vkg_finals_defer(h, 1), "finals_defer"), "finals_defer")
         if self.tie:
             # dh = dlogits tok ; head's share of dtok = dlogits^T h (overwrites tok.g32)
-            gemm(c.dev, self.dlog16, self.tok.w16, self.dh32, R, D, V, graph=gh, split_k=-1,
-                 name="head.dX")
+            gemm(c.dev, self.dlog16, self.tok.w16, self.dh32, R, D, V, graph=gh, name="head.dX")
             gemm(c.dev, self.dlog16, self.h16, self.tok.g32, V, D, R, trans_a=True, graph=gh,
                  name="head.dW")
             d = self.dh32
