@@ -23,7 +23,7 @@ import numpy as np
 
 from . import _lib
 from ._lib import ACT_GELU, ACT_NONE, ACT_RELU, F16, F32
-from .kernels import CONFIGS, TILE, Matmul, gemm, gemm_group, make_kernels
+from .kernels import CONFIGS, TILE, Matmul, gemm, gemm_group, k_slices, make_kernels
 from .vk import VkError, _check
 
 
@@ -338,16 +338,17 @@ class MLP:
                    "softmax_ce")
         self.ctx.launch(graph, go, "softmax_ce", B * pad * 10)
 
-    # Rows up to which a recorded backward runs the dW of all layers in one launch.  A group's
-    # tiles do not split their K, the batch, as a launch of its own may: 784-256-256-16 at 256 rows
-    # 14.5 -> 5.7 us, 256-256-256-16 at 4096 rows still 24.2 -> 21.9.
-    GROUP_ROWS = 4096
+    def _groups_dw(self):
+        """Whether a recorded backward runs the dW of all layers in one launch (784-256-256-16 at
+        256 rows 14.5 -> 5.7 us).  A group's tiles take K, the batch, whole, so it is for batches
+        that no layer's own launch would cut: the sums are then the same."""
+        return all(l.in_f % 8 == 0 and l.out_f % 8 == 0
+                   and k_slices(self.ctx.dev, l.in_f, l.out_f, self.batch) == 1 for l in self.layers)
 
     def _backward(self, graph):
         g16, g32 = self.dlog16, self.dlog32
         sink = None
-        if graph is not None and self.batch <= self.GROUP_ROWS and \
-                all(l.in_f % 8 == 0 and l.out_f % 8 == 0 for l in self.layers):
+        if graph is not None and self._groups_dw():
             sink = ([], [])
         for i in reversed(range(len(self.layers))):
             below = self.layers[i - 1] if i > 0 else None

@@ -107,6 +107,13 @@ def _gemm_args(dev, a, b, c, m, n, k, trans_a=False, trans_b=False,
     return args
 
 
+def k_slices(dev, m, n, k):
+    """How many slices the library cuts K into for a plain fp32 output (1: whole), by its rule of
+    m, n and k."""
+    args = GemmArgs(M=m, N=n, K=k, ldc=n, C=16, c_dtype=F32)
+    return max(dev.lib.vkg_gemm_workspace_bytes(C.byref(args)) // (4 * m * n), 1)
+
+
 def gemm(dev, a, b, c, m, n, k, trans_a=False, trans_b=False, graph=None, repeat=1, name="gemm",
          **kw):
     """C = op(A) op(B) with the fused epilogue of vkg_gemm (include/vkgrad_b200.h).
