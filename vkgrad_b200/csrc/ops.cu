@@ -991,6 +991,18 @@ __global__ void k_layernorm_vec(const float* __restrict__ x, const float* __rest
 
 constexpr int LNB_WARPS = 4;
 
+// One column's share of a row's two sums, and the row's gradient there.  Written out to the last
+// rounding, because two kernels share it and have to give the same bits: left to the compiler, which
+// of two products goes into an fma may differ from one to the next.
+__device__ __forceinline__ void ln_bwd_take(float dxh, float xh, float& s1, float& s2) {
+  s1 = __fadd_rn(s1, dxh);
+  s2 = __fmaf_rn(dxh, xh, s2);
+}
+__device__ __forceinline__ float ln_bwd_dx(float dy, float gamma, float xh, float r, float s1, float s2, float inv) {
+  const float centred = __fmaf_rn(dy, gamma, -__fmul_rn(s1, inv));
+  return __fmul_rn(r, __fmaf_rn(-__fmul_rn(xh, s2), inv, centred));
+}
+
 // Backward.  Each CTA owns a contiguous band of rows; warp w handles rows
 // band0+w, band0+w+4, ...  Per-column partial sums of dy*xhat and dy are kept
 // in the warp's private shared-memory strip, combined across the CTA's warps
@@ -1023,9 +1035,7 @@ k_layernorm_bwd(const float* __restrict__ dy, const float* __restrict__ x,
     for (int d = lane; d < D; d += 32) {
       float dyv = dy[base + d];
       float xh = (x[base + d] - m) * r;
-      float dxh = dyv * gamma[d];
-      s1 += dxh;
-      s2 += dxh * xh;
+      ln_bwd_take(dyv * gamma[d], xh, s1, s2);
       if (dyxh16) dyxh16[base + d] = __float2half_rn(dyv * xh);
       if (dy16) dy16[base + d] = __float2half_rn(dyv);
       if (scratch) {
@@ -1036,10 +1046,8 @@ k_layernorm_bwd(const float* __restrict__ dy, const float* __restrict__ x,
     s1 = warp_sum(s1);
     s2 = warp_sum(s2);
     for (int d = lane; d < D; d += 32) {
-      float xh = (x[base + d] - m) * r;
-      float dxh = dy[base + d] * gamma[d];
-      float o = r * (dxh - s1 * inv - xh * s2 * inv);
-      if (dres) o += dres[base + d];
+      float o = ln_bwd_dx(dy[base + d], gamma[d], (x[base + d] - m) * r, r, s1, s2, inv);
+      if (dres) o = __fadd_rn(o, dres[base + d]);
       if (dx) dx[base + d] = o;
       if (dx16) dx16[base + d] = __float2half_rn(o);
     }
@@ -1190,53 +1198,45 @@ k_layernorm_bwd_vec(const float* __restrict__ dy, const float* __restrict__ x,
   }
 }
 
-// Backward without parameter sums (they come from column sums over the dy * xhat and dy copies):
-// one warp per row, everything read once.  The scalar kernel read each row twice: 9.7 -> 4.1 us at
-// 1024 x 768.
+// Backward that leaves the parameter sums to column sums over its dy * xhat and dy copies: one warp
+// per row, the row in registers.  k_layernorm_bwd reads each row twice, the second time behind the
+// reductions: 6.7 -> 4.0 us at 1024 x 768, back to back.  A lane has the columns it has there,
+// 32 apart, and adds them in the same order, so the bits are the same.
 template <int NV>
 __global__ void __launch_bounds__(128)
 k_layernorm_bwd_rows(const float* __restrict__ dy, const float* __restrict__ x, const float* __restrict__ gamma,
                      const float* __restrict__ mu, const float* __restrict__ rstd, const float* __restrict__ dres,
                      float* __restrict__ dx, __half* __restrict__ dx16, __half* __restrict__ dyxh16,
                      __half* __restrict__ dy16, int rows) {
-  constexpr int D = NV * 128;
+  constexpr int D = NV * 128, N = NV * 4;
   pdl_trigger();
   pdl_wait();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int row = blockIdx.x * (blockDim.x >> 5) + warp;
   if (row >= rows) return;
-  const size_t base = (size_t)row * D;
-  const float m = mu[row], r = rstd[row];
-  float4 xv[NV], dv[NV];
+  const size_t base = (size_t)row * D + lane;
+  const float m = mu[row], r = rstd[row], inv = 1.0f / (float)D;
+  float xh[N], dv[N], s1 = 0.f, s2 = 0.f;
 #pragma unroll
-  for (int i = 0; i < NV; ++i) {
-    xv[i] = *reinterpret_cast<const float4*>(x + base + (i * 32 + lane) * 4);
-    dv[i] = *reinterpret_cast<const float4*>(dy + base + (i * 32 + lane) * 4);
+  for (int i = 0; i < N; ++i) {
+    xh[i] = x[base + i * 32];
+    dv[i] = dy[base + i * 32];
   }
-  float s1 = 0.f, s2 = 0.f;
 #pragma unroll
-  for (int i = 0; i < NV; ++i) {
-    const int c = (i * 32 + lane) * 4;
-    const float4 g = *reinterpret_cast<const float4*>(gamma + c);
-    xv[i] = make_float4((xv[i].x - m) * r, (xv[i].y - m) * r, (xv[i].z - m) * r, (xv[i].w - m) * r);
-    if (dy16) *reinterpret_cast<uint2*>(dy16 + base + c) = pack4_h(dv[i]);
-    if (dyxh16)
-      *reinterpret_cast<uint2*>(dyxh16 + base + c) =
-          pack4_h(make_float4(dv[i].x * xv[i].x, dv[i].y * xv[i].y, dv[i].z * xv[i].z, dv[i].w * xv[i].w));
-    dv[i] = make_float4(dv[i].x * g.x, dv[i].y * g.y, dv[i].z * g.z, dv[i].w * g.w);
-    s1 += (dv[i].x + dv[i].y) + (dv[i].z + dv[i].w);
-    s2 += (dv[i].x * xv[i].x + dv[i].y * xv[i].y) + (dv[i].z * xv[i].z + dv[i].w * xv[i].w);
+  for (int i = 0; i < N; ++i) {
+    xh[i] = (xh[i] - m) * r;
+    ln_bwd_take(dv[i] * gamma[i * 32 + lane], xh[i], s1, s2);
+    if (dyxh16) dyxh16[base + i * 32] = __float2half_rn(dv[i] * xh[i]);
+    if (dy16) dy16[base + i * 32] = __float2half_rn(dv[i]);
   }
-  s1 = warp_sum(s1) * (1.0f / D);
-  s2 = warp_sum(s2) * (1.0f / D);
+  s1 = warp_sum(s1);
+  s2 = warp_sum(s2);
 #pragma unroll
-  for (int i = 0; i < NV; ++i) {
-    const size_t at = base + (i * 32 + lane) * 4;
-    float4 o = make_float4(r * (dv[i].x - s1 - xv[i].x * s2), r * (dv[i].y - s1 - xv[i].y * s2),
-                           r * (dv[i].z - s1 - xv[i].z * s2), r * (dv[i].w - s1 - xv[i].w * s2));
-    if (dres) o = add4(o, *reinterpret_cast<const float4*>(dres + at));
-    if (dx) *reinterpret_cast<float4*>(dx + at) = o;
-    if (dx16) *reinterpret_cast<uint2*>(dx16 + at) = pack4_h(o);
+  for (int i = 0; i < N; ++i) {
+    float o = ln_bwd_dx(dv[i], gamma[i * 32 + lane], xh[i], r, s1, s2, inv);
+    if (dres) o = __fadd_rn(o, dres[base + i * 32]);
+    if (dx) dx[base + i * 32] = o;
+    if (dx16) dx16[base + i * 32] = __float2half_rn(o);
   }
 }
 
@@ -2198,10 +2198,11 @@ extern "C" int vkg_layernorm_bwd(vkg_device* dev, const float* dy, const float* 
   int nblocks = ln_bwd_blocks(rows);
   const bool aligned = ((((uintptr_t)dy | (uintptr_t)x | (uintptr_t)gamma | (uintptr_t)dres |
                           (uintptr_t)dx | (uintptr_t)scratch) & 15) == 0) && (((uintptr_t)dx16 & 7) == 0);
-  if (D % 128 == 0 && D <= 1024 && !fused && aligned && (((uintptr_t)dyxh16 | (uintptr_t)dy16) & 7) == 0) {
-#define VKG_LNR(NV)                                                                                            \
-  VKG_RUN(VKG_K_LN_BWD, (int64_t)rows * D <= SHORT_ROWS, k_layernorm_bwd_rows<NV>, dim3((unsigned)((rows + 3) / 4)), 128, \
-          dy, x, gamma, mu, rstd, dres, dx, (__half*)dx16, (__half*)dyxh16, (__half*)dy16, rows)
+  if (D % 128 == 0 && D <= 1024 && !fused && aligned && (dyxh16 || dy16)) {
+#define VKG_LNR(NV)                                                                                           \
+  VKG_RUN(VKG_K_LN_BWD, (int64_t)rows * D <= SHORT_ROWS, k_layernorm_bwd_rows<NV>,                            \
+          dim3((unsigned)((rows + 3) / 4)), 128, dy, x, gamma, mu, rstd, dres, dx, (__half*)dx16,             \
+          (__half*)dyxh16, (__half*)dy16, rows)
     switch (D / 128) {
       case 1: VKG_LNR(1); break;
       case 2: VKG_LNR(2); break;
