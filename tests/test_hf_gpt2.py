@@ -255,3 +255,22 @@ def test_forward_lengths_rows_and_held_results(dev, B, T, n):
     finally:
         ctx.destroy()
     assert all(np.array_equal(a, b) for a, b in zip(kept, copies))
+
+
+@pytest.mark.gpu
+def test_forward_without_memory_to_pin(dev):
+    """With nothing left to pin, the results are ordinary arrays with the same values."""
+    from vkgrad_b200.transformer import GPT, TCtx
+    ctx = TCtx(dev)
+    try:
+        fwd = hf_gpt2.Forward(GPT(ctx, 2, 136, 128, 2, 1, 250, tie=True))
+        ids = np.random.default_rng(0).integers(0, 250, (2, 136))
+        full, last = fwd(ids), fwd(ids, last=True)
+        del fwd.pools[False], fwd.pools[True]
+        fwd.pools.update({k: hf_gpt2.PinnedPool(dev, limit=2) for k in (False, True)})
+        for pool in fwd.pools.values():        # each call asks for more than an address space holds
+            pool.take = lambda shape, dtype, at_least=0, take=pool.take: take(shape, dtype, 1 << 50)
+        assert np.array_equal(fwd(ids), full) and np.array_equal(fwd(ids, last=True), last)
+        assert all(pool._state["n"] == 0 for pool in fwd.pools.values())
+    finally:
+        ctx.destroy()

@@ -289,3 +289,42 @@ def test_slices_of_k_follow_the_shape_alone():
         a.bias = 1 << 20           # an epilogue: K stays whole
         assert lib.vkg_gemm_workspace_bytes(C.byref(a)) == 0
     assert 30 < cut < len(shapes) - 30
+
+
+class _FakeHost:
+    """vkg_host_alloc / vkg_host_free over ordinary memory, with a limit on the bytes pinned."""
+
+    def __init__(self, limit):
+        self.limit, self.blocks, self.handle, self.lib = limit, {}, None, self
+
+    def vkg_host_alloc(self, handle, size, out):
+        if size + sum(map(len, self.blocks.values())) > self.limit:
+            return 1
+        block = (C.c_ubyte * size)()
+        out._obj.value = C.addressof(block)
+        self.blocks[C.addressof(block)] = block
+        return 0
+
+    def vkg_host_free(self, ptr):
+        del self.blocks[ptr]
+        return 0
+
+
+def test_pinned_pool_gives_none_where_the_system_has_nothing_to_pin():
+    """Refusals cost nothing later: the pool tries again, keeps its limit and gives everything back."""
+    from vkgrad_b200.vk import PinnedPool
+    host = _FakeHost(limit=100)
+    pool = PinnedPool(host, limit=2)
+    pool.reserve(200)
+    assert host.blocks == {} and pool.take((200,), np.uint8) is None
+    first = pool.take((60,), np.uint8)
+    first[:] = 7
+    assert pool.take((60,), np.uint8) is None
+    second = pool.take((10, 4), np.uint8)
+    assert second.shape == (10, 4) and pool.take((1,), np.uint8) is None     # both blocks in use
+    del second
+    assert pool.take((60,), np.uint8) is None and len(host.blocks) == 1      # 40 bytes go, 60 more do not fit
+    del pool
+    assert (first == 7).all() and len(host.blocks) == 1
+    del first
+    assert host.blocks == {}

@@ -423,8 +423,11 @@ extern "C" int vkg_host_alloc(vkg_device* dev, size_t bytes, void** hptr) {
   if (vkg_bind(dev)) return 1;
   VKG_REQUIRE(hptr, "null output pointer");
   *hptr = nullptr;
-  VKG_CUDA(cudaHostAlloc(hptr, bytes ? bytes : 16, cudaHostAllocPortable));
-  return 0;
+  cudaError_t e = cudaHostAlloc(hptr, bytes ? bytes : 16, cudaHostAllocPortable);
+  if (e == cudaSuccess) return 0;
+  cudaGetLastError();            // callers carry on without: the next launch must not find it
+  *hptr = nullptr;
+  VKG_FAIL("cudaHostAlloc(%zu) failed: %s", bytes, cudaGetErrorString(e));
 }
 
 extern "C" int vkg_host_free(void* hptr) {

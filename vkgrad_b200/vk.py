@@ -109,7 +109,7 @@ class PinnedPool:
 
     A block returns to the pool when the last view of its array is gone, and to the system when
     the pool has been closed as well, so an array outlives the pool, the model and the device
-    that filled it.  With every block still in use take() returns None.  Blocks move through a
+    that filled it.  Where there is none to give, take() returns None.  Blocks move through a
     deque (atomic appends and pops): finalizers may run in any thread, at any point."""
 
     def __init__(self, dev, limit=2):
@@ -143,8 +143,8 @@ class PinnedPool:
         self.take((nbytes,), np.uint8)      # the array is dropped here: its block is free again
 
     def take(self, shape, dtype, at_least=0):
-        """An uninitialised pinned array, or None while every block is in use.  A new block holds
-        at_least that many bytes."""
+        """An uninitialised pinned array, or None while every block is in use or when the system
+        has no more memory to pin.  A new block holds at_least that many bytes."""
         st, nbytes = self._state, int(np.prod(shape)) * np.dtype(dtype).itemsize
         block = None
         try:
@@ -158,8 +158,8 @@ class PinnedPool:
                 return None
         if block is None:
             p, size = C.c_void_p(), max(nbytes, int(at_least))
-            _check(st["lib"].vkg_host_alloc(self.dev.handle, size, C.byref(p)),
-                   f"pinned block of {size} bytes")
+            if st["lib"].vkg_host_alloc(self.dev.handle, size, C.byref(p)) != 0:
+                return None
             block = (p.value, size)
             st["n"] += 1
         raw = (C.c_ubyte * nbytes).from_address(block[0])
