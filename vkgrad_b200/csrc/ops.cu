@@ -2018,7 +2018,11 @@ extern "C" int vkg_adamw_multi(vkg_device* dev, void* table, const float* hp) {
   if (vkg_bind(dev)) return 1;
   VKG_REQUIRE(table && hp, "adamw_multi: bad arguments");
   AdamTable* t = (AdamTable*)table;
-  const float* host = host_view(hp);
+  // A capture that the caller began on this device's stream is not ours to refresh: there the kernel
+  // reads the scalars itself, whenever the graph runs.
+  cudaStreamCaptureStatus theirs = cudaStreamCaptureStatusNone;
+  if (!dev->capturing) VKG_CUDA(cudaStreamIsCapturing(dev->stream, &theirs));
+  const float* host = theirs == cudaStreamCaptureStatusNone ? host_view(hp) : nullptr;
   AdamHp val = {};
   if (host) {
     memcpy(val.v, host, 7 * sizeof(float));
