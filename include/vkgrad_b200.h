@@ -105,6 +105,10 @@ int vkg_sync(vkg_device* dev);
  * never).  Returns what the wait returns; *aborted = number of aborts issued. */
 int vkg_selftest_wait_deadline(int64_t ready_after_polls, int64_t async_error_at,
                                double timeout_s, int* aborted);
+/* No reference counterpart, no device needed: two threads enter a fresh device together, `rounds`
+ * times; *unmarked receives how often neither noticed the other (vkg_sync may skip its wait only
+ * while one thread uses the device). */
+int vkg_selftest_first_threads(int rounds, int* unmarked);
 
 /* dev.buffer(size, kind) (vk.py:1256, memory kinds vk.py:1161-1200).
  * kind 0 "device": HBM only.  kind 1 "shared": pinned, mapped host memory the

@@ -238,6 +238,13 @@ def test_host_wait_reports_an_asynchronous_communicator_error_before_the_deadlin
     assert time.perf_counter() - t0 < 5.0
 
 
+def test_two_threads_that_enter_a_device_together_notice_each_other():
+    from vkgrad_b200 import _lib
+    unmarked = C.c_int32(-1)
+    assert _lib.load().vkg_selftest_first_threads(20000, C.byref(unmarked)) == 0
+    assert unmarked.value == 0
+
+
 def _slices(M, N, K):
     """The rule of M, N and K by which a GEMM's K is cut, restated: the cheapest of up to 8 slices
     (16 where the partial sums fit 1 MB), of waves of tiles on 148 SMs plus the reduction."""

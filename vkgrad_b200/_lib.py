@@ -67,6 +67,7 @@ _SIGNATURES = {
     "vkg_set_tuning": (i32, [vp, i32, i64]),
     "vkg_sync": (i32, [vp]),
     "vkg_selftest_wait_deadline": (i32, [i64, i64, C.c_double, C.POINTER(i32)]),
+    "vkg_selftest_first_threads": (i32, [i32, C.POINTER(i32)]),
     "vkg_alloc": (i32, [vp, sz, i32, C.POINTER(vp), C.POINTER(vp)]),
     "vkg_free": (i32, [vp, vp, vp, i32]),
     "vkg_upload": (i32, [vp, vp, vp, sz]),

@@ -203,6 +203,15 @@ int vkg_launch_col_sum_final(vkg_device* dev, const float* partial, float* sums,
     }                            \
   } while (0)
 
+// The first thread to enter leaves its mark; any other one marks the device as shared.  Of two that
+// enter for the first time together, exactly one is first.
+static inline void vkg_note_thread(std::atomic<const void*>& first, std::atomic<bool>& shared, const void* self) {
+  const void* seen = first.load(std::memory_order_relaxed);
+  if (seen == self) return;
+  if (seen == nullptr && first.compare_exchange_strong(seen, self)) return;
+  shared.store(true);
+}
+
 // Makes `dev` current on this thread and checks the launch that just happened.
 static inline int vkg_bind(vkg_device* dev) {
   if (!dev) {
@@ -210,11 +219,7 @@ static inline int vkg_bind(vkg_device* dev) {
     return 1;
   }
   static thread_local char self;
-  const void* seen = dev->thread.load(std::memory_order_relaxed);
-  if (seen != &self) {
-    if (seen == nullptr) dev->thread.store(&self);
-    else dev->stream_shared.store(true);
-  }
+  vkg_note_thread(dev->thread, dev->stream_shared, &self);
   dev->entered.fetch_add(1);
   cudaError_t e = cudaSetDevice(dev->ordinal);
   if (e != cudaSuccess) {

@@ -360,6 +360,35 @@ extern "C" int vkg_selftest_wait_deadline(int64_t ready_after_polls, int64_t asy
   return rc;
 }
 
+// Two threads that enter a fresh device together, `rounds` times: how often neither of them marked it
+// as shared.  For tests without a GPU.
+extern "C" int vkg_selftest_first_threads(int rounds, int* unmarked) {
+  VKG_REQUIRE(rounds > 0 && unmarked, "selftest: bad arguments");
+  std::atomic<const void*> first{nullptr};
+  std::atomic<bool> shared{false};
+  std::atomic<int> go{0}, done{0};
+  *unmarked = 0;
+  const auto enter = [&](const void* self) {
+    for (int i = 1; i <= rounds; ++i) {
+      while (go.load() < i) std::this_thread::yield();
+      vkg_note_thread(first, shared, self);
+      done.fetch_add(1);
+    }
+  };
+  int a, b;
+  std::thread t1(enter, &a), t2(enter, &b);
+  for (int i = 1; i <= rounds; ++i) {
+    first.store(nullptr);
+    shared.store(false);
+    go.store(i);
+    while (done.load() < 2 * i) std::this_thread::yield();
+    if (!shared.load()) ++*unmarked;
+  }
+  t1.join();
+  t2.join();
+  return 0;
+}
+
 int vkg_stamp_finish(vkg_device* dev, const vkg_stamp* st, const char* what, double* seconds) {
   if (vkg_wait_device(dev, st, what)) return 1;
   if (seconds) *seconds = (double)st->host->ticks * 32e-9;
