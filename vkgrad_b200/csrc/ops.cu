@@ -678,18 +678,20 @@ __global__ void __launch_bounds__(32 * CSF_SLICES) k_col_sum_final_multi(const _
 
 // ---- softmax + cross entropy ---------------------------------------------------------
 
-// Running maximum m and sum s of exp(x - m): one more value, or another such pair.
+// Running maximum m and sum s of exp(x - m): one more value, or another such pair.  Written out to the
+// last rounding: the two kernels below have to give the same bits, and which of two products goes
+// into an fma is otherwise the compiler's choice in each of them.
 __device__ __forceinline__ void ce_take(float v, float& m, float& s) {
   if (v > m) {
-    s = s * __expf(m - v) + 1.0f;
+    s = __fmaf_rn(s, __expf(m - v), 1.0f);
     m = v;
   } else {
-    s += __expf(v - m);
+    s = __fadd_rn(s, __expf(v - m));
   }
 }
 __device__ __forceinline__ void ce_merge(float& m, float& s, float m2, float s2) {
   const float mm = fmaxf(m, m2);
-  s = s * __expf(m - mm) + s2 * __expf(m2 - mm);
+  s = __fmaf_rn(s, __expf(m - mm), __fmul_rn(s2, __expf(m2 - mm)));
   m = mm;
 }
 
@@ -753,10 +755,10 @@ k_softmax_ce(const float* __restrict__ logits, const uint32_t* __restrict__ labe
 
 // Narrow rows (a byte-level vocabulary, a classifier's head): one warp per row, the row in
 // registers, NV values per lane; a block per row spent its time on two barriers and eight idle
-// warps (2048 rows: 96 logits 11.6 -> 4.9 us, 256 logits 12.1 -> 7.1).  It adds in k_softmax_ce's order -- columns c and c + 256 in one
-// chain, 32 columns by a butterfly, the eight groups of 32 in turn -- so that the results are the
-// same bits: fp16 gradients without a loss scale are small enough for the last bit of a row's
-// normaliser to show in the weights.
+// warps (2048 rows: 96 logits 11.6 -> 4.9 us, 256 logits 12.1 -> 7.1).  It adds in k_softmax_ce's
+// order -- columns c and c + 256 in one chain, 32 columns by a butterfly, the eight groups of 32 in
+// turn -- so that the results are the same bits: fp16 gradients without a loss scale are small
+// enough for the last bit of a row's normaliser to show in the weights.
 template <int NV>
 __global__ void __launch_bounds__(128)
 k_softmax_ce_warp(const float* __restrict__ logits, const uint32_t* __restrict__ labels,
@@ -1257,7 +1259,7 @@ __global__ void k_attn_softmax(const float* __restrict__ s, const uint32_t* __re
   for (int j = st + lane; j <= q; j += 32) mx = fmaxf(mx, s[base + j] * scale);
   mx = warp_max(mx);
   float sum = 0.f;
-  for (int j = st + lane; j <= q; j += 32) sum += __expf(s[base + j] * scale - mx);
+  for (int j = st + lane; j <= q; j += 32) sum += __expf(fmaf(s[base + j], scale, -mx));
   sum = warp_sum(sum);
   const float inv = 1.0f / sum;
   // zeros above the diagonal: to the end of the row, or only to the end of the
@@ -1265,7 +1267,7 @@ __global__ void k_attn_softmax(const float* __restrict__ s, const uint32_t* __re
   const int jend = fill_block > 0 ? min(T, (q / fill_block + 1) * fill_block) : T;
   for (int j = lane; j < jend; j += 32) {
     float v = 0.f;
-    if (j >= st && j <= q) v = __expf(s[base + j] * scale - mx) * inv;
+    if (j >= st && j <= q) v = __expf(fmaf(s[base + j], scale, -mx)) * inv;
     p16[base + j] = __float2half_rn(v);
   }
 }
@@ -1279,7 +1281,7 @@ __global__ void k_attn_softmax_bwd(const float* __restrict__ dp, const __half* _
   const int64_t base = row * T;
   const int q = (int)(row % T);
   float dot = 0.f;
-  for (int j = lane; j <= q; j += 32) dot += dp[base + j] * __half2float(p16[base + j]);
+  for (int j = lane; j <= q; j += 32) dot = fmaf(dp[base + j], __half2float(p16[base + j]), dot);
   dot = warp_sum(dot);
   const int jend = fill_block > 0 ? min(T, (q / fill_block + 1) * fill_block) : T;
   for (int j = lane; j < jend; j += 32) {
