@@ -246,17 +246,16 @@ def test_two_threads_that_enter_a_device_together_notice_each_other():
 
 
 def _slices(M, N, K):
-    """The rule of M, N and K by which a GEMM's K is cut, restated: the cheapest of up to 8 slices
-    (16 where the partial sums fit 1 MB), of waves of tiles on 148 SMs plus the reduction."""
+    """The rule of M, N and K by which a GEMM's K is cut, restated: the cheapest number of up to 16
+    slices, in waves of tiles on 148 SMs and what the reduction takes."""
     up = lambda a, b: -(-a // b)
     kbs, out = up(K, 64), 4 * M * N
-    most = min(max((1 << 20) // out, 8), 16)
 
     def best(bm, slots, widths):
         times = []
         for bn in widths:
             kb_us = {256: 0.41, 192: 0.36}.get(bn, 0.33)
-            for sp in range(1, most + 1):
+            for sp in range(1, 17):
                 if sp == 1 or kbs // sp >= 4:
                     waves = up(up(M, bm) * up(N, bn) * sp, slots)
                     times.append((waves * (up(kbs, sp) * kb_us + 4.4 * bn / 256)

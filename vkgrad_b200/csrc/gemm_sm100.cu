@@ -1337,13 +1337,10 @@ bool may_split(const vkg_gemm_args* a) {
 // 2e-3 of that in its second step (512-wide model, 1800 rows: the head's dW).  The rule: few
 // 256-column pair tiles, or few single ones, are cut while that shortens the waves of a full B200 by
 // more than the reduction costs, by the k-block and epilogue times of an early version of the kernel.
-// At most 8 slices, or 16 where the partial sums are small.
-constexpr int SLICE_SMS = 148;
-constexpr int64_t SLICE_SMALL_BYTES = 1 << 20;
+constexpr int SLICE_SMS = 148, SLICE_MAX = 16;
 int k_slices(const vkg_gemm_args* a) {
   const int num_kb = (a->K + BK - 1) / BK, n_round = ((a->N + 63) / 64) * 64;
-  const int64_t out_bytes = (int64_t)a->M * a->N * 4, small = SLICE_SMALL_BYTES / out_bytes;
-  const int most = small < 8 ? 8 : small > 16 ? 16 : (int)small;
+  const int64_t out_bytes = (int64_t)a->M * a->N * 4;
   const auto slices = [&](int bm, int slots, int only_bn) {
     double best = -1.0;
     int got = 1;
@@ -1351,7 +1348,7 @@ int k_slices(const vkg_gemm_args* a) {
       if (only_bn ? bn != only_bn : bn > n_round && bn != 64) continue;
       const long long tiles = (long long)((a->M + bm - 1) / bm) * ((a->N + bn - 1) / bn);
       const double t_kb = bn == 256 ? 0.41 : bn == 192 ? 0.36 : 0.33;
-      for (int sp = 1; sp <= most; ++sp) {
+      for (int sp = 1; sp <= SLICE_MAX; ++sp) {
         if (sp > 1 && num_kb / sp < 4) break;
         const long long waves = (tiles * sp + slots - 1) / slots;
         double t = waves * ((num_kb + sp - 1) / sp * t_kb + 4.4 * bn / 256.0);
