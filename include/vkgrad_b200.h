@@ -428,7 +428,7 @@ int vkg_embed_bwd(vkg_device* dev, const float* dx, const uint32_t* ids,
                   int T);
 /* The same scatter-add without atomics: rows that hit one table row are added in row
  * order by one warp, so the result is bit-reproducible from run to run (the reference's
- * float atomics are not).  D a multiple of 128 up to 1024; scratch holds
+ * float atomics are not).  D a multiple of 4 up to 1024; scratch holds
  * vkg_embed_bwd_scratch_bytes(n / D) bytes. */
 int64_t vkg_embed_bwd_scratch_bytes(int64_t rows);
 int vkg_embed_bwd_det(vkg_device* dev, const float* dx, const uint32_t* ids,

@@ -467,19 +467,20 @@ k_embed_chain(const int* __restrict__ keys, int* __restrict__ next, int* __restr
   }
 }
 
+// A lane has four columns of every 128; of the last 128 those that are left of D.
 template <int NV>
 __global__ void __launch_bounds__(256)
 k_embed_bwd_chain(const float* __restrict__ dx, const uint32_t* __restrict__ ids,
                   const uint32_t* __restrict__ seg, const int* __restrict__ next,
                   const int* __restrict__ has_prev, float* __restrict__ dtok, float* __restrict__ dpos,
-                  int rows, int T) {
-  constexpr int D = NV * 128;
+                  int rows, int D, int T) {
   pdl_trigger();
   pdl_wait();
   const int which = blockIdx.y;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int r0 = blockIdx.x * (blockDim.x >> 5) + warp;
   if (r0 >= rows || has_prev[which * rows + r0]) return;
+  const bool last = ((NV - 1) * 32 + lane) * 4 < D;
   float4 acc[NV];
 #pragma unroll
   for (int i = 0; i < NV; ++i) acc[i] = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -500,16 +501,19 @@ k_embed_bwd_chain(const float* __restrict__ dx, const uint32_t* __restrict__ ids
       if (at[u] >= 0)
 #pragma unroll
         for (int i = 0; i < NV; ++i)
-          g[u][i] = *reinterpret_cast<const float4*>(dx + (size_t)at[u] * D + (i * 32 + lane) * 4);
+          if (i < NV - 1 || last)
+            g[u][i] = *reinterpret_cast<const float4*>(dx + (size_t)at[u] * D + (i * 32 + lane) * 4);
 #pragma unroll
     for (int u = 0; u < U; ++u)
       if (at[u] >= 0)
 #pragma unroll
-        for (int i = 0; i < NV; ++i) acc[i] = add4(acc[i], g[u][i]);
+        for (int i = 0; i < NV; ++i)
+          if (i < NV - 1 || last) acc[i] = add4(acc[i], g[u][i]);
   }
   float* row = (which == 0 ? dtok : dpos) + (size_t)embed_key(which, r0, ids, seg, T) * D;
 #pragma unroll
   for (int i = 0; i < NV; ++i) {
+    if (i == NV - 1 && !last) break;
     float4* p = reinterpret_cast<float4*>(row + (i * 32 + lane) * 4);
     float4 v = *p;
     v.x += acc[i].x; v.y += acc[i].y; v.z += acc[i].z; v.w += acc[i].w;
@@ -2422,9 +2426,9 @@ extern "C" int vkg_embed_bwd_det(vkg_device* dev, const float* dx, const uint32_
   if (vkg_bind(dev)) return 1;
   VKG_REQUIRE(dx && ids && dtok && dpos && scratch && n > 0 && D > 0 && T > 0,
               "embed_bwd_det: bad arguments");
-  VKG_REQUIRE(D % 128 == 0 && D <= 1024 && n % D == 0 && n / D < (1ll << 30) &&
+  VKG_REQUIRE(D % 4 == 0 && D <= 1024 && n % D == 0 && n / D < (1ll << 30) &&
                   ((((uintptr_t)dx | (uintptr_t)dtok | (uintptr_t)dpos | (uintptr_t)scratch) & 15) == 0),
-              "embed_bwd_det: D must be a multiple of 128 up to 1024 and the tables 16-byte aligned "
+              "embed_bwd_det: D must be a multiple of 4 up to 1024 and the tables 16-byte aligned "
               "(use vkg_embed_bwd otherwise)");
   const int rows = (int)(n / D), rows_p = (rows + 3) & ~3;
   int* keys = static_cast<int*>(scratch);
@@ -2437,10 +2441,10 @@ extern "C" int vkg_embed_bwd_det(vkg_device* dev, const float* dx, const uint32_
                       1, (const int*)keys, next, has_prev, rows, rows_p));
   if (vkg_check_launch("embed_chain")) return 1;
   const dim3 grid((unsigned)((rows + 7) / 8), 2);
-#define VKG_EB(NV)                                                                               \
-  VKG_CUDA(vkg_launch(dev, VKG_K_SMALL | vkg_short_if(n <= SHORT_ROWS), k_embed_bwd_chain<NV>, grid, dim3(256), 0, 1, dx, ids, seg, \
-                      (const int*)next, (const int*)has_prev, dtok, dpos, rows, T))
-  switch (D / 128) {
+#define VKG_EB(NV)                                                                            \
+  VKG_RUN(VKG_K_SMALL, n <= SHORT_ROWS, k_embed_bwd_chain<NV>, grid, 256, dx, ids, seg, next, \
+          has_prev, dtok, dpos, rows, D, T)
+  switch ((D + 127) / 128) {
     case 1: VKG_EB(1); break;
     case 2: VKG_EB(2); break;
     case 3: VKG_EB(3); break;

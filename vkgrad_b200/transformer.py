@@ -603,7 +603,7 @@ class GPT:
         # rows that share a token (or a position) are added in row order by one warp, so the
         # whole step is bit-reproducible; table widths the kernel has no instance for keep
         # the reference's atomic scatter-add
-        det = D % 128 == 0 and D <= 1024
+        det = D % 4 == 0 and D <= 1024
         if det and getattr(self, "_emb_scratch", None) is None:
             self._emb_scratch = c.buf(lib.vkg_embed_bwd_scratch_bytes(R))
 
