@@ -408,9 +408,10 @@ int vkg_finals_flush(vkg_device* dev);
  * vkg_col_sum_static_max_floats() floats (see vkg_col_sum_scratch_floats) are
  * refused with an error.  The first call on each device looks the array's
  * device address up (cudaGetSymbolAddress); make that first call before any
- * stream capture begins (during a capture it returns an error instead).  All calls on a device share the one array: two calls
- * whose kernels may overlap on the GPU (different streams or devices handles on
- * the same GPU) race on it, so keep them on one stream. */
+ * stream capture begins (during a capture it returns an error instead).  All
+ * calls on a device share the one array: two calls whose kernels may overlap on
+ * the GPU (different streams or devices handles on the same GPU) race on it, so
+ * keep them on one stream. */
 int vkg_col_sum_static(vkg_device* dev, const void* g, int g_dtype, float* sums,
                        int ncol, int nrow, int accumulate);
 int64_t vkg_col_sum_static_max_floats(void);

@@ -1420,7 +1420,8 @@ extern "C" int vkg_attn_fwd(vkg_device* dev, const void* qkv16, const uint32_t* 
   }
   const long long ctas = (long long)p.nqt * H * B;
   VKG_REQUIRE(ctas < (1ll << 31), "attn_fwd: too many tiles");
-  VKG_CUDA(vkg_launch(dev, VKG_K_ATTN_FWD | vkg_short_if(ctas <= 2ll * dev->sm_count), dev->attn_one_pass ? attn_fwd1_kernel : attn_fwd_kernel,
+  VKG_CUDA(vkg_launch(dev, VKG_K_ATTN_FWD | vkg_short_if(ctas <= 2ll * dev->sm_count),
+                      dev->attn_one_pass ? attn_fwd1_kernel : attn_fwd_kernel,
                       dim3((unsigned)ctas), dim3(FA_THREADS), FW_SMEM, 1, tm, p));
   return vkg_check_launch("attn_fwd_kernel");
 }
@@ -1467,9 +1468,10 @@ extern "C" int vkg_attn_bwd(vkg_device* dev, const void* qkv16, const void* dout
   // snake order; the dQ kernel goes first because it also writes delta
   const int sms = vkg_persistent_ctas(dev);
   const unsigned ctas = (unsigned)(n_items < sms ? n_items : sms);
-  VKG_CUDA(vkg_launch(dev, VKG_K_ATTN_BWD | vkg_short_if(n_items <= sms), attn_bwd_q_kernel, dim3(ctas), dim3(DQ_THREADS), DQ_SMEM, 1, tm, tmdo, tmo, p));
+  const unsigned family = VKG_K_ATTN_BWD | vkg_short_if(n_items <= sms);
+  VKG_CUDA(vkg_launch(dev, family, attn_bwd_q_kernel, dim3(ctas), dim3(DQ_THREADS), DQ_SMEM, 1, tm, tmdo, tmo, p));
   if (vkg_check_launch("attn_bwd_q_kernel")) return 1;
-  VKG_CUDA(vkg_launch(dev, VKG_K_ATTN_BWD | vkg_short_if(n_items <= sms), attn_bwd_kv_kernel, dim3(ctas), dim3(BW_THREADS), KV_SMEM, 1, tm, tmdo, p));
+  VKG_CUDA(vkg_launch(dev, family, attn_bwd_kv_kernel, dim3(ctas), dim3(BW_THREADS), KV_SMEM, 1, tm, tmdo, p));
   if (vkg_check_launch("attn_bwd_kv_kernel")) return 1;
   if (dbias)
     return vkg_launch_col_sum_final(dev, dbias_scratch, dbias, 3 * D, B * p.nqt * 4, 0);

@@ -432,11 +432,14 @@ struct CtaCtx {
   uint8_t* epi_stage;
 };
 
-// TMA producer (one lane): stream nkb k-blocks of a tile's operands into the ring.
-__device__ __forceinline__ bool produce_range(const CtaCtx& cx, const GemmParams& p,
-                                              const CUtensorMap* tmA, const CUtensorMap* tmB,
-                                              const TileCoord& tc, int kb0, int nkb, int& stage,
-                                              uint32_t& phase) {
+// TMA producer (one lane): stream the k-blocks of work unit t's operands into the ring.
+__device__ __forceinline__ bool produce_unit(const CtaCtx& cx, const GemmParams& p,
+                                             const CUtensorMap* tmA, const CUtensorMap* tmB, int t,
+                                             int& stage, uint32_t& phase) {
+  TileCoord tc = tile_coord(p, t);
+  int kb0, nkb;
+  kb_range(p, tc, kb0, nkb);
+  if (p.split_k > 1) tc.z1 = 0;   // operands are not batched along the slice index
   for (int kb = 0; kb < nkb; ++kb) {
     if (!mbar_wait(cx.empty0 + 8 * stage, phase ^ 1u, cx.abort_flag, p.err, 0x100u + stage)) return false;
     const uint32_t fb = cx.full0 + 8 * stage;
@@ -464,21 +467,13 @@ __device__ __forceinline__ bool produce_range(const CtaCtx& cx, const GemmParams
   return true;
 }
 
-// The k-blocks of work unit t.
-__device__ __forceinline__ bool produce_unit(const CtaCtx& cx, const GemmParams& p,
-                                             const CUtensorMap* tmA, const CUtensorMap* tmB, int t,
-                                             int& stage, uint32_t& phase) {
-  TileCoord tc = tile_coord(p, t);
+// MMA issue (the whole warp, converged; one elected lane issues each instruction): accumulate the
+// k-blocks of work unit t into one of the two TMEM accumulators.
+__device__ __forceinline__ bool mma_unit(const CtaCtx& cx, const GemmParams& p, int t, int& stage,
+                                         uint32_t& phase, int& acc, uint32_t& acc_phase) {
   int kb0, nkb;
-  kb_range(p, tc, kb0, nkb);
-  if (p.split_k > 1) tc.z1 = 0;   // operands are not batched along the slice index
-  return produce_range(cx, p, tmA, tmB, tc, kb0, nkb, stage, phase);
-}
-
-// MMA issue (the whole warp, converged; one elected lane issues each instruction): accumulate
-// nkb k-blocks into one of the two TMEM accumulators.
-__device__ __forceinline__ bool mma_range(const CtaCtx& cx, const GemmParams& p, int nkb, int& stage,
-                                          uint32_t& phase, int& acc, uint32_t& acc_phase) {
+  kb_range(p, tile_coord(p, t), kb0, nkb);
+  if (nkb <= 0) return true;   // skipped tile: no accumulator, no epilogue
   if (!mbar_wait_warp(cx.tempty0 + 8 * acc, acc_phase ^ 1u, cx.abort_flag, p.err, 0x200u + acc)) return false;
   tcgen05_fence_after();
   const uint32_t d_tmem = cx.tmem_base + (uint32_t)(acc * ACC_COLS);
@@ -511,14 +506,6 @@ __device__ __forceinline__ bool mma_range(const CtaCtx& cx, const GemmParams& p,
   return true;
 }
 
-__device__ __forceinline__ bool mma_unit(const CtaCtx& cx, const GemmParams& p, int t, int& stage,
-                                         uint32_t& phase, int& acc, uint32_t& acc_phase) {
-  int kb0, nkb;
-  kb_range(p, tile_coord(p, t), kb0, nkb);
-  if (nkb <= 0) return true;   // skipped tile: no accumulator, no epilogue
-  return mma_range(cx, p, nkb, stage, phase, acc, acc_phase);
-}
-
 // Where the lanes of an epilogue warp stand in a 32 x 16 chunk on the per-lane path: four rows
 // (8 i + lane / 4) and four columns each.
 struct ChunkAt {
@@ -536,14 +523,16 @@ __device__ __forceinline__ ChunkAt chunk_at(const GemmParams& p, long long batch
   return c;
 }
 
-// One warp's chunks c0, c0 + step, ... < cols of a tile whose accumulator (a row per TMEM lane) is
-// complete once `ready` has returned; col0: the tile's first column; `load` starts bringing 16
-// columns into registers.
-template <int MODE, typename Ready, typename Load>
-__device__ __forceinline__ bool drain_chunks(const GemmParams& p, const CUtensorMap* tmC, const CUtensorMap* tmP,
-                                             const TileCoord& tc, int q, int lane, uint8_t* stage,
-                                             int first, int step, int cols, int col0, const Ready& ready,
-                                             const Load& load) {
+// One epilogue warp's chunks of a tile: 16 columns from `first` on, every `step`.  The accumulator (a
+// row per TMEM lane) is waited for only after the first fused operands have been requested.
+template <int MODE>
+__device__ __forceinline__ bool drain_chunks(const CtaCtx& cx, const GemmParams& p, const CUtensorMap* tmC,
+                                             const CUtensorMap* tmP, const TileCoord& tc, int warp, int lane,
+                                             int acc, uint32_t acc_phase, uint32_t wait_code) {
+  const int q = warp & 3;  // TMEM lane quarter this warp may read
+  const int first = 16 * ((warp - 2) >> 2), step = 64, cols = p.bn, col0 = tc.n0;
+  const uint32_t t_row = cx.tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)(acc * ACC_COLS);
+  uint8_t* stage = cx.epi_stage + (warp - 2) * EPI_STAGE_BYTES;
   const long long batch_off = (long long)tc.z0 * p.sC0 + (long long)tc.z1 * p.sC1;
   const int row_base = tc.m0 + q * 32;
   const bool tma_out = (MODE & E_NO_TMA) == 0 && p.tma_store != 0;
@@ -554,7 +543,8 @@ __device__ __forceinline__ bool drain_chunks(const GemmParams& p, const CUtensor
     const ChunkAt at = chunk_at(p, batch_off, row_base, col0 + first, lane);
     epilogue_fetch<MODE>(p, extra, at.off0, row8, at.ok);
   }
-  if (!ready()) return false;
+  if (!mbar_wait_warp(cx.tfull0 + 8 * acc, acc_phase, cx.abort_flag, p.err, wait_code + acc)) return false;
+  tcgen05_fence_after();
   if ((MODE & E_NO_TMA) == 0 && tma_out) {
     if (row_base >= p.M) return true;
     const int end = min(cols, p.N - col0);           // chunks that start inside the matrix
@@ -562,16 +552,16 @@ __device__ __forceinline__ bool drain_chunks(const GemmParams& p, const CUtensor
     if constexpr ((MODE & (E_F16 | E_BF16)) != 0 && (MODE & E_PRE) == 0) {
       for (; c0 + step < end; c0 += 2 * step) {
         uint32_t r[2][16];
-        load(c0, r[0]);
-        load(c0 + step, r[1]);
+        tmem_ld16(t_row + c0, r[0]);
+        tmem_ld16(t_row + c0 + step, r[1]);
         tmem_wait_ld();
-        epilogue_chunks_tma<MODE, 2>(p, tmC, tmP, r, stage, lane, col0 + c0, col0 + c0 + step,
-                                            row_base, tc.z0, tc.z1);
+        epilogue_chunks_tma<MODE, 2>(p, tmC, tmP, r, stage, lane, col0 + c0, col0 + c0 + step, row_base,
+                                     tc.z0, tc.z1);
       }
     }
     for (; c0 < end; c0 += step) {
       uint32_t r[1][16];
-      load(c0, r[0]);
+      tmem_ld16(t_row + c0, r[0]);
       tmem_wait_ld();
       epilogue_chunks_tma<MODE, 1>(p, tmC, tmP, r, stage, lane, col0 + c0, 0, row_base, tc.z0, tc.z1);
     }
@@ -580,7 +570,7 @@ __device__ __forceinline__ bool drain_chunks(const GemmParams& p, const CUtensor
   for (int c0 = first; c0 < cols; c0 += step) {
     if (col0 + c0 >= p.N) break;  // uniform across the warp
     uint32_t r[16];
-    load(c0, r);
+    tmem_ld16(t_row + c0, r);
     tmem_wait_ld();
     // TMEM gives each lane one row; the chunk is transposed through shared memory so that global
     // loads and stores are row-contiguous (4 lanes x 16 B per row).  Rows are 64 B apart with the
@@ -619,24 +609,13 @@ template <int MODE>
 __device__ __forceinline__ bool epilogue_unit(const CtaCtx& cx, const GemmParams& p,
                                               const CUtensorMap* tmC, const CUtensorMap* tmP, int t,
                                               int warp, int lane, int& acc, uint32_t& acc_phase) {
-  const int q = warp & 3;  // TMEM lane quarter this warp may read
-  TileCoord tc = tile_coord(p, t);
+  const TileCoord tc = tile_coord(p, t);
   {
     int kb0, nkb;
     kb_range(p, tc, kb0, nkb);
     if (nkb <= 0) return true;
   }
-  const uint32_t t_row = cx.tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)(acc * ACC_COLS);
-  const auto ready = [&]() -> bool {
-    const bool got = mbar_wait_warp(cx.tfull0 + 8 * acc, acc_phase, cx.abort_flag, p.err, 0x400u + acc);
-    tcgen05_fence_after();
-    return got;
-  };
-  const auto load = [&](int c0, uint32_t (&r)[16]) { tmem_ld16(t_row + c0, r); };
-  if (!drain_chunks<MODE>(p, tmC, tmP, tc, q, lane,
-                                     cx.epi_stage + (warp - 2) * EPI_STAGE_BYTES,
-                                     16 * ((warp - 2) >> 2), 64, p.bn, tc.n0, ready, load))
-    return false;
+  if (!drain_chunks<MODE>(cx, p, tmC, tmP, tc, warp, lane, acc, acc_phase, 0x400u)) return false;
   tcgen05_fence_before();
   __syncwarp();
   if (lane == 0) mbar_arrive(cx.tempty0 + 8 * acc);
@@ -989,24 +968,13 @@ __device__ __forceinline__ bool pair_epilogue_unit(const CtaCtx& cx, const GemmP
                                                    const CUtensorMap* tmC, const CUtensorMap* tmP, int t,
                                                    uint32_t rank, int warp, int lane, int& acc,
                                                    uint32_t& acc_phase) {
-  const int q = warp & 3;
   const TileCoord tc = tile_coord(p, t, 2 * BM, (int)rank * BM);
   {
     int kb0, nkb;
     kb_range(p, tc, kb0, nkb);
     if (nkb <= 0) return true;
   }
-  const uint32_t t_row = cx.tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)(acc * ACC_COLS);
-  const auto ready = [&]() -> bool {
-    const bool got = mbar_wait_warp(cx.tfull0 + 8 * acc, acc_phase, cx.abort_flag, p.err, 0x800u + acc);
-    tcgen05_fence_after();
-    return got;
-  };
-  const auto load = [&](int c0, uint32_t (&r)[16]) { tmem_ld16(t_row + c0, r); };
-  if (!drain_chunks<MODE>(p, tmC, tmP, tc, q, lane,
-                                     cx.epi_stage + (warp - 2) * EPI_STAGE_BYTES,
-                                     16 * ((warp - 2) >> 2), 64, p.bn, tc.n0, ready, load))
-    return false;
+  if (!drain_chunks<MODE>(cx, p, tmC, tmP, tc, warp, lane, acc, acc_phase, 0x800u)) return false;
   tcgen05_fence_before();
   __syncwarp();
   if (lane == 0) {
@@ -1241,7 +1209,9 @@ int make_out_map(vkg_device* dev, CUtensorMap* map, const void* ptr, int dtype, 
 // tiles of a CTA pair, 64 to 256 columns wide.  How many slices K is cut into is not the model's to
 // choose (k_slices): it is part of the result.  Its constants were fitted to 208 shapes (M to 50272,
 // N and K alike, aligned and ragged, the three transpositions, every epilogue of a training step;
-// launches in a graph on B200, operands warm).
+// launches in a graph on B200, operands warm).  Over 180 others (drawn M, N, K up to 16384, and the
+// GEMMs of eight models) the choice takes 0.4 % longer than the best candidate on average, 14 % at
+// worst and more than 5 % for four.
 //
 // Per k-block (64 of K), microseconds by tile width 64 / 128 / 192 / 256.  A CTA pulls its operands
 // through an L2 port of 64 bytes a cycle; K-major operands go a little faster than MN-major ones.
@@ -1280,7 +1250,8 @@ double tiles_us(const vkg_gemm_args* a, bool pair, int bn, int split, int batch,
   const double rows_a = BM, rows_b = pair ? bn / 2 : bn;
   const double ragged = ((a->lda % 64 ? rows_a : 0) + (a->ldb % 64 ? rows_b : 0)) / (rows_a + rows_b);
   const double flops = 2.0 * M * N * K * batch;
-  tk *= (1.0 + PL_RAGGED[pair] * ragged) * (1.0 + PL_HOT[pair] * (flops < PL_HOT_FLOPS ? flops / PL_HOT_FLOPS : 1.0));
+  const double hot = flops < PL_HOT_FLOPS ? flops / PL_HOT_FLOPS : 1.0;
+  tk *= (1.0 + PL_RAGGED[pair] * ragged) * (1.0 + PL_HOT[pair] * hot);
   // bytes an output element costs the epilogue, written and read; the column sums count two
   const int out = split > 1 ? 4
                             : (a->c_dtype == VKG_F32 ? 4 : 2) + (a->pre ? 4 : 0) + (a->dact_z ? 4 : 0) +
@@ -1391,15 +1362,16 @@ Tiles choose_group_tiles(vkg_device* dev, const vkg_gemm_args* args, int n, bool
         const vkg_gemm_args* a = &args[i];
         const KBlockCost& kb = a->trans_a ? KB_TN : a->trans_b ? KB_NT : KB_NN;
         const long long t = (long long)((a->M + bm - 1) / bm) * ((a->N + bn - 1) / bn);
-        const double one = (double)((a->K + BK - 1) / BK) * (kind ? kb.pair[bn / 64 - 3] : kb.single[bn / 64 - 1]) * hot +
-                           PL_WAVE;
+        const double tk = kind ? kb.pair[bn / 64 - 3] : kb.single[bn / 64 - 1];
+        const double one = (double)((a->K + BK - 1) / BK) * tk * hot + PL_WAVE;
         units += t;
         work += t * one;
         longest = one > longest ? one : longest;
       }
       if (slots < 1 || units < 1) continue;
       const long long waves = (units + slots - 1) / slots;
-      const double us = PL_LAUNCH + PL_EPI + (kind ? PL_PAIR : 0.0) + PL_EPI_COL * bn + waves * (work / units > longest * 0.99 ? longest : work / units);
+      const double wave = work / units > longest * 0.99 ? longest : work / units;
+      const double us = PL_LAUNCH + PL_EPI + (kind ? PL_PAIR : 0.0) + PL_EPI_COL * bn + waves * wave;
       if (best.us < 0 || us < best.us) best = {kind != 0, bn, 1, us};
     }
   }
@@ -1582,8 +1554,8 @@ ReduceArgs reduce_args(vkg_device* dev, const vkg_gemm_args* a, const GemmParams
 int reduce_slices(vkg_device* dev, const vkg_gemm_args* a, const GemmParams& p) {
   if (p.split_k <= 1) return 0;
   const ReduceArgs r = reduce_args(dev, a, p);
-  VKG_CUDA(vkg_launch(dev, VKG_K_SMALL | vkg_short_if((long long)r.M * r.N4 <= (1 << 18)), k_splitk_reduce, r.grid, dim3(256), 0, 1, r.ws, r.C, r.M, r.N4, r.ldc,
-                      r.splits));
+  VKG_CUDA(vkg_launch(dev, VKG_K_SMALL | vkg_short_if((long long)r.M * r.N4 <= (1 << 18)), k_splitk_reduce,
+                      r.grid, dim3(256), 0, 1, r.ws, r.C, r.M, r.N4, r.ldc, r.splits));
   return vkg_check_launch("splitk_reduce");
 }
 
@@ -1650,7 +1622,8 @@ extern "C" int vkg_gemm_group_prepare(vkg_device* dev, const vkg_gemm_args* args
   long long units = 0;
   // CTA-pair tiles (256 x 256) when asked for and every problem has more than one row block
   const bool pair_ok = cta_pair > 0 && dev->sm_count >= 2 &&
-                       std::all_of(args, args + n, [](const vkg_gemm_args& a) { return a.M > BM && a.N >= PAIR_BN / 2; });
+                       std::all_of(args, args + n,
+                                   [](const vkg_gemm_args& a) { return a.M > BM && a.N >= PAIR_BN / 2; });
   for (int i = 0; i < n; ++i)
     if (check_args(&args[i])) return 1;
   const Tiles tiles = choose_group_tiles(dev, args, n, pair_ok);
@@ -1710,7 +1683,8 @@ extern "C" int vkg_gemm_group_launch(vkg_device* dev, const void* table, int n, 
   int ctas = vkg_persistent_ctas(dev) < total_units ? vkg_persistent_ctas(dev) : total_units;
   int stages = RING_BYTES / (A_STAGE_BYTES + bn * 128);
   if (stages > MAX_STAGES) stages = MAX_STAGES;
-  VKG_CUDA(vkg_launch(dev, VKG_K_GEMM_GROUP | vkg_short_if(total_units <= ctas), gemm_group_kernel, dim3((unsigned)ctas), dim3(NUM_THREADS), SMEM_BYTES, 1,
+  VKG_CUDA(vkg_launch(dev, VKG_K_GEMM_GROUP | vkg_short_if(total_units <= ctas), gemm_group_kernel,
+                      dim3((unsigned)ctas), dim3(NUM_THREADS), SMEM_BYTES, 1,
                       static_cast<const GroupEntry*>(table), n, total_units, bn, stages));
   return vkg_check_launch("gemm_group_kernel");
 }
@@ -1740,7 +1714,8 @@ int make_plan(vkg_device* dev, const vkg_gemm_args* a, GemmPlan* out) {
   int split = a->split_k > 0 ? a->split_k : may_split(a) ? k_slices(a) : 1;
   if (a->split_k <= 0)
     while (split > 1 && (int64_t)split * a->M * a->N * 4 > a->workspace_bytes) --split;
-  const Tiles t = choose_tiles(dev, a, !pair_only, pair_ok, pair_only && a->tile_n == 0 ? PAIR_BN : a->tile_n, split);
+  const int force_bn = pair_only && a->tile_n == 0 ? PAIR_BN : a->tile_n;
+  const Tiles t = choose_tiles(dev, a, !pair_only, pair_ok, force_bn, split);
   VKG_REQUIRE(t.us >= 0, "gemm: no tile of %d columns for %d x %d x %d on %d CTAs", a->tile_n, a->M, a->N, a->K,
               a->max_ctas);
   const bool use_pair = t.pair;
@@ -1811,8 +1786,8 @@ int find_plan(vkg_device* dev, const vkg_gemm_args* a, GemmPlan* out) {
 
 int launch_plan(vkg_device* dev, const vkg_gemm_args* a, const GemmPlan& pl) {
   const Problem& q = pl.q;
-  VKG_CUDA(vkg_launch(dev, pl.family | vkg_short_if(pl.one_wave), pl.fn, dim3(pl.grid), dim3(NUM_THREADS), SMEM_BYTES, pl.cluster, q.tmA, q.tmB,
-                      q.tmC, q.tmP, q.p));
+  VKG_CUDA(vkg_launch(dev, pl.family | vkg_short_if(pl.one_wave), pl.fn, dim3(pl.grid), dim3(NUM_THREADS),
+                      SMEM_BYTES, pl.cluster, q.tmA, q.tmB, q.tmC, q.tmP, q.p));
   if (vkg_check_launch("gemm")) return 1;
   if (reduce_slices(dev, a, q.p)) return 1;
   return finish_colsum(dev, a, pl.tile_rows);

@@ -562,8 +562,8 @@ template <> struct ColVec<float> {    // 4 columns per lane
 // reads them with one 16-byte load per row (scalar loads when ncol is not a multiple
 // of N or the base is unaligned).
 template <typename T>
-__device__ __forceinline__ void col_sum_block(const T* __restrict__ g, float* __restrict__ partial, int ncol, int nrow,
-                                              int rows_per_chunk, int vec_ok, int cx, int chunk,
+__device__ __forceinline__ void col_sum_block(const T* __restrict__ g, float* __restrict__ partial, int ncol,
+                                              int nrow, int rows_per_chunk, int vec_ok, int cx, int chunk,
                                               float (*red)[32 * ColVec<T>::N + 1]) {
   constexpr int N = ColVec<T>::N;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -615,8 +615,9 @@ k_col_sum_partial(const T* __restrict__ g, float* __restrict__ partial, int ncol
 // Stage 2: fixed-order sum of the partials.  A CTA owns 32 columns; its 8 warps each
 // add every 8th chunk, then the eight slices are added in order.
 constexpr int CSF_SLICES = 8;
-__device__ __forceinline__ void col_sum_final_block(const float* __restrict__ partial, float* __restrict__ sums, int ncol,
-                                                    int nchunk, int accumulate, int cx, float (*red)[32]) {
+__device__ __forceinline__ void col_sum_final_block(const float* __restrict__ partial, float* __restrict__ sums,
+                                                    int ncol, int nchunk, int accumulate, int cx,
+                                                    float (*red)[32]) {
   const int lane = threadIdx.x & 31, slice = threadIdx.x >> 5;
   const int c = cx * 32 + lane;
   float s = 0.f;
@@ -655,7 +656,8 @@ struct ColSumJobs {
   ColSumJob e[CSM_MAX];
 };
 
-__global__ void __launch_bounds__(CS_WARPS * 32) k_col_sum_partial_multi(const __grid_constant__ ColSumJobs jobs) {
+__global__ void __launch_bounds__(CS_WARPS * 32)
+k_col_sum_partial_multi(const __grid_constant__ ColSumJobs jobs) {
   __shared__ float red[CS_WARPS][32 * ColVec<__half>::N + 1];
   pdl_trigger();
   pdl_wait();
@@ -670,7 +672,8 @@ __global__ void __launch_bounds__(CS_WARPS * 32) k_col_sum_partial_multi(const _
                          reinterpret_cast<float(*)[32 * ColVec<float>::N + 1]>(red));
 }
 
-__global__ void __launch_bounds__(32 * CSF_SLICES) k_col_sum_final_multi(const __grid_constant__ ColSumJobs jobs) {
+__global__ void __launch_bounds__(32 * CSF_SLICES)
+k_col_sum_final_multi(const __grid_constant__ ColSumJobs jobs) {
   __shared__ float red[CSF_SLICES][32];
   pdl_trigger();
   pdl_wait();
@@ -1384,7 +1387,8 @@ k_attn_softmax_bwd_reg(const float* __restrict__ dp, const __half* __restrict__ 
     if (32 * g >= jend) break;
 #pragma unroll
     for (int i = g; i < g + 4; ++i)
-      if (lane + 32 * i < jend) ds16[base + 32 * i] = __float2half_rn(32 * i <= last ? p[i] * (d[i] - dot) * scale : 0.f);
+      if (lane + 32 * i < jend)
+        ds16[base + 32 * i] = __float2half_rn(32 * i <= last ? p[i] * (d[i] - dot) * scale : 0.f);
   }
 }
 
@@ -1851,7 +1855,7 @@ extern "C" int vkg_finals_flush(vkg_device* dev) {
       blocks += vec ? (en.W + 127) / 128 : (en.W + 31) / 32;
       tab.e[tab.n++] = en;
     }
-    VKG_CUDA(vkg_launch(dev, VKG_K_SMALL | VKG_SHORT, k_finals_multi, dim3((unsigned)blocks), dim3(32 * FIN_SLICES), 0, 1, tab));
+    VKG_RUN(VKG_K_SMALL, true, k_finals_multi, dim3((unsigned)blocks), 32 * FIN_SLICES, tab);
     if (vkg_check_launch("finals_multi")) return 1;
   }
   return 0;
@@ -1957,8 +1961,9 @@ extern "C" int vkg_softmax_ce(vkg_device* dev, const float* logits, const uint32
   }
   if (stride <= 1024) {
 #define VKG_CE(NV)                                                                                          \
-  VKG_RUN(VKG_K_CE, (int64_t)rows * stride <= SHORT_ELEMS, k_softmax_ce_warp<NV>, dim3((unsigned)((rows + 3) / 4)), 128, \
-          logits, labels, w, (__half*)dl16, dl32, loss, rows, stride, ncls, grad_scale)
+  VKG_RUN(VKG_K_CE, (int64_t)rows * stride <= SHORT_ELEMS, k_softmax_ce_warp<NV>,                           \
+          dim3((unsigned)((rows + 3) / 4)), 128, logits, labels, w, (__half*)dl16, dl32, loss, rows,        \
+          stride, ncls, grad_scale)
     if (stride <= 32) VKG_CE(1);
     else if (stride <= 64) VKG_CE(2);
     else if (stride <= 128) VKG_CE(4);
@@ -2151,9 +2156,9 @@ extern "C" int vkg_layernorm(vkg_device* dev, const float* x, const float* gamma
                        (((uintptr_t)y16 & 7) == 0);
   if (aligned && D % 128 == 0 && D <= 1024) {
     const unsigned grid = (rows + wpb - 1) / wpb;
-#define VKG_LN(NV) \
-  VKG_CUDA(vkg_launch(dev, VKG_K_LN | vkg_short_if((int64_t)rows * D <= SHORT_ROWS), k_layernorm_vec<NV>, dim3(grid), dim3(wpb * 32), 0, 1, x, gamma, beta, \
-                      (__half*)y16, mu, rstd, rows))
+#define VKG_LN(NV)                                                                                                \
+  VKG_RUN(VKG_K_LN, (int64_t)rows * D <= SHORT_ROWS, k_layernorm_vec<NV>, dim3(grid), wpb * 32, x, gamma, beta, \
+          (__half*)y16, mu, rstd, rows)
     switch (D / 128) {
       case 1: VKG_LN(1); break;
       case 2: VKG_LN(2); break;
@@ -2190,8 +2195,9 @@ static void launch_ln_bwd_vec(vkg_device* dev, int nblocks, const float* dy, con
                               const float* dres, float* dx, void* dx16, float* scratch, int rows,
                               int nparts) {
   // a failed launch is picked up by the caller's vkg_check_launch
-  vkg_launch(dev, VKG_K_LN_BWD | vkg_short_if((int64_t)rows * NV * 128 <= SHORT_ROWS), k_layernorm_bwd_vec<NV>, dim3((unsigned)nblocks), dim3(LNV_WARPS * 32), 0, 1, dy, x,
-             gamma, mu, rstd, dres, dx, (__half*)dx16, scratch, rows, nparts);
+  vkg_launch(dev, VKG_K_LN_BWD | vkg_short_if((int64_t)rows * NV * 128 <= SHORT_ROWS), k_layernorm_bwd_vec<NV>,
+             dim3((unsigned)nblocks), dim3(LNV_WARPS * 32), 0, 1, dy, x, gamma, mu, rstd, dres, dx, (__half*)dx16,
+             scratch, rows, nparts);
 }
 
 extern "C" int vkg_layernorm_bwd(vkg_device* dev, const float* dy, const float* x, const float* gamma,
@@ -2280,7 +2286,8 @@ extern "C" int vkg_attn_softmax(vkg_device* dev, const float* s, const uint32_t*
   if (T <= 1024 && rows % T == 0 && rows / T < (1ll << 31)) {
 #define VKG_SM(NV)                                                                                          \
   VKG_RUN(VKG_K_SMALL, rows * T <= SHORT_ELEMS, k_attn_softmax_reg<NV>,                                     \
-          dim3((unsigned)(rows / T), (unsigned)((T + 7) / 8)), 256, s, seg, (__half*)p16, T, H > 0 ? H : 1, scale, fill_block)
+          dim3((unsigned)(rows / T), (unsigned)((T + 7) / 8)), 256, s, seg, (__half*)p16, T, H > 0 ? H : 1, \
+          scale, fill_block)
     if (T <= 128) VKG_SM(4);
     else if (T <= 256) VKG_SM(8);
     else if (T <= 512) VKG_SM(16);
@@ -2299,10 +2306,10 @@ extern "C" int vkg_attn_softmax_bwd(vkg_device* dev, const float* dp, const void
   VKG_REQUIRE(dp && p16 && ds16 && rows > 0 && T > 0, "attn_softmax_bwd: bad arguments");
   const int wpb = 8;
   if (T <= 1024 && rows % T == 0 && rows / T < (1ll << 31)) {
-#define VKG_SM(NV)                                                                                              \
-  VKG_RUN(VKG_K_SMALL, rows * T <= SHORT_ELEMS, k_attn_softmax_bwd_reg<NV>,                                     \
-          dim3((unsigned)(rows / T), (unsigned)((T + 7) / 8)), 256, dp, (const __half*)p16, (__half*)ds16, T, scale,     \
-          fill_block)
+#define VKG_SM(NV)                                                                                          \
+  VKG_RUN(VKG_K_SMALL, rows * T <= SHORT_ELEMS, k_attn_softmax_bwd_reg<NV>,                                 \
+          dim3((unsigned)(rows / T), (unsigned)((T + 7) / 8)), 256, dp, (const __half*)p16, (__half*)ds16,  \
+          T, scale, fill_block)
     if (T <= 128) VKG_SM(4);
     else if (T <= 256) VKG_SM(8);
     else if (T <= 512) VKG_SM(16);
@@ -2383,8 +2390,8 @@ extern "C" int vkg_embed(vkg_device* dev, const float* tok, const float* pos, co
   if (vkg_bind(dev)) return 1;
   VKG_REQUIRE(tok && pos && ids && x && n > 0, "embed: bad arguments");
   if (D % 4 == 0 && n < (1ll << 31) && ((((uintptr_t)tok | (uintptr_t)pos | (uintptr_t)x) & 15) == 0)) {
-    VKG_CUDA(vkg_launch(dev, VKG_K_SMALL | vkg_short_if(n <= SHORT_ROWS), k_embed_v4, dim3(flat_grid(dev, n / 4)), dim3(TPB), 0, 1, (const float4*)tok,
-                        (const float4*)pos, ids, seg, (float4*)x, (int)(n / 4), D / 4, T));
+    VKG_RUN(VKG_K_SMALL, n <= SHORT_ROWS, k_embed_v4, dim3(flat_grid(dev, n / 4)), TPB, (const float4*)tok,
+            (const float4*)pos, ids, seg, (float4*)x, (int)(n / 4), D / 4, T);
     return vkg_check_launch("embed_v4");
   }
   k_embed<<<flat_grid(dev, n), TPB, 0, dev->stream>>>(tok, pos, ids, seg, x, n, D, T);
@@ -2407,8 +2414,8 @@ extern "C" int vkg_embed_bwd(vkg_device* dev, const float* dx, const uint32_t* i
   if (vkg_bind(dev)) return 1;
   VKG_REQUIRE(dx && ids && dtok && dpos && n > 0, "embed_bwd: bad arguments");
   if (D % 4 == 0 && n < (1ll << 31) && ((((uintptr_t)dx | (uintptr_t)dtok | (uintptr_t)dpos) & 15) == 0)) {
-    VKG_CUDA(vkg_launch(dev, VKG_K_SMALL | vkg_short_if(n <= SHORT_ROWS), k_embed_bwd_v4, dim3(flat_grid(dev, n / 4)), dim3(TPB), 0, 1,
-                        (const float4*)dx, ids, seg, (float4*)dtok, (float4*)dpos, (int)(n / 4), D / 4, T));
+    VKG_RUN(VKG_K_SMALL, n <= SHORT_ROWS, k_embed_bwd_v4, dim3(flat_grid(dev, n / 4)), TPB, (const float4*)dx, ids,
+            seg, (float4*)dtok, (float4*)dpos, (int)(n / 4), D / 4, T);
     return vkg_check_launch("embed_bwd_v4");
   }
   k_embed_bwd<<<flat_grid(dev, n), TPB, 0, dev->stream>>>(dx, ids, seg, dtok, dpos, n, D, T);
@@ -2434,11 +2441,11 @@ extern "C" int vkg_embed_bwd_det(vkg_device* dev, const float* dx, const uint32_
   int* keys = static_cast<int*>(scratch);
   int* next = keys + 2 * (size_t)rows_p;
   int* has_prev = next + 2 * (size_t)rows;
-  VKG_CUDA(vkg_launch(dev, VKG_K_SMALL | vkg_short_if(n <= SHORT_ROWS), k_embed_keys, dim3((unsigned)((2 * rows_p + 255) / 256)),
-                      dim3(256), 0, 1, ids, seg, keys, has_prev, rows, rows_p, T));
+  VKG_RUN(VKG_K_SMALL, n <= SHORT_ROWS, k_embed_keys, dim3((unsigned)((2 * rows_p + 255) / 256)), 256, ids, seg,
+          keys, has_prev, rows, rows_p, T);
   if (vkg_check_launch("embed_keys")) return 1;
-  VKG_CUDA(vkg_launch(dev, VKG_K_SMALL | vkg_short_if(n <= SHORT_ROWS), k_embed_chain, dim3((unsigned)((2 * rows + 7) / 8)), dim3(256), 0,
-                      1, (const int*)keys, next, has_prev, rows, rows_p));
+  VKG_RUN(VKG_K_SMALL, n <= SHORT_ROWS, k_embed_chain, dim3((unsigned)((2 * rows + 7) / 8)), 256, keys, next,
+          has_prev, rows, rows_p);
   if (vkg_check_launch("embed_chain")) return 1;
   const dim3 grid((unsigned)((rows + 7) / 8), 2);
 #define VKG_EB(NV)                                                                            \

@@ -536,7 +536,8 @@ extern "C" int vkg_memset0(vkg_device* dev, void* dptr, size_t bytes) {
   if (vkg_bind(dev)) return 1;
   if (bytes > 0 && bytes <= ZERO_KERNEL_MAX && ((bytes | (uintptr_t)dptr) & 15) == 0) {
     const int n = (int)(bytes / 16);
-    VKG_CUDA(vkg_launch(dev, VKG_K_SMALL | VKG_SHORT, k_zero, dim3((n + 255) / 256), dim3(256), 0, 1, (uint4*)dptr, n));
+    VKG_CUDA(vkg_launch(dev, VKG_K_SMALL | VKG_SHORT, k_zero, dim3((n + 255) / 256), dim3(256), 0, 1,
+                        (uint4*)dptr, n));
     return vkg_check_launch("zero");
   }
   VKG_CUDA(cudaMemsetAsync(dptr, 0, bytes, dev->stream));

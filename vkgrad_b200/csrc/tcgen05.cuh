@@ -319,10 +319,6 @@ __device__ __forceinline__ void bulk_commit_group() {
 }
 // the issuing thread's bulk stores have finished READING shared memory (it may be reused);
 // their global writes complete on their own, at the latest when the kernel ends
-template <int PENDING>
-__device__ __forceinline__ void bulk_wait_read() {
-  asm volatile("cp.async.bulk.wait_group.read %0;" ::"n"(PENDING) : "memory");
-}
 __device__ __forceinline__ void bulk_wait_read_all() {
   asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
 }

@@ -485,8 +485,8 @@ class GPT:
         return out
 
     def forward(self, ids_buf, graph=None, seg=None, keep=True):
-        """Logits (rows, pad_vocab) fp32; keep=False when no backward will follow.  seg: optional (B*T,) u32, the index in its
-        row where each token's packed sample starts.  graph: a Graph, None for
+        """Logits (rows, pad_vocab) fp32; keep=False when no backward will follow.  seg: optional
+        (B*T,) u32, the index in its row where each token's packed sample starts.  graph: a Graph, None for
         eager, or a stage -> Graph callable (see record)."""
         c = self.ctx
         g = graph if callable(graph) else (lambda stage: graph)
