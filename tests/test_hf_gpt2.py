@@ -274,3 +274,22 @@ def test_forward_without_memory_to_pin(dev):
         assert all(pool._state["n"] == 0 for pool in fwd.pools.values())
     finally:
         ctx.destroy()
+
+
+@pytest.mark.gpu
+def test_forward_of_a_wide_model_with_few_words(dev):
+    """The tied head's K is cut where a small vocabulary meets a wide model, at some numbers of rows
+    and not at others: the logits are those of the full length all the same."""
+    from vkgrad_b200.kernels import k_slices
+    from vkgrad_b200.transformer import GPT, TCtx
+    assert k_slices(dev, 256, 256, 1024) > 1 == k_slices(dev, 128, 256, 1024)
+    ctx = TCtx(dev)
+    try:
+        fwd = hf_gpt2.Forward(GPT(ctx, 1, 256, 1024, 16, 1, 250, tie=True))
+        ids = np.random.default_rng(3).integers(0, 250, (1, 256))
+        full = fwd(ids)
+        assert np.array_equal(fwd(ids, last=True), full[:, 255])
+        assert np.array_equal(fwd(ids[:, :100]), full[:, :100])
+        assert np.array_equal(fwd(ids[:, :100], last=True), full[:, 99])
+    finally:
+        ctx.destroy()

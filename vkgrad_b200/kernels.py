@@ -108,8 +108,10 @@ def _gemm_args(dev, a, b, c, m, n, k, trans_a=False, trans_b=False,
 
 
 def k_slices(dev, m, n, k):
-    """How many slices the library cuts K into for a plain fp32 output (1: whole), by its rule of
-    m, n and k."""
+    """How many slices gemm() cuts K into for a plain fp32 output (1: whole): the library's rule of
+    m, n and k, where it is given a workspace."""
+    if m * n * 4 > SPLIT_K_MAX_TILE_BYTES:
+        return 1
     args = GemmArgs(M=m, N=n, K=k, ldc=n, C=16, c_dtype=F32)
     return max(dev.lib.vkg_gemm_workspace_bytes(C.byref(args)) // (4 * m * n), 1)
 

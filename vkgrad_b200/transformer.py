@@ -31,7 +31,7 @@ import numpy as np
 
 from ._lib import ACT_GELU, ACT_NONE, F16, F32, TUNE_SM_LIMIT
 from .autograd import Ctx, Param, mean32
-from .kernels import gemm, gemm_group
+from .kernels import gemm, gemm_group, k_slices
 from .tkernels import make_transformer_kernels
 from .vk import _check
 
@@ -480,9 +480,14 @@ class GPT:
         dense(h16, b.fc2, x, residual=res)
         c.launch(graph, lambda: norm(x, self.lnf), "layernorm", B * D * 6)
         W, bias = (self.tok.w16, None) if self.tie else (self.head.W.w16, self.head.b.w32)
-        gemm(c.dev, y16, W, out, B, V, D, trans_b=self.tie, bias=bias, split_k=1, graph=graph,
-             name="head.rows")
+        gemm(c.dev, y16, W, out, B, V, D, trans_b=self.tie, bias=bias, graph=graph,
+             split_k=self._head_slices() if self.tie else 1, name="head.rows")
         return out
+
+    def _head_slices(self):
+        """K slices of the tied head's product over all B x T rows the model was made for: a pass
+        over fewer of them (at_length, forward_rows) adds up in the same order."""
+        return k_slices(self.ctx.dev, self.B * self.pos.shape[0], self.pad_vocab, self.D)
 
     def forward(self, ids_buf, graph=None, seg=None, keep=True):
         """Logits (rows, pad_vocab) fp32; keep=False when no backward will follow.  seg: optional
@@ -498,7 +503,7 @@ class GPT:
         if self.tie:
             # logits = h tok^T; tok is stored V x D, hence trans_b
             gemm(c.dev, hf, self.tok.w16, self.logits, R, V, D, trans_b=True, graph=g(L),
-                 name="head.fwd")
+                 split_k=self._head_slices(), name="head.fwd")
         else:
             self.head.forward(hf, graph=g(L), out=self.logits)
         return self.logits
