@@ -341,8 +341,9 @@ class MLP:
     def _groups_dw(self):
         """Whether a recorded backward runs the dW of all layers in one launch (784-256-256-16 at
         256 rows 14.5 -> 5.7 us).  A group's tiles take K, the batch, whole, so it is for batches
-        that no layer's own launch would cut: the sums are then the same."""
-        return all(l.in_f % 8 == 0 and l.out_f % 8 == 0
+        that no layer's own launch would cut: the sums are then the same.  It also wants whole
+        16-byte rows, which gradients moved into a buffer of the caller's need not have."""
+        return all(l.in_f % 8 == 0 and l.out_f % 8 == 0 and l.W.g32.dptr % 16 == 0
                    and k_slices(self.ctx.dev, l.in_f, l.out_f, self.batch) == 1 for l in self.layers)
 
     def _backward(self, graph):
