@@ -224,7 +224,8 @@ class Matmul:
             # the argument block depends on nothing but these values; a destroyed buffer has no
             # address and is caught below.  Building it and the closures around it took 7 us of
             # a 29 us call whose kernel runs for 5.
-            key = (a.dptr, a.kind, b.dptr, b.kind, c.dptr, m, n, k, nbatch, tuple(strides), self.tile_n)
+            key = (a.dptr, a.kind, b.dptr, b.kind, c.dptr, m, n, k, nbatch, tuple(strides), self.tile_n,
+                   self.acc16, self.in_dtype, self.trans_a, self.trans_b, self.batched)
             args = self._calls.get(key)
             if args is not None:
                 return _run(self.dev, args, repeat, self.name)
