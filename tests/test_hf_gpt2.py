@@ -293,3 +293,22 @@ def test_forward_of_a_wide_model_with_few_words(dev):
         assert np.array_equal(fwd(ids[:, :100], last=True), full[:, 99])
     finally:
         ctx.destroy()
+
+
+@pytest.mark.gpu
+def test_recorded_passes_go_with_the_forward_object(dev):
+    """Each length of prompt has its own; the full-length one stays the caller's."""
+    from vkgrad_b200.transformer import GPT, TCtx
+    ctx = TCtx(dev)
+    try:
+        fwd = hf_gpt2.Forward(GPT(ctx, 1, 384, 128, 2, 1, 250, tie=True))
+        for n in (5, 130, 384):
+            fwd(np.zeros((1, n), np.int64), last=n > 100)
+        graphs, first = list(fwd.graphs.values()), fwd.graph
+        assert len(graphs) == 4
+        del fwd
+        assert [g._handle is None for g in graphs] == [g is not first for g in graphs]
+        first.submit()
+        first.destroy()
+    finally:
+        ctx.destroy()

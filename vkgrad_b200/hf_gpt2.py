@@ -17,6 +17,7 @@ x @ weight + bias, exactly what Dense does with W (in_f, out_f): nothing is tran
 import json
 import os
 import struct
+import weakref
 
 import numpy as np
 
@@ -208,7 +209,15 @@ class Forward:
         self.graphs, self.last_out = {}, None
         self.out = model.logits
         self.graph = self._graph(model.T, False)
+        # the passes recorded on the way go with the object; `graph` is the caller's to destroy
+        weakref.finalize(self, self._drop, self.graphs, self.graph).atexit = False
         self.submit_s = self.copy_s = 0.0
+
+    @staticmethod
+    def _drop(graphs, kept):
+        for g in graphs.values():
+            if g is not kept:
+                g.destroy()
 
     def _graph(self, T, last):
         """The pass over B rows of T positions, recorded on first use."""
