@@ -41,12 +41,6 @@ constexpr int FA_HD = 64;          // head dimension
 constexpr int FA_TILE_BYTES = FA_T * FA_HD * 2;  // 16 KB: one 128 x 64 fp16 tile, 128 B rows
 constexpr int FA_THREADS = 320;      // producer + MMA + eight softmax warps
 constexpr int FA_SOFTMAX_WARPS = 8;
-constexpr int BW_SOFTMAX_WARPS = 16;   // dK / dV kernel: four warps per TMEM lane quarter, 32 keys of a row each
-constexpr int DQ_SOFTMAX_WARPS = 16;   // dQ kernel: 8 or 16 (2 or 4 per lane quarter; 8 measured 2 % slower)
-constexpr int DQ_MMA2_WARP = 2 + DQ_SOFTMAX_WARPS;        // the warp that issues dQ += dS K
-constexpr int DQ_THREADS = (3 + DQ_SOFTMAX_WARPS) * 32;
-constexpr int KV_MMA2_WARP = 2 + BW_SOFTMAX_WARPS;        // the warp that issues dV / dK
-constexpr int BW_THREADS = (3 + BW_SOFTMAX_WARPS) * 32;
 constexpr float LOG2E = 1.4426950408889634f;
 // The softmax warps' waits suspend (mbarrier.try_wait with a time hint); the producer's and the
 // MMA warps', which sit on the critical chain, poll.  Polling in the softmax warps too measured
@@ -396,7 +390,15 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm, const AttnParams p) {
 // partner.  The rescale sits between "P V of the previous tile has retired" (the wait that
 // guards the P buffer anyway) and this warp's arrival on p_full, so it needs no barrier of its
 // own: O~ is quiet exactly there.
+// P~ in tensor memory leaves shared memory for three stages of K and two of V.  With two and one, a
+// single V stage made every load (0.8 us) wait for the product before it, and the producer, which
+// issues loads in order, held K of the next tile behind that V: a tile took load + product, 1.45 us,
+// wherever one CTA has an SM to itself.
 constexpr float FW1_LAZY = 8.0f;      // log2 of the largest P~ the running reference allows
+constexpr int F1_K_STAGES = 3, F1_V_STAGES = 2;
+constexpr int F1_K = FW_K, F1_V = F1_K + F1_K_STAGES * FA_TILE_BYTES;
+constexpr int F1_OUT = F1_V;          // output staging, once every product has retired
+static_assert(F1_V + F1_V_STAGES * FA_TILE_BYTES <= FW_BAR, "one-pass forward: shared memory");
 
 __global__ void __launch_bounds__(FA_THREADS, 2)
 attn_fwd1_kernel(const __grid_constant__ CUtensorMap tm, const AttnParams p) {
@@ -404,7 +406,7 @@ attn_fwd1_kernel(const __grid_constant__ CUtensorMap tm, const AttnParams p) {
   const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
   uint8_t* gbase = smem_raw + (base - smem_u32(smem_raw));
   const uint32_t bar = base + FW_BAR;
-  // barriers: 0 q_full, 1-2 k_full, 3-4 k_empty, 5 v_full, 6 v_empty, 7 s_full, 8 s_free,
+  // barriers: 0 q_full, 1-2 v_full, 3-4 v_empty, 5-7 k_full, 12-14 k_empty, 15 s_full, 8 s_free,
   //           9 p_full, 10 p_free, 11 o_full
   auto B_ = [bar](int i) { return bar + 8u * i; };
   volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(gbase + FW_BAR + 128);
@@ -424,7 +426,7 @@ attn_fwd1_kernel(const __grid_constant__ CUtensorMap tm, const AttnParams p) {
   pdl_trigger();
   if (threadIdx.x == 0) {
     prefetch_tensormap(&tm);
-    for (int i = 0; i < 12; ++i) mbar_init(B_(i), (i == 8 || i == 9) ? FA_SOFTMAX_WARPS : 1);
+    for (int i = 0; i < 16; ++i) mbar_init(B_(i), (i == 8 || i == 9) ? FA_SOFTMAX_WARPS : 1);
     *abort_flag = 0u;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
@@ -442,14 +444,20 @@ attn_fwd1_kernel(const __grid_constant__ CUtensorMap tm, const AttnParams p) {
     if (lane == 0) {
       mbar_expect_tx(B_(0), FA_TILE_BYTES);
       tma_load_2d(base + FW_Q, &tm, B_(0), h * FA_HD, row0 + q0);
+      int ks = 0;
+      uint32_t kph = 0;
       for (int j = 0; j < nj; ++j) {
-        const int s = j & 1;
-        if (!mbar_wait<true>(B_(3 + s), ((j >> 1) & 1) ^ 1u, abort_flag, p.err, 0x6100u + s)) break;
-        mbar_expect_tx(B_(1 + s), FA_TILE_BYTES);
-        tma_load_2d(base + FW_K + s * FA_TILE_BYTES, &tm, B_(1 + s), p.D + h * FA_HD, row0 + j * FA_T);
-        if (!mbar_wait<true>(B_(6), (j & 1) ^ 1u, abort_flag, p.err, 0x6200u)) break;
-        mbar_expect_tx(B_(5), FA_TILE_BYTES);
-        tma_load_2d(base + FW_V, &tm, B_(5), 2 * p.D + h * FA_HD, row0 + j * FA_T);
+        if (!mbar_wait<true>(B_(12 + ks), kph ^ 1u, abort_flag, p.err, 0x6100u + ks)) break;
+        mbar_expect_tx(B_(5 + ks), FA_TILE_BYTES);
+        tma_load_2d(base + F1_K + ks * FA_TILE_BYTES, &tm, B_(5 + ks), p.D + h * FA_HD, row0 + j * FA_T);
+        if (++ks == F1_K_STAGES) {
+          ks = 0;
+          kph ^= 1u;
+        }
+        const int vs = j & 1;
+        if (!mbar_wait<true>(B_(3 + vs), ((j >> 1) & 1) ^ 1u, abort_flag, p.err, 0x6200u + vs)) break;
+        mbar_expect_tx(B_(1 + vs), FA_TILE_BYTES);
+        tma_load_2d(base + F1_V + vs * FA_TILE_BYTES, &tm, B_(1 + vs), 2 * p.D + h * FA_HD, row0 + j * FA_T);
       }
     }
   } else if (warp == 1) {
@@ -459,17 +467,22 @@ attn_fwd1_kernel(const __grid_constant__ CUtensorMap tm, const AttnParams p) {
     bool ok = mbar_wait_warp<true>(B_(0), 0, abort_flag, p.err, 0x7000u);
     // descriptor halves (tcgen05.cuh): start address and leading offset in the low word
     const uint32_t d_hi = smem_desc_hi(1024);
-    const uint32_t q_lo = smem_desc_lo(base + FW_Q, 16), k_lo = smem_desc_lo(base + FW_K, 16);
-    const uint32_t v_lo = smem_desc_lo(base + FW_V, 8192);
+    const uint32_t q_lo = smem_desc_lo(base + FW_Q, 16), k_lo = smem_desc_lo(base + F1_K, 16);
+    const uint32_t v_lo = smem_desc_lo(base + F1_V, 8192);
+    int ks = 0;
+    uint32_t kph = 0;
     auto issue_s = [&](int n) -> bool {
-      const int s = n & 1;
-      if (!(mbar_wait_warp<true>(B_(1 + s), (n >> 1) & 1, abort_flag, p.err, 0x7100u + s) &&
+      if (!(mbar_wait_warp<true>(B_(5 + ks), kph, abort_flag, p.err, 0x7100u + ks) &&
             mbar_wait_warp<true>(B_(8), (n & 1) ^ 1u, abort_flag, p.err, 0x7200u)))
         return false;
       tcgen05_fence_after();
-      umma_f16_chain<4>(tS, q_lo, 2, k_lo + (uint32_t)s * (FA_TILE_BYTES >> 4), 2, d_hi, idesc_s, 0u);
-      umma_commit_one(B_(3 + s));   // K stage free once these retire
-      umma_commit_one(B_(7));       // S ready
+      umma_f16_chain<4>(tS, q_lo, 2, k_lo + (uint32_t)ks * (FA_TILE_BYTES >> 4), 2, d_hi, idesc_s, 0u);
+      umma_commit_one(B_(12 + ks));   // K stage free once these retire
+      umma_commit_one(B_(15));        // S ready
+      if (++ks == F1_K_STAGES) {
+        ks = 0;
+        kph ^= 1u;
+      }
       return true;
     };
     int n = 0;
@@ -480,12 +493,13 @@ attn_fwd1_kernel(const __grid_constant__ CUtensorMap tm, const AttnParams p) {
         if (!ok) break;
       }
       ok = mbar_wait_warp<true>(B_(9), j & 1, abort_flag, p.err, 0x7300u) &&
-           mbar_wait_warp<true>(B_(5), j & 1, abort_flag, p.err, 0x7400u);
+           mbar_wait_warp<true>(B_(1 + (j & 1)), (j >> 1) & 1, abort_flag, p.err, 0x7400u);
       if (!ok) break;
       tcgen05_fence_after();
       // P~ from tensor memory; V: MN-major, 16 keys = two 8-row groups further down
-      umma_f16_ts_chain<8>(tO, tP, v_lo, 128, d_hi, idesc_o, j ? 1u : 0u);
-      umma_commit_one(B_(6));     // V free
+      umma_f16_ts_chain<8>(tO, tP, v_lo + (uint32_t)(j & 1) * (FA_TILE_BYTES >> 4), 128, d_hi, idesc_o,
+                           j ? 1u : 0u);
+      umma_commit_one(B_(3 + (j & 1)));     // V stage free
       umma_commit_one(B_(10));    // P free, and O~ quiet until the next p_full
     }
     if (ok) umma_commit_one(B_(11));
@@ -499,7 +513,7 @@ attn_fwd1_kernel(const __grid_constant__ CUtensorMap tm, const AttnParams p) {
     float m_ref = -1e30f, l = 0.f;              // reference maximum (scaled units), row sum
     bool ok = true;
     for (int j = 0; j < nj && ok; ++j) {
-      ok = mbar_wait_warp<SM_SPIN>(B_(7), j & 1, abort_flag, p.err, 0x8100u);
+      ok = mbar_wait_warp<SM_SPIN>(B_(15), j & 1, abort_flag, p.err, 0x8100u);
       if (!ok) break;
       tcgen05_fence_after();
       const bool need_mask = (j == qt) || (p.seg != nullptr);
@@ -604,7 +618,7 @@ attn_fwd1_kernel(const __grid_constant__ CUtensorMap tm, const AttnParams p) {
       }
       const int q_w = q0 + (warp & 3) * 32;
       __half* dst = p.out + (size_t)(row0 + q_w) * p.D + h * FA_HD + half * 32;
-      warp_store_rows<4>(hv, gbase + FW_P + (warp - 2) * 2048, lane, reinterpret_cast<uint8_t*>(dst),
+      warp_store_rows<4>(hv, gbase + F1_OUT + (warp - 2) * 2048, lane, reinterpret_cast<uint8_t*>(dst),
                          (size_t)p.D * 2, p.T - q_w);
     }
   }
@@ -625,76 +639,88 @@ attn_fwd1_kernel(const __grid_constant__ CUtensorMap tm, const AttnParams p) {
 
 // ---- backward --------------------------------------------------------------------------
 //
-// One 32-key chunk of a (query row, key tile) pair: rebuild P from S and the saved
-// log-sum-exp and form dS = P (dP - delta) scale, both rounded to fp16 and packed into registers
-// (four 16-byte groups each); bwd_chunk_store writes them into the swizzled [query row][key]
-// layout once the buffer, which the tensor core may still be reading, is free.  nlse = -lse2
-// (or -inf for a row past the end of the sequence, which makes its P exactly 0), dsc = -delta *
-// scale: each element costs two FMAs, one exp2, one multiply and the conversions.  MASK adds the
-// per-element causal / packed-sample test and is only compiled into the tiles that need it.
-template <bool MASK>
-__device__ __forceinline__ void bwd_chunk_regs(const uint32_t* rs, const uint32_t* rdp, int c,
-                                               int key0, int qi, int st, float cscale, float scale,
-                                               float nlse, float dsc, uint4* outp, uint4* outd) {
+// Two persistent kernels, one CTA per SM, 24 warps each:
+//   warp 0        TMA producer
+//   warp 1        S and dP products        warp 2   the gradient products (dQ, or dV and dK)
+//   warps 4..7    epilogue: read a finished item's accumulators out, store them, fold their column
+//                 sums; in the dQ kernel also delta = rowsum(dO * O) of the item ahead
+//   warps 8..23   softmax: four per TMEM lane quarter, 32 of a tile's 128 columns each
+// The pipeline runs across items: an item's own operands have two buffers, so the next item's are
+// there when its first products are wanted, and nothing the softmax warps do depends on where an
+// item ends.  Before (single buffers, accumulators read out and delta formed by the softmax warps) an
+// item boundary cost 5000 cycles, 16 to 18 us of each kernel's 50 at 8 x 1024 tokens, 12 heads.
+// Registers: 768 threads are launched with 80 each; the softmax warps, which hold 64 scores and
+// gradients at a time, take 96 of what the other eight warps give back.
+constexpr int BW_EPI_WARP = 4, BW_EPI_WARPS = 4, BW_SM_WARP = 8, BW_SM_WARPS = 16;
+constexpr int BW_THREADS = (BW_SM_WARP + BW_SM_WARPS) * 32;
+constexpr int BW_REGS_ISSUE = 40, BW_REGS_EPI = 56, BW_REGS_SM = 96;
+static_assert(4 * (BW_REGS_ISSUE + BW_REGS_EPI) + BW_SM_WARPS * BW_REGS_SM <= (BW_SM_WARP + BW_SM_WARPS) * 80,
+              "a split above what the block was launched with would wait forever");
+
+template <int N>
+__device__ __forceinline__ void regs_less() {
+  asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(N));
+}
+template <int N>
+__device__ __forceinline__ void regs_more() {
+  asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(N));
+}
+
+// A warp's 32 rows x 8 NU accumulator columns (lane = row) as fp16 into its staging slice: rows of NU
+// 16-byte pieces, piece u of row r at u ^ (r & (NU - 1)).
+template <int NU>
+__device__ __forceinline__ void stage_acc(uint32_t taddr, uint8_t* stage, int lane) {
+#pragma unroll 1
+  for (int c = 0; c < NU / 4; ++c) {
+    uint32_t rr[32];
+    tmem_ld16(taddr + c * 32, rr);
+    tmem_ld16(taddr + c * 32 + 16, rr + 16);
+    tmem_wait_ld();
 #pragma unroll
-  for (int u = 0; u < 4; ++u) {
-    __half2 hp[4], hd[4];
+    for (int u = 0; u < 4; ++u) {
+      uint32_t w[4];
 #pragma unroll
-    for (int e = 0; e < 4; ++e) {
-      float pv[2], dv[2];
-#pragma unroll
-      for (int w = 0; w < 2; ++w) {
-        const int idx = u * 8 + 2 * e + w;
-        float pr = vkg_ex2(fmaf(__uint_as_float(rs[idx]), cscale, nlse));
-        if (MASK) {
-          const int key = key0 + c * 32 + idx;
-          if (key > qi || key < st) pr = 0.f;
-        }
-        pv[w] = pr;
-        dv[w] = pr * fmaf(__uint_as_float(rdp[idx]), scale, dsc);
+      for (int e = 0; e < 4; ++e) {
+        const __half2 h = __floats2half2_rn(__uint_as_float(rr[u * 8 + 2 * e]),
+                                            __uint_as_float(rr[u * 8 + 2 * e + 1]));
+        w[e] = *reinterpret_cast<const uint32_t*>(&h);
       }
-      hp[e] = __floats2half2_rn(pv[0], pv[1]);
-      hd[e] = __floats2half2_rn(dv[0], dv[1]);
+      *reinterpret_cast<uint4*>(stage + lane * (NU * 16) + (((c * 4 + u) ^ (lane & (NU - 1))) << 4)) =
+          make_uint4(w[0], w[1], w[2], w[3]);
     }
-    outp[u] = *reinterpret_cast<uint4*>(hp);
-    outd[u] = *reinterpret_cast<uint4*>(hd);
   }
 }
 
-__device__ __forceinline__ void bwd_chunk_store(int c, int r, const uint4* outp, const uint4* outd,
-                                                uint8_t* sp, uint8_t* sds) {
-  const uint32_t row_off = (uint32_t)(r * 128), rx = (uint32_t)(r & 7);
+// The staged slice to global rows of `pitch` bytes (32 / NU whole rows per store instruction) and, with
+// `sums`, its 8 NU column sums over the rows_ok rows that exist, as stored: NU / 4 adjacent columns per
+// lane, the rows in a fixed tree (r + r+16, then 8, 4, 2, 1 apart).
+template <int NU>
+__device__ __forceinline__ void store_staged(const uint8_t* stage, int lane, uint8_t* dst_row0, size_t pitch,
+                                             int rows_ok, float* sums) {
+  static_assert(NU == 4 || NU == 8, "32 or 64 columns");
+  const int u = lane % NU;
 #pragma unroll
-  for (int u = 0; u < 4; ++u) {
-    const int cc = c * 4 + u;
-    const uint32_t off = (uint32_t)((cc >> 3) * FA_TILE_BYTES) + row_off + ((((uint32_t)cc & 7u) ^ rx) << 4);
-    *reinterpret_cast<uint4*>(sp + off) = outp[u];
-    *reinterpret_cast<uint4*>(sds + off) = outd[u];
+  for (int i = 0; i < NU; ++i) {
+    const int row = i * (32 / NU) + lane / NU;
+    const uint4 x = *reinterpret_cast<const uint4*>(stage + row * (NU * 16) + ((u ^ (row & (NU - 1))) << 4));
+    if (row < rows_ok) *reinterpret_cast<uint4*>(dst_row0 + (size_t)row * pitch + u * 16) = x;
   }
-}
-
-// Column sums of one warp's 32 rows x NC columns (lane = row; fp16 values as stored, 0 for rows
-// that do not exist) without shared memory: a reduce-scatter over the lanes.  Each step halves
-// the columns a lane holds and adds the partner lane's share of the half it keeps, so after five
-// steps lane l holds the sums of columns l * NC / 32 .. (l + 1) * NC / 32 - 1 and writes them to
-// dst.  The order of the additions is fixed, so the result does not depend on timing.
-template <int NC>
-__device__ __forceinline__ void warp_col_sums(float (&v)[NC], int lane, float* dst) {
-  static_assert(NC == 32 || NC == 64, "one or two columns per lane");
-#pragma unroll
-  for (int step = 0; step < 5; ++step) {
-    const int off = 16 >> step, n = NC >> (step + 1);
-    const bool upper = (lane & off) != 0;
-#pragma unroll
-    for (int c = 0; c < n; ++c) {
-      const float keep = upper ? v[c + n] : v[c];
-      const float send = upper ? v[c] : v[c + n];
-      v[c] = keep + __shfl_xor_sync(0xffffffffu, send, off);
-    }
-  }
-  constexpr int PER = NC / 32;
-#pragma unroll
-  for (int c = 0; c < PER; ++c) dst[lane * PER + c] = v[c];
+  if (!sums) return;
+  // NU = 4: a lane's one column is the half of its column pair that its lowest bit names
+  const int pair = NU == 8 ? lane : lane >> 1;
+  const int piece = pair >> 2, word = (pair & 3) * 4;
+  auto at = [&](int r) -> float2 {
+    const __half2 h = *reinterpret_cast<const __half2*>(stage + r * (NU * 16) + ((piece ^ (r & (NU - 1))) << 4) + word);
+    return r < rows_ok ? __half22float2(h) : make_float2(0.f, 0.f);
+  };
+  auto add = [](float2 a, float2 b) { return make_float2(a.x + b.x, a.y + b.y); };
+  // the tree from its leaves: t8(r) covers rows r, r+16, r+8, r+24
+  auto t8 = [&](int r) { return add(add(at(r), at(r + 16)), add(at(r + 8), at(r + 24))); };
+  auto t4 = [&](int r) { return add(t8(r), t8(r + 4)); };
+  auto t2 = [&](int r) { return add(t4(r), t4(r + 2)); };
+  const float2 sum = add(t2(0), t2(1));
+  if (NU == 8) *reinterpret_cast<float2*>(sums + 2 * lane) = sum;
+  else sums[lane] = (lane & 1) ? sum.y : sum.x;
 }
 
 // Item number j of persistent CTA c out of G: rows of G items are dealt left to right and right
@@ -704,30 +730,56 @@ __device__ __forceinline__ int snake_item(int j, int G, int c) {
   return j * G + ((j & 1) ? G - 1 - c : c);
 }
 
-// dK / dV: persistent CTAs, one per SM, each taking (key tile, head, sequence) items
-// blockIdx.x, blockIdx.x + gridDim.x, ... (items are ordered heaviest key tile first) and, per
-// item, looping over the query tiles at or below the diagonal.  The pipeline runs across item
-// boundaries: barrier phases follow a per-CTA count of (item, query tile) steps, the producer
-// reloads K / V as soon as the item's last S / dP products have retired (kv_free) and the tensor
-// core starts the next item's first S / dP before this item's last dV / dK, so a CTA pays the
-// load -> S -> softmax -> dV latency chain once per launch instead of once per item (measured
-// at 5.6 us per item when every item was its own CTA).  The accumulators are handed back by the
-// softmax warps (acc_free) before the next item's first dV / dK overwrites them.
-// TMEM: S [0,128) dP [128,256) dV [256,320) dK [320,384).
-// Q / dO go through a ring of three stages and P / dS have ONE buffer.  A Q / dO stage is read
-// by S / dP of its step and again by dV / dK of the same step a softmax later; with two stages
-// (and P / dS double-buffered, which is what the shared memory then allowed) the load of step
-// g + 1 waited for dV / dK of step g - 1 and the chain dV / dK -> load -> S / dP set the pace:
-// 2.25 us per step measured against 1.45 us of tensor work.  With one P / dS buffer the softmax
-// warps form the next step's P / dS in registers while the tensor core still reads the buffer
-// for dV / dK, and only their stores wait for it.
+// dK / dV: an item is a (key tile, head, sequence), heaviest key tile first, and loops over the query
+// tiles at or below the diagonal.  The scores are formed transposed, S^T = K Q^T and dP^T = V dO^T
+// (TMEM lane = key, column = query), so that P^T and dS^T, which dV += P^T dO and dK += dS^T Q want as
+// A operands, go back into tensor memory (fp16 pairs of queries) and never through shared memory:
+// writing both there (64 KB a step beside the tensor core's own reads of it) took 670 of a step's
+// 2150 cycles.  lse and delta then belong to columns: a warp keeps those of its 32 queries in 256
+// bytes of shared memory, read as broadcasts.
+// TMEM columns: S^T [0, 128) dP^T [128, 256) dV [256, 320) dK [320, 384) P^T [384, 448) dS^T [448, 512).
 constexpr int KV_STAGES = 3;
-constexpr int KV_K = 0, KV_V = FA_TILE_BYTES, KV_Q = 2 * FA_TILE_BYTES,
-              KV_DO = (2 + KV_STAGES) * FA_TILE_BYTES, KV_P = (2 + 2 * KV_STAGES) * FA_TILE_BYTES,
-              KV_DS = KV_P + 2 * FA_TILE_BYTES, KV_OUT = KV_DS + 2 * FA_TILE_BYTES,   // output staging
-              KV_BAR = KV_OUT + 2 * FA_TILE_BYTES, KV_SMEM = KV_BAR + 256 + 1024;
-constexpr int KV_NBAR = 14 + 2 * KV_STAGES, KV_QD_FULL = 14, KV_QD_EMPTY = 14 + KV_STAGES;
+constexpr int KV_K = 0,                                        // two buffers of K and V
+              KV_Q = 4 * FA_TILE_BYTES, KV_DO = (4 + KV_STAGES) * FA_TILE_BYTES,
+              KV_OUT = (4 + 2 * KV_STAGES) * FA_TILE_BYTES,    // staging: dV and dK of 32 keys per epilogue warp
+              KV_STAT = KV_OUT + BW_EPI_WARPS * 8192,          // (-lse, -delta scale) of 32 queries per softmax warp
+              KV_SEG = KV_STAT + BW_SM_WARPS * 256,            // and where their samples start
+              KV_BAR = KV_SEG + BW_SM_WARPS * 128, KV_SMEM = KV_BAR + 256 + 1024;
 static_assert(KV_SMEM <= 227 * 1024, "dK / dV kernel: shared memory");
+constexpr int KV_KV_FULL = 0, KV_KV_FREE = 2, KV_SDP_FULL = 4, KV_SDP_FREE = 5, KV_PDS_FULL = 6, KV_PDS_FREE = 7,
+              KV_OUT_FULL = 8, KV_ACC_FREE = 9, KV_QD_FULL = 10, KV_QD_EMPTY = 10 + KV_STAGES,
+              KV_NBAR = 10 + 2 * KV_STAGES;
+
+// P and dS = P (dP - delta) scale of one key row against 16 queries, as fp16 pairs (queries 2i, 2i + 1)
+// in pp[i] and pd[i], ready for tcgen05.st.  P is rebuilt from the saved log-sum-exp; stat holds
+// (-lse2, -delta scale) per query, -lse2 = -inf for a query past the end of the sequence, which makes
+// its P exactly 0: an element costs two FMAs, one exp2, one multiply and the conversions.  The
+// per-element tests, MASK = 1 causal, 2 packed samples too, are only compiled into the tiles that need
+// them.
+template <int MASK>
+__device__ __forceinline__ void bwd_pds_pack(const uint32_t* rs, const uint32_t* rdp, const float4* stat,
+                                             const int* seg, int q0, int key, float cscale, float scale,
+                                             uint32_t* pp, uint32_t* pd) {
+#pragma unroll
+  for (int i = 0; i < 8; ++i) {
+    const float4 s2 = stat[i];
+    const float nlse[2] = {s2.x, s2.z}, dsc[2] = {s2.y, s2.w};
+    float pv[2], dv[2];
+#pragma unroll
+    for (int w = 0; w < 2; ++w) {
+      const int idx = 2 * i + w;
+      float pr = vkg_ex2(fmaf(__uint_as_float(rs[idx]), cscale, nlse[w]));
+      if (MASK) {
+        if (key > q0 + idx || (MASK == 2 && key < seg[idx])) pr = 0.f;
+      }
+      pv[w] = pr;
+      dv[w] = pr * fmaf(__uint_as_float(rdp[idx]), scale, dsc[w]);
+    }
+    const __half2 hp = __floats2half2_rn(pv[0], pv[1]), hd = __floats2half2_rn(dv[0], dv[1]);
+    pp[i] = *reinterpret_cast<const uint32_t*>(&hp);
+    pd[i] = *reinterpret_cast<const uint32_t*>(&hd);
+  }
+}
 
 __global__ void __launch_bounds__(BW_THREADS, 1)
 attn_bwd_kv_kernel(const __grid_constant__ CUtensorMap tm, const __grid_constant__ CUtensorMap tmdo,
@@ -736,8 +788,6 @@ attn_bwd_kv_kernel(const __grid_constant__ CUtensorMap tm, const __grid_constant
   const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
   uint8_t* gbase = smem_raw + (base - smem_u32(smem_raw));
   const uint32_t bar = base + KV_BAR;
-  // 0 kv_full, 5 sdp_full, 6 sdp_free, 7 pds_full, 8 pds_free, 9 out_full, 12 kv_free,
-  // 13 acc_free, 14.. qd_full[stage], then qd_empty[stage]
   auto B_ = [bar](int i) { return bar + 8u * i; };
   volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(gbase + KV_BAR + 192);
   volatile uint32_t* abort_flag = reinterpret_cast<volatile uint32_t*>(gbase + KV_BAR + 200);
@@ -750,7 +800,7 @@ attn_bwd_kv_kernel(const __grid_constant__ CUtensorMap tm, const __grid_constant
     prefetch_tensormap(&tm);
     prefetch_tensormap(&tmdo);
     for (int i = 0; i < KV_NBAR; ++i)
-      mbar_init(B_(i), (i == 6 || i == 7 || i == 13) ? BW_SOFTMAX_WARPS : 1);
+      mbar_init(B_(i), i == KV_SDP_FREE || i == KV_PDS_FULL ? BW_SM_WARPS : i == KV_ACC_FREE ? BW_EPI_WARPS : 1);
     *abort_flag = 0u;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
@@ -761,207 +811,185 @@ attn_bwd_kv_kernel(const __grid_constant__ CUtensorMap tm, const __grid_constant
   tcgen05_fence_after();
   pdl_wait();
   const uint32_t tmem = *tmem_slot;
-  const uint32_t tS = tmem, tdP = tmem + 128, tdV = tmem + 256, tdK = tmem + 320;
+  const uint32_t tS = tmem, tdP = tmem + 128, tdV = tmem + 256, tdK = tmem + 320, tP = tmem + 384, tdS = tmem + 448;
 
-  if (warp == 0) {
-    if (lane == 0) {
-      int g = 0, j = 0;        // steps and items this CTA has started
-      bool ok = true;
-      for (;; ++j) {
-        const int item = snake_item(j, G, (int)blockIdx.x);
-        if (item >= n_items || !ok) break;
-        const int kt = item / HB, hb = item % HB;
-        const int h = hb % p.H, b = hb / p.H;
-        const int row0 = b * p.T, k0 = kt * FA_T, ni = p.nqt - kt;
-        // K / V of the previous item are read by its S / dP products only
-        if (j > 0 && !mbar_wait<true>(B_(12), (j - 1) & 1, abort_flag, p.err, 0x4900u)) break;
-        mbar_expect_tx(B_(0), 2 * FA_TILE_BYTES);
-        tma_load_2d(base + KV_K, &tm, B_(0), p.D + h * FA_HD, row0 + k0);
-        tma_load_2d(base + KV_V, &tm, B_(0), 2 * p.D + h * FA_HD, row0 + k0);
-        for (int it = 0; it < ni; ++it, ++g) {
-          const int s = g % KV_STAGES;
-          const uint32_t ph = (uint32_t)(g / KV_STAGES) & 1u;
-          if (!mbar_wait<true>(B_(KV_QD_EMPTY + s), ph ^ 1u, abort_flag, p.err, 0x4100u + s)) {
-            ok = false;
-            break;
+  if (warp < BW_EPI_WARP) {
+    regs_less<BW_REGS_ISSUE>();
+    if (warp == 0) {
+      if (lane == 0) {
+        int j = 0, s = 0;
+        uint32_t ph = 0;
+        bool ok = true;
+        for (;; ++j) {
+          const int item = snake_item(j, G, (int)blockIdx.x);
+          if (item >= n_items || !ok) break;
+          const int kt = item / HB, hb = item % HB;
+          const int h = hb % p.H, b = hb / p.H;
+          const int row0 = b * p.T, k0 = kt * FA_T, ni = p.nqt - kt;
+          const int kb = j & 1;
+          // K / V of the item before last are read by its S / dP products only
+          if (!mbar_wait<true>(B_(KV_KV_FREE + kb), ((j >> 1) & 1) ^ 1u, abort_flag, p.err, 0x4900u)) break;
+          mbar_expect_tx(B_(KV_KV_FULL + kb), 2 * FA_TILE_BYTES);
+          tma_load_2d(base + KV_K + (2 * kb) * FA_TILE_BYTES, &tm, B_(KV_KV_FULL + kb), p.D + h * FA_HD, row0 + k0);
+          tma_load_2d(base + KV_K + (2 * kb + 1) * FA_TILE_BYTES, &tm, B_(KV_KV_FULL + kb), 2 * p.D + h * FA_HD,
+                      row0 + k0);
+          for (int it = 0; it < ni; ++it) {
+            if (!mbar_wait<true>(B_(KV_QD_EMPTY + s), ph ^ 1u, abort_flag, p.err, 0x4100u + s)) {
+              ok = false;
+              break;
+            }
+            mbar_expect_tx(B_(KV_QD_FULL + s), 2 * FA_TILE_BYTES);
+            const int qrow = row0 + (kt + it) * FA_T;
+            tma_load_2d(base + KV_Q + s * FA_TILE_BYTES, &tm, B_(KV_QD_FULL + s), h * FA_HD, qrow);
+            tma_load_2d(base + KV_DO + s * FA_TILE_BYTES, &tmdo, B_(KV_QD_FULL + s), h * FA_HD, qrow);
+            if (++s == KV_STAGES) {
+              s = 0;
+              ph ^= 1u;
+            }
           }
-          mbar_expect_tx(B_(KV_QD_FULL + s), 2 * FA_TILE_BYTES);
-          const int qrow = row0 + (kt + it) * FA_T;
-          tma_load_2d(base + KV_Q + s * FA_TILE_BYTES, &tm, B_(KV_QD_FULL + s), h * FA_HD, qrow);
-          tma_load_2d(base + KV_DO + s * FA_TILE_BYTES, &tmdo, B_(KV_QD_FULL + s), h * FA_HD, qrow);
         }
       }
-    }
-  } else if (warp == 1) {
-    // S = Q K^T and dP = dO V^T of every step (dV / dK are issued by a warp of their own, as in
-    // the dQ kernel).  The whole warp runs this converged; one elected lane issues each tcgen05
-    // instruction.
-    const uint32_t idesc_s = make_idesc(0, 0, 0, FA_T);    // [q x hd] . [key x hd]^T
-    const uint32_t d_hi = smem_desc_hi(1024);              // descriptor halves (tcgen05.cuh)
-    const uint32_t k_lo = smem_desc_lo(base + KV_K, 16), v_lo = smem_desc_lo(base + KV_V, 16);
-    const uint32_t q_lo = smem_desc_lo(base + KV_Q, 16), do_lo = smem_desc_lo(base + KV_DO, 16);
-    int s = 0;
-    uint32_t ph = 0, par = 0;
-    bool ok = true;
-    for (int j = 0; ok; ++j) {
-      const int item = snake_item(j, G, (int)blockIdx.x);
-      if (item >= n_items) break;
-      const int ni = p.nqt - item / HB;
-      ok = mbar_wait_warp<true>(B_(0), j & 1, abort_flag, p.err, 0x4200u);
-      for (int it = 0; it < ni && ok; ++it) {
-        ok = mbar_wait_warp<true>(B_(KV_QD_FULL + s), ph, abort_flag, p.err, 0x4300u + s) &&
-             mbar_wait_warp<true>(B_(6), par ^ 1u, abort_flag, p.err, 0x4400u);
-        if (!ok) break;
-        tcgen05_fence_after();
-        const uint32_t so = (uint32_t)s * (FA_TILE_BYTES >> 4);
-        umma_f16_chain<4>(tS, q_lo + so, 2, k_lo, 2, d_hi, idesc_s, 0u);
-        umma_f16_chain<4>(tdP, do_lo + so, 2, v_lo, 2, d_hi, idesc_s, 0u);
-        umma_commit_one(B_(5));
-        if (it == ni - 1) umma_commit_one(B_(12));    // the item's K / V may be replaced
-        par ^= 1u;
-        if (++s == KV_STAGES) {
-          s = 0;
-          ph ^= 1u;
-        }
-      }
-    }
-  } else if (warp == KV_MMA2_WARP) {
-    // dV += P^T dO and dK += dS^T Q of every step.  Its commits cover this warp's instructions
-    // only; a Q / dO stage is free when dV / dK of its step have retired, because the S / dP
-    // that read it retired before the softmax warps could produce the P / dS these waited for.
-    const uint32_t idesc_g = make_idesc(0, 1, 1, FA_HD);   // [q x key]^T . [q x hd]
-    const uint32_t d_hi = smem_desc_hi(1024);
-    const uint32_t qm_lo = smem_desc_lo(base + KV_Q, 8192), dom_lo = smem_desc_lo(base + KV_DO, 8192);
-    const uint32_t pt_lo = smem_desc_lo(base + KV_P, FA_TILE_BYTES);
-    const uint32_t dst_lo = smem_desc_lo(base + KV_DS, FA_TILE_BYTES);
-    int g = 0, s = 0;
-    bool ok = true;
-    for (int j = 0; ok; ++j) {
-      const int item = snake_item(j, G, (int)blockIdx.x);
-      if (item >= n_items) break;
-      const int ni = p.nqt - item / HB;
-      for (int it = 0; it < ni; ++it, ++g) {
-        ok = mbar_wait_warp<true>(B_(7), g & 1, abort_flag, p.err, 0x4500u);     // P / dS written
-        if (!ok) break;
-        if (it == 0 && j > 0) {              // the previous item's dV / dK have been read out
-          ok = mbar_wait_warp<true>(B_(13), (j - 1) & 1, abort_flag, p.err, 0x4a00u);
+    } else if (warp == 1) {
+      // S^T = K Q^T and dP^T = V dO^T of every step (dV / dK are issued by a warp of their own: one
+      // warp's stream of waits, instructions and commits for both paced the step).  The whole warp runs
+      // this converged; one elected lane issues each tcgen05 instruction.
+      const uint32_t idesc_s = make_idesc(0, 0, 0, FA_T);    // [key x hd] . [q x hd]^T
+      const uint32_t d_hi = smem_desc_hi(1024);              // descriptor halves (tcgen05.cuh)
+      const uint32_t k_lo = smem_desc_lo(base + KV_K, 16), v_lo = smem_desc_lo(base + KV_K + FA_TILE_BYTES, 16);
+      const uint32_t q_lo = smem_desc_lo(base + KV_Q, 16), do_lo = smem_desc_lo(base + KV_DO, 16);
+      int s = 0;
+      uint32_t ph = 0, par = 0;
+      bool ok = true;
+      for (int j = 0; ok; ++j) {
+        const int item = snake_item(j, G, (int)blockIdx.x);
+        if (item >= n_items) break;
+        const int ni = p.nqt - item / HB;
+        const int kb = j & 1;
+        const uint32_t ko = (uint32_t)(2 * kb) * (FA_TILE_BYTES >> 4);
+        ok = mbar_wait_warp<true>(B_(KV_KV_FULL + kb), (j >> 1) & 1, abort_flag, p.err, 0x4200u);
+        for (int it = 0; it < ni && ok; ++it) {
+          ok = mbar_wait_warp<true>(B_(KV_QD_FULL + s), ph, abort_flag, p.err, 0x4300u + s) &&
+               mbar_wait_warp<true>(B_(KV_SDP_FREE), par ^ 1u, abort_flag, p.err, 0x4400u);
           if (!ok) break;
+          tcgen05_fence_after();
+          const uint32_t so = (uint32_t)s * (FA_TILE_BYTES >> 4);
+          umma_f16_chain<4>(tS, k_lo + ko, 2, q_lo + so, 2, d_hi, idesc_s, 0u);
+          umma_f16_chain<4>(tdP, v_lo + ko, 2, do_lo + so, 2, d_hi, idesc_s, 0u);
+          umma_commit_one(B_(KV_SDP_FULL));
+          if (it == ni - 1) umma_commit_one(B_(KV_KV_FREE + kb));    // the item's K / V may be replaced
+          par ^= 1u;
+          if (++s == KV_STAGES) {
+            s = 0;
+            ph ^= 1u;
+          }
         }
-        tcgen05_fence_after();
-        // K = 128 query rows, 16 at a time: every operand is MN-major here (P^T, dS^T with their
-        // two 64-key blocks a tile apart; dO, Q with their 8-row groups 1024 bytes apart)
-        const uint32_t so = (uint32_t)s * (FA_TILE_BYTES >> 4);
-        umma_f16_chain<8>(tdV, pt_lo, 128, dom_lo + so, 128, d_hi, idesc_g, it ? 1u : 0u);
-        umma_f16_chain<8>(tdK, dst_lo, 128, qm_lo + so, 128, d_hi, idesc_g, it ? 1u : 0u);
-        umma_commit_one(B_(KV_QD_EMPTY + s));   // Q / dO stage free
-        umma_commit_one(B_(8));                 // P / dS may be overwritten
-        if (it == ni - 1) umma_commit_one(B_(9));
-        if (++s == KV_STAGES) s = 0;
+      }
+    } else if (warp == 2) {
+      // dV += P^T dO and dK += dS^T Q of every step.  Its commits cover this warp's instructions
+      // only; a Q / dO stage is free when dV / dK of its step have retired, because the S / dP
+      // that read it retired before the softmax warps could produce the P / dS these waited for.
+      const uint32_t idesc_g = make_idesc(0, 0, 1, FA_HD);   // [key x q] in tensor memory . [q x hd] (MN-major)
+      const uint32_t d_hi = smem_desc_hi(1024);
+      const uint32_t qm_lo = smem_desc_lo(base + KV_Q, 8192), dom_lo = smem_desc_lo(base + KV_DO, 8192);
+      int g = 0, s = 0;
+      bool ok = true;
+      for (int j = 0; ok; ++j) {
+        const int item = snake_item(j, G, (int)blockIdx.x);
+        if (item >= n_items) break;
+        const int ni = p.nqt - item / HB;
+        for (int it = 0; it < ni; ++it, ++g) {
+          ok = mbar_wait_warp<true>(B_(KV_PDS_FULL), g & 1, abort_flag, p.err, 0x4500u);     // P / dS written
+          if (!ok) break;
+          if (it == 0) {                       // the previous item's dV / dK have been read out
+            ok = mbar_wait_warp<true>(B_(KV_ACC_FREE), (j & 1) ^ 1u, abort_flag, p.err, 0x4a00u);
+            if (!ok) break;
+          }
+          tcgen05_fence_after();
+          const uint32_t so = (uint32_t)s * (FA_TILE_BYTES >> 4);
+          umma_f16_ts_chain<8>(tdV, tP, dom_lo + so, 128, d_hi, idesc_g, it ? 1u : 0u);
+          umma_f16_ts_chain<8>(tdK, tdS, qm_lo + so, 128, d_hi, idesc_g, it ? 1u : 0u);
+          umma_commit_one(B_(KV_QD_EMPTY + s));   // Q / dO stage free
+          umma_commit_one(B_(KV_PDS_FREE));       // P / dS may be overwritten
+          if (it == ni - 1) umma_commit_one(B_(KV_OUT_FULL));
+          if (++s == KV_STAGES) s = 0;
+        }
       }
     }
-  } else {
-    const int part = (warp - 2) >> 2;            // which 32 of the tile's 128 keys
-    const int r = (warp & 3) * 32 + lane;
-    const uint32_t t_lane = ((uint32_t)((warp & 3) * 32)) << 16;
-    bool ok = true;
-    // dV / dK of a finished item: wait for its last products, read the accumulators, hand them
-    // back, store.  Runs after the NEXT item's first step, so the hand-off to the tensor core
-    // (S, dP -> P, dS) does not stall at an item boundary.
-    int pend_item = -1, pend_j = 0;
-    auto store_item = [&](int item, int jj) -> bool {
+  } else if (warp < BW_SM_WARP) {
+    // dV / dK of a finished item: into staging as fp16, accumulators handed back, then stored (slices 2
+    // and 1 of dqkv) and added up by columns
+    regs_less<BW_REGS_EPI>();
+    const int w = warp & 3;
+    const uint32_t t_lane = ((uint32_t)(w * 32)) << 16;
+    uint8_t* stage = gbase + KV_OUT + w * 8192;
+    for (int j = 0;; ++j) {
+      const int item = snake_item(j, G, (int)blockIdx.x);
+      if (item >= n_items) break;
+      if (snake_item(j + 1, G, (int)blockIdx.x) >= n_items) break;   // the last one: see the softmax warps
       const int kt = item / HB, hb = item % HB;
       const int h = hb % p.H, b = hb / p.H;
-      const int row0 = b * p.T, k0 = kt * FA_T;
-      if (!mbar_wait_warp<SM_SPIN>(B_(9), jj & 1, abort_flag, p.err, 0x4800u)) return false;
+      if (!mbar_wait_warp<SM_SPIN>(B_(KV_OUT_FULL), j & 1, abort_flag, p.err, 0x4800u)) break;
       tcgen05_fence_after();
-      const int key = k0 + r;     // accumulator rows are keys here
-      // parts 0, 1 store the two 32-column halves of dV (slice 2 of dqkv), parts 2, 3 those of
-      // dK (slice 1)
-      uint32_t rr[32];
-      const int slice = part < 2 ? 2 : 1, col0 = (part & 1) * 32;
-      const uint32_t t = (part < 2 ? tdV : tdK) + t_lane + (uint32_t)col0;
-      tmem_ld16(t, rr);
-      tmem_ld16(t + 16, rr + 16);
-      tmem_wait_ld();
+      stage_acc<8>(tdV + t_lane, stage, lane);
+      stage_acc<8>(tdK + t_lane, stage + 4096, lane);
       tcgen05_fence_before();
       __syncwarp();
-      if (lane == 0) mbar_arrive(B_(13));           // the accumulators may be overwritten
-      {
-        uint4 hv[4];
-#pragma unroll
-        for (int u = 0; u < 4; ++u) {
-          __half2 h2[4];
-#pragma unroll
-          for (int e = 0; e < 4; ++e)
-            h2[e] = __floats2half2_rn(__uint_as_float(rr[u * 8 + 2 * e]),
-                                      __uint_as_float(rr[u * 8 + 2 * e + 1]));
-          hv[u] = *reinterpret_cast<uint4*>(h2);
-        }
-        const int key_w = k0 + (warp & 3) * 32;      // first key of this warp's 32 rows
-        __half* dst = p.dqkv + (size_t)(row0 + key_w) * 3 * p.D + slice * p.D + h * FA_HD + col0;
-        warp_store_rows<4>(hv, gbase + KV_OUT + (warp - 2) * 2048, lane, reinterpret_cast<uint8_t*>(dst),
-                           (size_t)3 * p.D * 2, p.T - key_w);
+      if (lane == 0) mbar_arrive(B_(KV_ACC_FREE));     // the accumulators may be overwritten
+      const int key_w = kt * FA_T + w * 32;            // first key of this warp's 32 rows
+      float* sums = p.colsum ? p.colsum + ((size_t)(b * p.nqt + kt) * 4 + w) * 3 * p.D + h * FA_HD : nullptr;
+#pragma unroll 1
+      for (int slice = 2; slice >= 1; --slice) {
+        __half* dst = p.dqkv + (size_t)(b * p.T + key_w) * 3 * p.D + slice * p.D + h * FA_HD;
+        store_staged<8>(stage + (2 - slice) * 4096, lane, reinterpret_cast<uint8_t*>(dst), (size_t)3 * p.D * 2,
+                        p.T - key_w, sums ? sums + slice * p.D : nullptr);
       }
-      if (p.colsum) {
-        // the qkv bias gradient: column sums of dV / dK as stored
-        float val[32];
-#pragma unroll
-        for (int c = 0; c < 32; ++c)
-          val[c] = key < p.T ? __half2float(__float2half_rn(__uint_as_float(rr[c]))) : 0.f;
-        float* dst = p.colsum + ((size_t)(b * p.nqt + kt) * 4 + (warp & 3)) * 3 * p.D + slice * p.D +
-                     h * FA_HD + col0;
-        warp_col_sums<32>(val, lane, dst);
-      }
-      return true;
-    };
-    // statistics of this thread's row in the first query tile of an item
-    auto first_stat = [&](int item, float& lse, float& dl, int& st) {
-      const int kt = item / HB, hb = item % HB;
-      const int qi = kt * FA_T + r;
+      __syncwarp();                                    // the staging is filled again
+    }
+  } else {
+    regs_more<BW_REGS_SM>();
+    const int part = (warp - BW_SM_WARP) >> 2;   // which 32 of the tile's 128 queries
+    const int r = (warp & 3) * 32 + lane;        // key within the tile = TMEM lane
+    const uint32_t t_lane = ((uint32_t)((warp & 3) * 32)) << 16;
+    float2* stat = reinterpret_cast<float2*>(gbase + KV_STAT + (warp - BW_SM_WARP) * 256);
+    int* seg_s = reinterpret_cast<int*>(gbase + KV_SEG + (warp - BW_SM_WARP) * 128);
+    bool ok = true;
+    // statistics of the query this lane looks after (part * 32 + lane) in the step ahead, fetched while
+    // this one is worked on (a load from global memory at the start of a step would sit on the critical
+    // path)
+    float lse_n = 0.f, dl_n = 0.f;
+    int st_n = 0;
+    auto fetch_stat = [&](int hb, int qt) {
+      const int qi = qt * FA_T + part * 32 + lane;
       const bool q_ok = qi < p.T;
-      const size_t i = (size_t)((hb / p.H) * p.H + hb % p.H) * p.T + (q_ok ? qi : 0);
-      lse = p.lse2[i];
-      dl = p.delta[i];
-      st = (p.seg && q_ok) ? (int)p.seg[(hb / p.H) * p.T + qi] : 0;
+      const int i = hb * p.T + (q_ok ? qi : 0);
+      // a query past the end of the sequence gets lse = +inf, hence P = 0 and dS = 0
+      lse_n = q_ok ? p.lse2[i] : INFINITY;
+      dl_n = p.delta[i];
+      if (p.seg) st_n = q_ok ? (int)p.seg[(hb / p.H) * p.T + qi] : 0;
     };
-    float lse_f = 0.f, dl_f = 0.f;
-    int st_f = 0;
-    if ((int)blockIdx.x < n_items) first_stat((int)blockIdx.x, lse_f, dl_f, st_f);
-    int g = 0, j = 0;
-    for (;; ++j) {
+    if ((int)blockIdx.x < n_items) fetch_stat((int)blockIdx.x % HB, (int)blockIdx.x / HB);
+    int g = 0, last = -1, last_j = 0;
+    // Barriers are looked at ahead of need, and waited for only if they were not complete by then: a
+    // wait that is already satisfied takes 200 to 300 cycles beside a busy tensor core.
+    bool ready = false;
+    for (int j = 0; ok; ++j) {
       const int item = snake_item(j, G, (int)blockIdx.x);
-      if (item >= n_items || !ok) break;
+      if (item >= n_items) break;
       const int kt = item / HB, hb = item % HB;
-      const int h = hb % p.H, b = hb / p.H;
-      const int row0 = b * p.T, k0 = kt * FA_T, ni = p.nqt - kt;
-      // row statistics of query tile kt + it; the next tile's are fetched one step ahead, the
-      // first tile's of the next item one item ahead (a load from global memory at the start
-      // of an item would sit on the critical path)
-      const float* lse_h = p.lse2 + (size_t)(b * p.H + h) * p.T;
-      const float* delta_h = p.delta + (size_t)(b * p.H + h) * p.T;
-      auto row_stat = [&](int qi, float& lse, float& dl, int& st) {
-        const bool q_ok = qi < p.T;
-        const int i = q_ok ? qi : 0;
-        lse = lse_h[i];
-        dl = delta_h[i];
-        st = (p.seg && q_ok) ? (int)p.seg[row0 + qi] : 0;
-      };
-      float lse_n = lse_f, dl_n = dl_f;
-      int st_n = st_f;
-      {
-        const int nxt = snake_item(j + 1, G, (int)blockIdx.x);
-        if (nxt < n_items) first_stat(nxt, lse_f, dl_f, st_f);
-      }
-      for (int it = 0; it < ni && ok; ++it, ++g) {
-        const int qt = kt + it;
-        const int qi = qt * FA_T + r;
-        const bool q_ok = qi < p.T;
-        // a row past the end of the sequence gets lse = +inf, hence P = 0 and dS = 0
-        const float nlse = q_ok ? -lse_n : -INFINITY, dsc = -dl_n * p.scale;
-        const int st = st_n;
-        if (it + 1 < ni) row_stat(qi + FA_T, lse_n, dl_n, st_n);
-        const bool need_mask = (qt == kt) || (p.seg != nullptr);
-        ok = mbar_wait_warp<SM_SPIN>(B_(5), g & 1, abort_flag, p.err, 0x4600u);
+      const int key = kt * FA_T + r;
+      last = item;
+      last_j = j;
+      for (int qt = kt; qt < p.nqt && ok; ++qt, ++g) {
+        stat[lane] = make_float2(-lse_n, -dl_n * p.scale);
+        if (p.seg) seg_s[lane] = st_n;
+        __syncwarp();
+        if (qt + 1 < p.nqt) {
+          fetch_stat(hb, qt + 1);
+        } else {
+          const int nxt = snake_item(j + 1, G, (int)blockIdx.x);
+          if (nxt < n_items) fetch_stat(nxt % HB, nxt / HB);
+        }
+        ok = ready || mbar_wait_warp<SM_SPIN>(B_(KV_SDP_FULL), g & 1, abort_flag, p.err, 0x4600u);
         if (!ok) break;
         tcgen05_fence_after();
         uint32_t rs[32], rdp[32];
@@ -972,28 +1000,46 @@ attn_bwd_kv_kernel(const __grid_constant__ CUtensorMap tm, const __grid_constant
         tmem_wait_ld();
         tcgen05_fence_before();
         __syncwarp();
-        if (lane == 0) mbar_arrive(B_(6));          // S / dP may be overwritten
-        // P and dS of this step, packed, in registers; the buffer is still being read
-        uint4 hp[4], hd[4];
-        if (need_mask) bwd_chunk_regs<true>(rs, rdp, part, k0, qi, st, p.cscale, p.scale, nlse, dsc, hp, hd);
-        else bwd_chunk_regs<false>(rs, rdp, part, k0, qi, st, p.cscale, p.scale, nlse, dsc, hp, hd);
-        ok = mbar_wait_warp<SM_SPIN>(B_(8), (g & 1) ^ 1u, abort_flag, p.err, 0x4700u);   // dV / dK of step g - 1 done
+        if (lane == 0) mbar_arrive(B_(KV_SDP_FREE));          // S / dP may be overwritten
+        // P and dS, overwriting the scores and products they came from
+        const float4* st4 = reinterpret_cast<const float4*>(stat);
+        const int q0 = qt * FA_T + part * 32;
+        if (p.seg) bwd_pds_pack<2>(rs, rdp, st4, seg_s, q0, key, p.cscale, p.scale, rs, rdp);
+        else if (qt == kt) bwd_pds_pack<1>(rs, rdp, st4, nullptr, q0, key, p.cscale, p.scale, rs, rdp);
+        else bwd_pds_pack<0>(rs, rdp, st4, nullptr, 0, 0, p.cscale, p.scale, rs, rdp);
+        ready = mbar_test_wait(B_(KV_PDS_FREE), (g & 1) ^ 1u) != 0;
+        if (p.seg) bwd_pds_pack<2>(rs + 16, rdp + 16, st4 + 8, seg_s + 16, q0 + 16, key, p.cscale, p.scale, rs + 8, rdp + 8);
+        else if (qt == kt) bwd_pds_pack<1>(rs + 16, rdp + 16, st4 + 8, nullptr, q0 + 16, key, p.cscale, p.scale, rs + 8, rdp + 8);
+        else bwd_pds_pack<0>(rs + 16, rdp + 16, st4 + 8, nullptr, 0, 0, p.cscale, p.scale, rs + 8, rdp + 8);
+        // dV / dK of step g - 1 done
+        ok = __all_sync(0xffffffffu, ready) ||
+             mbar_wait_warp<SM_SPIN>(B_(KV_PDS_FREE), (g & 1) ^ 1u, abort_flag, p.err, 0x4700u);
         if (!ok) break;
-        uint8_t* sp = gbase + KV_P;
-        uint8_t* sds = gbase + KV_DS;
-        bwd_chunk_store(part, r, hp, hd, sp, sds);
-        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+        tcgen05_fence_after();
+        tmem_st16(tP + t_lane + part * 16, rs);
+        tmem_st16(tdS + t_lane + part * 16, rdp);
+        ready = mbar_test_wait(B_(KV_SDP_FULL), (g & 1) ^ 1u) != 0;
+        tmem_wait_st();
+        tcgen05_fence_before();
         __syncwarp();
-        if (lane == 0) mbar_arrive(B_(7));
-        if (pend_item >= 0) {      // the previous item's accumulators, now surely complete
-          ok = store_item(pend_item, pend_j);
-          pend_item = -1;
-        }
+        if (lane == 0) mbar_arrive(B_(KV_PDS_FULL));
+        ready = __all_sync(0xffffffffu, ready);
       }
-      pend_item = item;       // read this item's dV / dK out after the next item's first step
-      pend_j = j;
     }
-    if (ok && pend_item >= 0) ok = store_item(pend_item, pend_j);
+    // The CTA's last item (its only one in a small problem) has nothing to overlap with: all sixteen
+    // warps read it out, 32 columns each (dV by parts 0 and 1, dK by 2 and 3), through the idle ring.
+    if (ok && last >= 0 && mbar_wait_warp<SM_SPIN>(B_(KV_OUT_FULL), last_j & 1, abort_flag, p.err, 0x4c00u)) {
+      tcgen05_fence_after();
+      uint8_t* stage = gbase + KV_Q + (warp - BW_SM_WARP) * 2048;
+      stage_acc<4>(tdV + t_lane + part * 32, stage, lane);
+      __syncwarp();
+      const int kt = last / HB, hb = last % HB, b = hb / p.H;
+      const int key_w = kt * FA_T + (warp & 3) * 32;
+      const int col = (part < 2 ? 2 : 1) * p.D + (hb % p.H) * FA_HD + (part & 1) * 32;
+      store_staged<4>(stage, lane, reinterpret_cast<uint8_t*>(p.dqkv + (size_t)(b * p.T + key_w) * 3 * p.D + col),
+                      (size_t)3 * p.D * 2, p.T - key_w,
+                      p.colsum ? p.colsum + ((size_t)(b * p.nqt + kt) * 4 + (warp & 3)) * 3 * p.D + col : nullptr);
+    }
   }
   __syncwarp();
   tcgen05_fence_before();
@@ -1009,40 +1055,41 @@ attn_bwd_kv_kernel(const __grid_constant__ CUtensorMap tm, const __grid_constant
   }
 }
 
-// dQ: persistent CTAs like the dK / dV kernel; an item is a (query tile, head, sequence),
-// heaviest query tile first, and loops over the key tiles up to the diagonal.  Q / dO are the
-// per-item operands (reloaded once the item's last S / dP have retired: qd_free), K / V the
-// per-step ones, in a ring of three stages: a stage is read by S / dP of its step and again by
-// dQ of the same step a softmax later.
+// dQ: an item is a (query tile, head, sequence), heaviest query tile first, and loops over the key
+// tiles up to the diagonal.  Q / dO / O are the per-item operands, K / V the per-step ones, in a ring
+// of three stages: a stage is read by S / dP of its step and again by dQ of the same step a softmax
+// later.
 // dS never passes through shared memory: the softmax warps write it (fp16 pairs) into one of
 // two areas of tensor memory with tcgen05.st, and dQ += dS K reads it there as the A operand.
-// What paces a step is the warp that issues the MMAs: it shares its scheduler with softmax
-// warps, a wait that is already satisfied costs it about 180 cycles and a loop iteration 400,
-// so its loop is kept as short as it can be (one elected lane per instruction, descriptor
-// halves stepped by adds, no wait that another wait implies).  Splitting a step into two
-// half-steps with two softmax groups half a step apart doubled that warp's waits and commits
-// and measured 15 % slower, although the softmax warps then idled less.
+// The warps that issue the MMAs keep their loops as short as they can be (one elected lane per
+// instruction, descriptor halves stepped by adds, no wait that another wait implies): a wait that is
+// already satisfied costs such a warp about 180 cycles and a loop iteration 400.  Splitting a step into
+// two half-steps with two softmax groups half a step apart doubled their waits and commits and
+// measured 15 % slower, although the softmax warps then idled less.
 // This kernel also forms delta = rowsum(dO * O) (tkernels.py:176-179 computes the same number
-// as sum_j dP_ij P_ij): the O tile of an item is loaded beside Q and dO, every softmax thread
-// sums its row's 64 products from shared memory at the start of the item, and the rows are
-// written out for the dK / dV kernel, which is launched after this one.
-// TMEM columns: S [0, 128) dP [128, 256) dQ [256, 320) dS [320 + 64 b, +64) for buffer b.
+// as sum_j dP_ij P_ij): the epilogue warps add a row's 64 products up from the O and dO tiles of the
+// item ahead, for the softmax warps and, written out, for the dK / dV kernel, which is launched after
+// this one.
+// TMEM columns: S [0, 128) dP [128, 256) dQ [256 + 64 a, +64) of two items in turn, dS [384 + 64 b, +64).
 constexpr int DQ_STAGES = 3;
-constexpr int DQ_Q = 0, DQ_DO = FA_TILE_BYTES, DQ_O = 2 * FA_TILE_BYTES, DQ_K = 3 * FA_TILE_BYTES,
-              DQ_V = (3 + DQ_STAGES) * FA_TILE_BYTES,
-              DQ_OUT = (3 + 2 * DQ_STAGES) * FA_TILE_BYTES,    // output staging, one tile
-              DQ_BAR = DQ_OUT + FA_TILE_BYTES, DQ_SMEM = DQ_BAR + 256 + 1024;
+constexpr int DQ_Q = 0,                                        // two buffers of Q, dO and O
+              DQ_K = 6 * FA_TILE_BYTES, DQ_V = (6 + DQ_STAGES) * FA_TILE_BYTES,
+              DQ_OUT = (6 + 2 * DQ_STAGES) * FA_TILE_BYTES,    // output staging, one tile
+              DQ_DELTA = DQ_OUT + FA_TILE_BYTES,               // [2][128] floats
+              DQ_BAR = DQ_DELTA + 1024, DQ_SMEM = DQ_BAR + 256 + 1024;
 static_assert(DQ_SMEM <= 227 * 1024, "dQ kernel: shared memory");
-constexpr int DQ_NBAR = 14 + 2 * DQ_STAGES, DQ_KV_FULL = 14, DQ_KV_EMPTY = 14 + DQ_STAGES;
+constexpr int DQ_QD_FULL = 0, DQ_QD_FREE = 2, DQ_OD_FREE = 4, DQ_DL_FULL = 6, DQ_SDP_FULL = 8, DQ_SDP_FREE = 9,
+              DQ_DS_FULL = 10, DQ_DS_FREE = 12, DQ_OUT_FULL = 14, DQ_ACC_FREE = 16, DQ_KV_FULL = 18,
+              DQ_KV_EMPTY = 18 + DQ_STAGES, DQ_NBAR = 18 + 2 * DQ_STAGES;
 
-// dS = P (dP - delta) scale for 32 keys of one query row, as fp16 pairs (keys 2i, 2i + 1) in
-// pk[i], ready for tcgen05.st; P is rebuilt from the saved log-sum-exp as in bwd_chunk_regs.
+// dS = P (dP - delta) scale for 16 keys of one query row, as fp16 pairs (keys 2i, 2i + 1) in
+// pk[i], ready for tcgen05.st; P is rebuilt from the saved log-sum-exp as in bwd_pds_pack.
 template <bool MASK>
 __device__ __forceinline__ void bwd_ds_pack(const uint32_t* rs, const uint32_t* rdp, int key0, int qi,
                                             int st, float cscale, float scale, float nlse, float dsc,
                                             uint32_t* pk) {
 #pragma unroll
-  for (int i = 0; i < 16; ++i) {
+  for (int i = 0; i < 8; ++i) {
     float dv[2];
 #pragma unroll
     for (int w = 0; w < 2; ++w) {
@@ -1059,31 +1106,30 @@ __device__ __forceinline__ void bwd_ds_pack(const uint32_t* rs, const uint32_t* 
   }
 }
 
-__global__ void __launch_bounds__(DQ_THREADS, 1)
+__global__ void __launch_bounds__(BW_THREADS, 1)
 attn_bwd_q_kernel(const __grid_constant__ CUtensorMap tm, const __grid_constant__ CUtensorMap tmdo,
                   const __grid_constant__ CUtensorMap tmo, const AttnParams p) {
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
   uint8_t* gbase = smem_raw + (base - smem_u32(smem_raw));
   const uint32_t bar = base + DQ_BAR;
-  // 0 qd_full, 1 od_free (delta formed from the dO / O tiles), 5 sdp_full, 6 sdp_free,
-  // 7/10 ds_full[2], 8/11 ds_free[2], 9 out_full, 12 qd_free, 13 acc_free, 14.. kv_full[stage],
-  // then kv_empty[stage]
   auto B_ = [bar](int i) { return bar + 8u * i; };
   volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(gbase + DQ_BAR + 192);
   volatile uint32_t* abort_flag = reinterpret_cast<volatile uint32_t*>(gbase + DQ_BAR + 200);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int HB = p.H * p.B;
   const int n_items = p.nqt * HB, G = (int)gridDim.x;
-  constexpr int OUT_WARPS = DQ_SOFTMAX_WARPS < 8 ? DQ_SOFTMAX_WARPS : 8;   // warps that read dQ out
 
   pdl_trigger();
   if (threadIdx.x == 0) {
     prefetch_tensormap(&tm);
     prefetch_tensormap(&tmdo);
     prefetch_tensormap(&tmo);
-    for (int i = 0; i < DQ_NBAR; ++i)
-      mbar_init(B_(i), (i == 1 || i == 6 || i == 7 || i == 10) ? DQ_SOFTMAX_WARPS : (i == 13 ? OUT_WARPS : 1));
+    for (int i = 0; i < DQ_NBAR; ++i) {
+      const bool sm = i == DQ_SDP_FREE || (i >= DQ_DS_FULL && i < DQ_DS_FULL + 2);
+      const bool epi = (i >= DQ_OD_FREE && i < DQ_DL_FULL + 2) || (i >= DQ_ACC_FREE && i < DQ_ACC_FREE + 2);
+      mbar_init(B_(i), sm ? BW_SM_WARPS : epi ? BW_EPI_WARPS : 1);
+    }
     *abort_flag = 0u;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
@@ -1094,260 +1140,266 @@ attn_bwd_q_kernel(const __grid_constant__ CUtensorMap tm, const __grid_constant_
   tcgen05_fence_after();
   pdl_wait();
   const uint32_t tmem = *tmem_slot;
-  const uint32_t tS = tmem, tdP = tmem + 128, tdQ = tmem + 256, tdS = tmem + 320;
+  const uint32_t tS = tmem, tdP = tmem + 128, tdQ = tmem + 256, tdS = tmem + 384;
 
-  if (warp == 0) {
-    if (lane == 0) {
-      int g = 0, j = 0;
-      bool ok = true;
-      for (;; ++j) {
-        const int item = snake_item(j, G, (int)blockIdx.x);
-        if (item >= n_items || !ok) break;
-        const int qt = p.nqt - 1 - item / HB, hb = item % HB;
-        const int h = hb % p.H, b = hb / p.H;
-        const int row0 = b * p.T, q0 = qt * FA_T, nj = qt + 1;
-        // the previous item's Q / dO have been read by its last S / dP, its dO / O by every
-        // softmax warp
-        if (j > 0 && !(mbar_wait<true>(B_(12), (j - 1) & 1, abort_flag, p.err, 0x5900u) &&
-                       mbar_wait<true>(B_(1), (j - 1) & 1, abort_flag, p.err, 0x5b00u)))
-          break;
-        mbar_expect_tx(B_(0), 3 * FA_TILE_BYTES);
-        tma_load_2d(base + DQ_Q, &tm, B_(0), h * FA_HD, row0 + q0);
-        tma_load_2d(base + DQ_DO, &tmdo, B_(0), h * FA_HD, row0 + q0);
-        tma_load_2d(base + DQ_O, &tmo, B_(0), h * FA_HD, row0 + q0);
-        for (int kt = 0; kt < nj; ++kt, ++g) {
-          const int s = g % DQ_STAGES;
-          const uint32_t ph = (uint32_t)(g / DQ_STAGES) & 1u;
-          if (!mbar_wait<true>(B_(DQ_KV_EMPTY + s), ph ^ 1u, abort_flag, p.err, 0x5100u + s)) {
-            ok = false;
+  if (warp < BW_EPI_WARP) {
+    regs_less<BW_REGS_ISSUE>();
+    if (warp == 0) {
+      if (lane == 0) {
+        int j = 0, s = 0;
+        uint32_t ph = 0;
+        bool ok = true;
+        for (;; ++j) {
+          const int item = snake_item(j, G, (int)blockIdx.x);
+          if (item >= n_items || !ok) break;
+          const int qt = p.nqt - 1 - item / HB, hb = item % HB;
+          const int h = hb % p.H, b = hb / p.H;
+          const int row0 = b * p.T, q0 = qt * FA_T, nj = qt + 1;
+          const int qb = j & 1;
+          const uint32_t qd = base + DQ_Q + (uint32_t)(3 * qb) * FA_TILE_BYTES;
+          const uint32_t old = ((j >> 1) & 1) ^ 1u;
+          // Q / dO of the item before last have been read by its S / dP, its dO / O by the epilogue warps
+          if (!(mbar_wait<true>(B_(DQ_QD_FREE + qb), old, abort_flag, p.err, 0x5900u) &&
+                mbar_wait<true>(B_(DQ_OD_FREE + qb), old, abort_flag, p.err, 0x5b00u)))
             break;
+          mbar_expect_tx(B_(DQ_QD_FULL + qb), 3 * FA_TILE_BYTES);
+          tma_load_2d(qd, &tm, B_(DQ_QD_FULL + qb), h * FA_HD, row0 + q0);
+          tma_load_2d(qd + FA_TILE_BYTES, &tmdo, B_(DQ_QD_FULL + qb), h * FA_HD, row0 + q0);
+          tma_load_2d(qd + 2 * FA_TILE_BYTES, &tmo, B_(DQ_QD_FULL + qb), h * FA_HD, row0 + q0);
+          for (int kt = 0; kt < nj; ++kt) {
+            if (!mbar_wait<true>(B_(DQ_KV_EMPTY + s), ph ^ 1u, abort_flag, p.err, 0x5100u + s)) {
+              ok = false;
+              break;
+            }
+            mbar_expect_tx(B_(DQ_KV_FULL + s), 2 * FA_TILE_BYTES);
+            tma_load_2d(base + DQ_K + s * FA_TILE_BYTES, &tm, B_(DQ_KV_FULL + s), p.D + h * FA_HD, row0 + kt * FA_T);
+            tma_load_2d(base + DQ_V + s * FA_TILE_BYTES, &tm, B_(DQ_KV_FULL + s), 2 * p.D + h * FA_HD,
+                        row0 + kt * FA_T);
+            if (++s == DQ_STAGES) {
+              s = 0;
+              ph ^= 1u;
+            }
           }
-          mbar_expect_tx(B_(DQ_KV_FULL + s), 2 * FA_TILE_BYTES);
-          tma_load_2d(base + DQ_K + s * FA_TILE_BYTES, &tm, B_(DQ_KV_FULL + s), p.D + h * FA_HD,
-                      row0 + kt * FA_T);
-          tma_load_2d(base + DQ_V + s * FA_TILE_BYTES, &tm, B_(DQ_KV_FULL + s), 2 * p.D + h * FA_HD,
-                      row0 + kt * FA_T);
         }
       }
-    }
-  } else if (warp == 1) {
-    // S = Q K^T and dP = dO V^T of every step.  The whole warp runs this converged; one elected
-    // lane issues each tcgen05 instruction.
-    const uint32_t idesc_s = make_idesc(0, 0, 0, FA_T);
-    const uint32_t d_hi = smem_desc_hi(1024);      // descriptor halves (tcgen05.cuh)
-    const uint32_t q_lo = smem_desc_lo(base + DQ_Q, 16), do_lo = smem_desc_lo(base + DQ_DO, 16);
-    const uint32_t k_lo = smem_desc_lo(base + DQ_K, 16), v_lo = smem_desc_lo(base + DQ_V, 16);
-    int s = 0;
-    uint32_t ph = 0, par = 0;
-    bool ok = true;
-    for (int j = 0; ok; ++j) {
-      const int item = snake_item(j, G, (int)blockIdx.x);
-      if (item >= n_items) break;
-      const int nj = p.nqt - item / HB;               // key tiles of the item: qt + 1
-      ok = mbar_wait_warp<true>(B_(0), j & 1, abort_flag, p.err, 0x5200u);
-      for (int kt = 0; kt < nj && ok; ++kt) {
-        ok = mbar_wait_warp<true>(B_(DQ_KV_FULL + s), ph, abort_flag, p.err, 0x5300u + s) &&
-             mbar_wait_warp<true>(B_(6), par ^ 1u, abort_flag, p.err, 0x5400u);
-        if (!ok) break;
-        tcgen05_fence_after();
-        const uint32_t so = (uint32_t)s * (FA_TILE_BYTES >> 4);
-        umma_f16_chain<4>(tS, q_lo, 2, k_lo + so, 2, d_hi, idesc_s, 0u);
-        umma_f16_chain<4>(tdP, do_lo, 2, v_lo + so, 2, d_hi, idesc_s, 0u);
-        umma_commit_one(B_(5));
-        if (kt == nj - 1) umma_commit_one(B_(12));    // the item's Q / dO may be replaced
-        par ^= 1u;
-        if (++s == DQ_STAGES) {
-          s = 0;
-          ph ^= 1u;
-        }
-      }
-    }
-  } else if (warp == DQ_MMA2_WARP) {
-    // dQ += dS K of every step, issued by a warp of its own: the instruction stream of one warp
-    // for both (waits, 16 instructions, commits, about 1900 cycles per step next to busy softmax
-    // warps) was what paced the kernel.  Its commits cover this warp's instructions only; a
-    // K / V stage is free when dQ of its step has retired, because the S / dP that read it
-    // retired before the softmax warps could produce the dS this dQ waited for.
-    const uint32_t idesc_q = make_idesc(0, 0, 1, FA_HD);   // dS (tensor memory) . K (MN-major), N = 64
-    const uint32_t d_hi = smem_desc_hi(1024);
-    const uint32_t km_lo = smem_desc_lo(base + DQ_K, 8192);
-    int g = 0, s = 0;
-    bool ok = true;
-    for (int j = 0; ok; ++j) {
-      const int item = snake_item(j, G, (int)blockIdx.x);
-      if (item >= n_items) break;
-      const int nj = p.nqt - item / HB;
-      for (int kt = 0; kt < nj; ++kt, ++g) {
-        const int pb = g & 1;
-        ok = mbar_wait_warp<true>(B_(7 + 3 * pb), (g >> 1) & 1, abort_flag, p.err, 0x5500u);
-        if (!ok) break;
-        if (kt == 0 && j > 0) {
-          ok = mbar_wait_warp<true>(B_(13), (j - 1) & 1, abort_flag, p.err, 0x5a00u);
+    } else if (warp == 1) {
+      // S = Q K^T and dP = dO V^T of every step.  The whole warp runs this converged; one elected
+      // lane issues each tcgen05 instruction.
+      const uint32_t idesc_s = make_idesc(0, 0, 0, FA_T);
+      const uint32_t d_hi = smem_desc_hi(1024);      // descriptor halves (tcgen05.cuh)
+      const uint32_t q_lo = smem_desc_lo(base + DQ_Q, 16), do_lo = smem_desc_lo(base + DQ_Q + FA_TILE_BYTES, 16);
+      const uint32_t k_lo = smem_desc_lo(base + DQ_K, 16), v_lo = smem_desc_lo(base + DQ_V, 16);
+      int s = 0;
+      uint32_t ph = 0, par = 0;
+      bool ok = true;
+      for (int j = 0; ok; ++j) {
+        const int item = snake_item(j, G, (int)blockIdx.x);
+        if (item >= n_items) break;
+        const int nj = p.nqt - item / HB;               // key tiles of the item: qt + 1
+        const int qb = j & 1;
+        const uint32_t qo = (uint32_t)(3 * qb) * (FA_TILE_BYTES >> 4);
+        ok = mbar_wait_warp<true>(B_(DQ_QD_FULL + qb), (j >> 1) & 1, abort_flag, p.err, 0x5200u);
+        for (int kt = 0; kt < nj && ok; ++kt) {
+          ok = mbar_wait_warp<true>(B_(DQ_KV_FULL + s), ph, abort_flag, p.err, 0x5300u + s) &&
+               mbar_wait_warp<true>(B_(DQ_SDP_FREE), par ^ 1u, abort_flag, p.err, 0x5400u);
           if (!ok) break;
+          tcgen05_fence_after();
+          const uint32_t so = (uint32_t)s * (FA_TILE_BYTES >> 4);
+          umma_f16_chain<4>(tS, q_lo + qo, 2, k_lo + so, 2, d_hi, idesc_s, 0u);
+          umma_f16_chain<4>(tdP, do_lo + qo, 2, v_lo + so, 2, d_hi, idesc_s, 0u);
+          umma_commit_one(B_(DQ_SDP_FULL));
+          if (kt == nj - 1) umma_commit_one(B_(DQ_QD_FREE + qb));    // the item's Q / dO may be replaced
+          par ^= 1u;
+          if (++s == DQ_STAGES) {
+            s = 0;
+            ph ^= 1u;
+          }
         }
-        tcgen05_fence_after();
-        // K = 128 keys: dS from tensor memory (8 columns per step), K MN-major
-        umma_f16_ts_chain<8>(tdQ, tdS + 64 * pb, km_lo + (uint32_t)s * (FA_TILE_BYTES >> 4), 128, d_hi, idesc_q,
-                             kt ? 1u : 0u);
-        umma_commit_one(B_(DQ_KV_EMPTY + s));   // K / V stage free
-        umma_commit_one(B_(8 + 3 * pb));        // this dS area free
-        if (kt == nj - 1) umma_commit_one(B_(9));
-        if (++s == DQ_STAGES) s = 0;
+      }
+    } else if (warp == 2) {
+      // dQ += dS K of every step, issued by a warp of its own: the instruction stream of one warp
+      // for both (waits, 16 instructions, commits, about 1900 cycles per step next to busy softmax
+      // warps) was what paced the kernel.  Its commits cover this warp's instructions only; a
+      // K / V stage is free when dQ of its step has retired, because the S / dP that read it
+      // retired before the softmax warps could produce the dS this dQ waited for.
+      const uint32_t idesc_q = make_idesc(0, 0, 1, FA_HD);   // dS (tensor memory) . K (MN-major), N = 64
+      const uint32_t d_hi = smem_desc_hi(1024);
+      const uint32_t km_lo = smem_desc_lo(base + DQ_K, 8192);
+      int g = 0, s = 0;
+      bool ok = true;
+      for (int j = 0; ok; ++j) {
+        const int item = snake_item(j, G, (int)blockIdx.x);
+        if (item >= n_items) break;
+        const int nj = p.nqt - item / HB;
+        const int ab = j & 1;
+        for (int kt = 0; kt < nj; ++kt, ++g) {
+          const int pb = g & 1;
+          ok = mbar_wait_warp<true>(B_(DQ_DS_FULL + pb), (g >> 1) & 1, abort_flag, p.err, 0x5500u);
+          if (!ok) break;
+          if (kt == 0) {                        // dQ of the item before last has been read out
+            ok = mbar_wait_warp<true>(B_(DQ_ACC_FREE + ab), ((j >> 1) & 1) ^ 1u, abort_flag, p.err, 0x5a00u);
+            if (!ok) break;
+          }
+          tcgen05_fence_after();
+          // K = 128 keys: dS from tensor memory (8 columns per step), K MN-major
+          umma_f16_ts_chain<8>(tdQ + 64 * ab, tdS + 64 * pb, km_lo + (uint32_t)s * (FA_TILE_BYTES >> 4), 128, d_hi,
+                               idesc_q, kt ? 1u : 0u);
+          umma_commit_one(B_(DQ_KV_EMPTY + s));   // K / V stage free
+          umma_commit_one(B_(DQ_DS_FREE + pb));   // this dS area free
+          if (kt == nj - 1) umma_commit_one(B_(DQ_OUT_FULL + ab));
+          if (++s == DQ_STAGES) s = 0;
+        }
       }
     }
-  } else {
-    constexpr int PARTS = DQ_SOFTMAX_WARPS / 4;  // warps per TMEM lane quarter
-    constexpr int CPT = FA_T / PARTS;            // keys of a row per thread: 32 or 64
-    const int part = (warp - 2) >> 2;            // which CPT of a key tile's 128 keys
-    const int r = (warp & 3) * 32 + lane;
-    const uint32_t t_lane = ((uint32_t)((warp & 3) * 32)) << 16;
-    bool ok = true;
-    // dQ of a finished item, read out after the NEXT item's first step (see the dK / dV kernel)
-    // by the first OUT_WARPS warps, 64 / (OUT_WARPS / 4) columns each
-    constexpr int OC = FA_HD / (OUT_WARPS / 4);
-    int pend_item = -1, pend_j = 0;
-    auto store_item = [&](int item, int jj) -> bool {
-      const int qt = p.nqt - 1 - item / HB, hb = item % HB;
-      const int h = hb % p.H, b = hb / p.H;
-      const int row0 = b * p.T, qi = qt * FA_T + r;
-      const bool q_ok = qi < p.T;
-      if (!mbar_wait_warp<SM_SPIN>(B_(9), jj & 1, abort_flag, p.err, 0x5800u)) return false;
-      tcgen05_fence_after();
-      uint32_t rr[OC];
+  } else if (warp < BW_SM_WARP) {
+    regs_less<BW_REGS_EPI>();
+    const int w = warp & 3;
+    const int r = w * 32 + lane;                 // query row within the tile = TMEM lane
+    uint8_t* stage = gbase + DQ_OUT + w * 4096;
+    float* delta_s = reinterpret_cast<float*>(gbase + DQ_DELTA);
+    // delta of item j's rows from its dO and O tiles (128-byte rows, 16-byte pieces XOR-ed with the
+    // row's low three bits, as the tensor map wrote them).  Item j - 2's delta has been read by then:
+    // its dQ, which this warp has stored, came after.
+    auto form_delta = [&](int j) -> bool {
+      const int item = snake_item(j, G, (int)blockIdx.x);
+      const int qb = j & 1;
+      if (!mbar_wait_warp<SM_SPIN>(B_(DQ_QD_FULL + qb), (j >> 1) & 1, abort_flag, p.err, 0x5c00u)) return false;
+      const uint8_t* dor = gbase + DQ_Q + (3 * qb + 1) * FA_TILE_BYTES + r * 128;
+      const uint8_t* orow = dor + FA_TILE_BYTES;
+      float dl = 0.f;
 #pragma unroll
-      for (int c = 0; c < OC / 16; ++c) tmem_ld16(tdQ + t_lane + part * OC + c * 16, rr + c * 16);
-      tmem_wait_ld();
-      tcgen05_fence_before();
-      __syncwarp();
-      if (lane == 0) mbar_arrive(B_(13));           // dQ may be overwritten
-      {
-        uint4 hv[OC / 8];
+      for (int c = 0; c < 8; ++c) {
+        const uint32_t off = ((uint32_t)c ^ (uint32_t)(r & 7)) << 4;
+        const uint4 a = *reinterpret_cast<const uint4*>(dor + off);
+        const uint4 o = *reinterpret_cast<const uint4*>(orow + off);
+        const __half2* ah = reinterpret_cast<const __half2*>(&a);
+        const __half2* oh = reinterpret_cast<const __half2*>(&o);
 #pragma unroll
-        for (int u = 0; u < OC / 8; ++u) {
-          __half2 h2[4];
-#pragma unroll
-          for (int e = 0; e < 4; ++e)
-            h2[e] = __floats2half2_rn(__uint_as_float(rr[u * 8 + 2 * e]),
-                                      __uint_as_float(rr[u * 8 + 2 * e + 1]));
-          hv[u] = *reinterpret_cast<uint4*>(h2);
+        for (int e = 0; e < 4; ++e) {
+          const float2 x = __half22float2(ah[e]), y = __half22float2(oh[e]);
+          dl = fmaf(x.x, y.x, dl);
+          dl = fmaf(x.y, y.y, dl);
         }
-        const int q_w = qt * FA_T + (warp & 3) * 32;   // first query row of this warp's 32
-        __half* dst = p.dqkv + (size_t)(row0 + q_w) * 3 * p.D + h * FA_HD + part * OC;
-        warp_store_rows<OC / 8>(hv, gbase + DQ_OUT + (warp - 2) * (OC * 64), lane,
-                                reinterpret_cast<uint8_t*>(dst), (size_t)3 * p.D * 2, p.T - q_w);
       }
-      if (p.colsum) {
-        float val[OC];
-#pragma unroll
-        for (int c = 0; c < OC; ++c)
-          val[c] = q_ok ? __half2float(__float2half_rn(__uint_as_float(rr[c]))) : 0.f;
-        float* dst = p.colsum + ((size_t)(b * p.nqt + qt) * 4 + (warp & 3)) * 3 * p.D + h * FA_HD +
-                     part * OC;
-        warp_col_sums<OC>(val, lane, dst);
+      delta_s[qb * FA_T + r] = dl;
+      const int qi = (p.nqt - 1 - item / HB) * FA_T + r;
+      if (qi < p.T) p.delta_out[(size_t)(item % HB) * p.T + qi] = dl;
+      __syncwarp();
+      if (lane == 0) {
+        mbar_arrive(B_(DQ_DL_FULL + qb));
+        mbar_arrive(B_(DQ_OD_FREE + qb));
       }
       return true;
     };
-    // statistics of this thread's query row in an item
+    bool ok = (int)blockIdx.x < n_items && form_delta(0);
+    for (int j = 0; ok; ++j) {
+      const int item = snake_item(j, G, (int)blockIdx.x);
+      if (item >= n_items) break;
+      if (snake_item(j + 1, G, (int)blockIdx.x) >= n_items) break;   // the last one: see the softmax warps
+      ok = form_delta(j + 1);
+      if (!ok) break;
+      const int qt = p.nqt - 1 - item / HB, hb = item % HB;
+      const int h = hb % p.H, b = hb / p.H;
+      const int ab = j & 1;
+      if (!mbar_wait_warp<SM_SPIN>(B_(DQ_OUT_FULL + ab), (j >> 1) & 1, abort_flag, p.err, 0x5800u)) break;
+      tcgen05_fence_after();
+      stage_acc<8>(tdQ + 64 * ab + (((uint32_t)(w * 32)) << 16), stage, lane);
+      tcgen05_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(B_(DQ_ACC_FREE + ab));     // dQ may be overwritten
+      const int q_w = qt * FA_T + w * 32;                   // first query row of this warp's 32
+      __half* dst = p.dqkv + (size_t)(b * p.T + q_w) * 3 * p.D + h * FA_HD;
+      store_staged<8>(stage, lane, reinterpret_cast<uint8_t*>(dst), (size_t)3 * p.D * 2, p.T - q_w,
+                      p.colsum ? p.colsum + ((size_t)(b * p.nqt + qt) * 4 + w) * 3 * p.D + h * FA_HD : nullptr);
+      __syncwarp();                                         // the staging is filled again
+    }
+  } else {
+    regs_more<BW_REGS_SM>();
+    const int part = (warp - BW_SM_WARP) >> 2;   // which 32 of a key tile's 128 keys
+    const int r = (warp & 3) * 32 + lane;
+    const uint32_t t_lane = ((uint32_t)((warp & 3) * 32)) << 16;
+    const float* delta_s = reinterpret_cast<const float*>(gbase + DQ_DELTA);
+    bool ok = true;
+    // statistics of this thread's query row in an item, fetched one item ahead
     auto item_stat = [&](int item, float& lse, int& st) {
       const int qt = p.nqt - 1 - item / HB, hb = item % HB;
       const int qi = qt * FA_T + r;
       const bool q_ok = qi < p.T;
-      const size_t i = (size_t)((hb / p.H) * p.H + hb % p.H) * p.T + (q_ok ? qi : 0);
-      lse = p.lse2[i];
+      lse = p.lse2[(size_t)hb * p.T + (q_ok ? qi : 0)];
       st = (p.seg && q_ok) ? (int)p.seg[(hb / p.H) * p.T + qi] : 0;
     };
     float lse_f = 0.f;
     int st_f = 0;
     if ((int)blockIdx.x < n_items) item_stat((int)blockIdx.x, lse_f, st_f);
-    int g = 0, j = 0;
+    int g = 0, j = 0, last = -1;
+    bool ready = false;          // as in the dK / dV kernel
     for (;; ++j) {
       const int item = snake_item(j, G, (int)blockIdx.x);
       if (item >= n_items || !ok) break;
       const int qt = p.nqt - 1 - item / HB, nj = qt + 1;
       const int qi = qt * FA_T + r;
-      const bool q_ok = qi < p.T;
-      // this row's statistics were fetched while the previous item was being worked on
-      const float nlse = q_ok ? -lse_f : -INFINITY;
+      last = item;
+      // a row past the end of the sequence gets lse = +inf, hence P = 0 and dS = 0
+      const float nlse = qi < p.T ? -lse_f : -INFINITY;
       const int st = st_f;
       {
         const int nxt = snake_item(j + 1, G, (int)blockIdx.x);
         if (nxt < n_items) item_stat(nxt, lse_f, st_f);
       }
-      // delta of this row from the item's dO and O tiles (128-byte rows, 16-byte pieces XOR-ed
-      // with the row's low three bits, as the tensor map wrote them)
-      ok = mbar_wait_warp<SM_SPIN>(B_(0), j & 1, abort_flag, p.err, 0x5c00u);
+      ok = mbar_wait_warp<SM_SPIN>(B_(DQ_DL_FULL + (j & 1)), (j >> 1) & 1, abort_flag, p.err, 0x5d00u);
       if (!ok) break;
-      float dl = 0.f;
-      {
-        const uint8_t* dor = gbase + DQ_DO + r * 128;
-        const uint8_t* orow = gbase + DQ_O + r * 128;
-#pragma unroll
-        for (int c = 0; c < 8; ++c) {
-          const uint32_t off = ((uint32_t)c ^ (uint32_t)(r & 7)) << 4;
-          const uint4 a = *reinterpret_cast<const uint4*>(dor + off);
-          const uint4 o = *reinterpret_cast<const uint4*>(orow + off);
-          const __half2* ah = reinterpret_cast<const __half2*>(&a);
-          const __half2* oh = reinterpret_cast<const __half2*>(&o);
-#pragma unroll
-          for (int e = 0; e < 4; ++e) {
-            const float2 x = __half22float2(ah[e]), y = __half22float2(oh[e]);
-            dl = fmaf(x.x, y.x, dl);
-            dl = fmaf(x.y, y.y, dl);
-          }
-        }
-      }
-      __syncwarp();
-      if (lane == 0) mbar_arrive(B_(1));             // this warp is done with the dO / O tiles
-      if (part == 0 && q_ok) {
-        const int hb = item % HB;
-        p.delta_out[(size_t)((hb / p.H) * p.H + hb % p.H) * p.T + qi] = dl;
-      }
-      const float dsc = -dl * p.scale;
+      const float dsc = -delta_s[(j & 1) * FA_T + r] * p.scale;
       for (int kt = 0; kt < nj && ok; ++kt, ++g) {
-        const bool need_mask = (kt == qt) || (p.seg != nullptr);
-        ok = mbar_wait_warp<SM_SPIN>(B_(5), g & 1, abort_flag, p.err, 0x5600u);
+        ok = ready || mbar_wait_warp<SM_SPIN>(B_(DQ_SDP_FULL), g & 1, abort_flag, p.err, 0x5600u);
         if (!ok) break;
         tcgen05_fence_after();
-        uint32_t rs[CPT], rdp[CPT];
-#pragma unroll
-        for (int c = 0; c < CPT / 16; ++c) tmem_ld16(tS + t_lane + part * CPT + c * 16, rs + c * 16);
-#pragma unroll
-        for (int c = 0; c < CPT / 16; ++c) tmem_ld16(tdP + t_lane + part * CPT + c * 16, rdp + c * 16);
+        uint32_t rs[32], rdp[32];
+        tmem_ld16(tS + t_lane + part * 32, rs);
+        tmem_ld16(tS + t_lane + part * 32 + 16, rs + 16);
+        tmem_ld16(tdP + t_lane + part * 32, rdp);
+        tmem_ld16(tdP + t_lane + part * 32 + 16, rdp + 16);
         tmem_wait_ld();
         tcgen05_fence_before();
         __syncwarp();
-        if (lane == 0) mbar_arrive(B_(6));
+        if (lane == 0) mbar_arrive(B_(DQ_SDP_FREE));
         // dS as fp16 pairs, overwriting the scores they came from
-        const int key0 = kt * FA_T + part * CPT;
-#pragma unroll
-        for (int c = 0; c < CPT / 32; ++c) {
-          if (need_mask)
-            bwd_ds_pack<true>(rs + 32 * c, rdp + 32 * c, key0 + 32 * c, qi, st, p.cscale, p.scale, nlse, dsc,
-                              rs + 16 * c);
-          else
-            bwd_ds_pack<false>(rs + 32 * c, rdp + 32 * c, 0, 0, 0, p.cscale, p.scale, nlse, dsc, rs + 16 * c);
-        }
+        const int key0 = kt * FA_T + part * 32;
+        const bool need_mask = (kt == qt) || (p.seg != nullptr);
+        if (need_mask) bwd_ds_pack<true>(rs, rdp, key0, qi, st, p.cscale, p.scale, nlse, dsc, rs);
+        else bwd_ds_pack<false>(rs, rdp, 0, 0, 0, p.cscale, p.scale, nlse, dsc, rs);
         const int pb = g & 1;
+        ready = mbar_test_wait(B_(DQ_DS_FREE + pb), ((g >> 1) & 1) ^ 1u) != 0;
+        if (need_mask) bwd_ds_pack<true>(rs + 16, rdp + 16, key0 + 16, qi, st, p.cscale, p.scale, nlse, dsc, rs + 8);
+        else bwd_ds_pack<false>(rs + 16, rdp + 16, 0, 0, 0, p.cscale, p.scale, nlse, dsc, rs + 8);
         // dQ of step g - 2 has read this dS area
-        ok = mbar_wait_warp<SM_SPIN>(B_(8 + 3 * pb), ((g >> 1) & 1) ^ 1u, abort_flag, p.err, 0x5700u);
+        ok = __all_sync(0xffffffffu, ready) ||
+             mbar_wait_warp<SM_SPIN>(B_(DQ_DS_FREE + pb), ((g >> 1) & 1) ^ 1u, abort_flag, p.err, 0x5700u);
         if (!ok) break;
         tcgen05_fence_after();
-#pragma unroll
-        for (int c = 0; c < CPT / 32; ++c)
-          tmem_st16(tdS + 64 * pb + t_lane + part * (CPT / 2) + c * 16, rs + 16 * c);
+        tmem_st16(tdS + 64 * pb + t_lane + part * 16, rs);
+        ready = mbar_test_wait(B_(DQ_SDP_FULL), (g & 1) ^ 1u) != 0;
         tmem_wait_st();
         tcgen05_fence_before();
         __syncwarp();
-        if (lane == 0) mbar_arrive(B_(7 + 3 * pb));
-        if (pend_item >= 0) {
-          if (warp - 2 < OUT_WARPS) ok = store_item(pend_item, pend_j);
-          pend_item = -1;
-        }
+        if (lane == 0) mbar_arrive(B_(DQ_DS_FULL + pb));
+        ready = __all_sync(0xffffffffu, ready);
       }
-      pend_item = item;       // read this item's dQ out after the next item's first step
-      pend_j = j;
     }
-    if (ok && pend_item >= 0 && warp - 2 < OUT_WARPS) ok = store_item(pend_item, pend_j);
+    // the CTA's last item, as in the dK / dV kernel: 32 columns each by parts 0 and 1
+    const int la = (j - 1) & 1;
+    if (ok && last >= 0 && part < 2 &&
+        mbar_wait_warp<SM_SPIN>(B_(DQ_OUT_FULL + la), ((j - 1) >> 1) & 1, abort_flag, p.err, 0x5f00u)) {
+      tcgen05_fence_after();
+      uint8_t* stage = gbase + DQ_K + (warp - BW_SM_WARP) * 2048;
+      stage_acc<4>(tdQ + 64 * la + t_lane + part * 32, stage, lane);
+      __syncwarp();
+      const int qt = p.nqt - 1 - last / HB, hb = last % HB, b = hb / p.H;
+      const int q_w = qt * FA_T + (warp & 3) * 32;
+      const int col = (hb % p.H) * FA_HD + part * 32;
+      store_staged<4>(stage, lane, reinterpret_cast<uint8_t*>(p.dqkv + (size_t)(b * p.T + q_w) * 3 * p.D + col),
+                      (size_t)3 * p.D * 2, p.T - q_w,
+                      p.colsum ? p.colsum + ((size_t)(b * p.nqt + qt) * 4 + (warp & 3)) * 3 * p.D + col : nullptr);
+    }
   }
   __syncwarp();
   tcgen05_fence_before();
@@ -1469,7 +1521,7 @@ extern "C" int vkg_attn_bwd(vkg_device* dev, const void* qkv16, const void* dout
   const int sms = vkg_persistent_ctas(dev);
   const unsigned ctas = (unsigned)(n_items < sms ? n_items : sms);
   const unsigned family = VKG_K_ATTN_BWD | vkg_short_if(n_items <= sms);
-  VKG_CUDA(vkg_launch(dev, family, attn_bwd_q_kernel, dim3(ctas), dim3(DQ_THREADS), DQ_SMEM, 1, tm, tmdo, tmo, p));
+  VKG_CUDA(vkg_launch(dev, family, attn_bwd_q_kernel, dim3(ctas), dim3(BW_THREADS), DQ_SMEM, 1, tm, tmdo, tmo, p));
   if (vkg_check_launch("attn_bwd_q_kernel")) return 1;
   VKG_CUDA(vkg_launch(dev, family, attn_bwd_kv_kernel, dim3(ctas), dim3(BW_THREADS), KV_SMEM, 1, tm, tmdo, p));
   if (vkg_check_launch("attn_bwd_kv_kernel")) return 1;
