@@ -155,3 +155,48 @@ def test_backward(dev, B, T, H, packed):
         assert relerr(got[:, sl], merge(ref)) < 3e-3, name
     for x in (bq, bdo, bo, bl, bdelta, bdq) + (() if bs is None else (bs,)):
         x.destroy()
+
+
+# Packed batches pass over tiles that lie before every row's sample: the edges of that rule are tiles with
+# one row left over, starts on tile borders, and starts in no order at all (nothing sorts them).  The
+# last case gives a CTA several items.
+@pytest.mark.parametrize("B,T,H", [(3, 513, 2), (2, 1000, 8), (1, 385, 60)])
+@pytest.mark.parametrize("starts", ["samples", "tiles", "unordered"])
+def test_packed_tiles(dev, B, T, H, starts):
+    from vkgrad_b200._lib import TUNE_ATTN_ONE_PASS
+    from vkgrad_b200.vk import _check
+    hd, D = 64, H * 64
+    rng = np.random.default_rng(T + H)
+    t = np.arange(T)
+    if starts == "samples":
+        cut = np.sort(rng.integers(0, T, (B, T // 60)), axis=1)
+        cut[:, 0] = 0
+        seg = np.stack([c[np.searchsorted(c, t, side="right") - 1] for c in cut])
+    elif starts == "tiles":
+        seg = np.tile(t // 128 * 128, (B, 1))
+    else:
+        seg = rng.integers(0, t + 1, (B, T))
+    seg = seg.astype(np.uint32)
+    qkv = rng.standard_normal((B * T, 3 * D)).astype(np.float16)
+    dout = (0.1 * rng.standard_normal((B * T, D))).astype(np.float16)
+    scale = 1.0 / np.sqrt(hd)
+    bq, bdo, bs = up(dev, qkv), up(dev, dout), up(dev, seg)
+    bo, bdq = up(dev, np.full((B * T, D), np.nan, np.float16)), up(dev, np.full((B * T, 3 * D), np.nan, np.float16))
+    bl, bdelta = (up(dev, np.zeros((B * H, T), np.float32)) for _ in range(2))
+    _check(dev.lib.vkg_set_tuning(dev.handle, TUNE_ATTN_ONE_PASS, 1), "tune")
+    _check(dev.lib.vkg_attn_fwd(dev.handle, bq.dptr, bs.dptr, bo.dptr, bl.dptr, B, T, H, hd, scale), "attn_fwd")
+    _check(dev.lib.vkg_attn_bwd(dev.handle, bq.dptr, bdo.dptr, bo.dptr, bl.dptr, bs.dptr, bdq.dptr, bdelta.dptr,
+                                None, None, B, T, H, hd, scale), "attn_bwd")
+    dev.sync()
+    q, k, v, p, o, lse2, _ = reference_attention(qkv, B, T, H, scale, seg)
+    assert relerr(get(bo, np.float16, (B * T, D)).astype(np.float32), o) < 2e-3
+    assert np.abs(get(bl, np.float32, (B, H, T)) - lse2).max() < 1e-3
+    dao = dout.astype(np.float32).reshape(B, T, H, hd).transpose(0, 2, 1, 3)
+    dp = dao @ v.transpose(0, 1, 3, 2)
+    ds = orc.r16(p * (dp - (dp * p).sum(-1, keepdims=True)) * scale)
+    got = get(bdq, np.float16, (B * T, 3 * D)).astype(np.float32)
+    merge = lambda x: x.transpose(0, 2, 1, 3).reshape(B * T, D)
+    for i, ref in enumerate((ds @ k, ds.transpose(0, 1, 3, 2) @ q, p.transpose(0, 1, 3, 2) @ dao)):
+        assert relerr(got[:, i * D:(i + 1) * D], merge(ref)) < 3e-3, "qkv"[i]
+    for x in (bq, bdo, bs, bo, bdq, bl, bdelta):
+        x.destroy()

@@ -53,6 +53,7 @@ struct AttnParams {
   float cscale;            // softmax scale * log2(e)
   float scale;
   const uint32_t* seg;     // optional packed-sample starts (b*T + t)
+  int skip_tiles;          // packed, and worth looking for tiles that are wholly masked
   __half* out;             // forward: O, head-merged (rows, D)
   float* lse2;             // (B*H, T): row log2-sum-exp of the scaled scores
   const float* delta;      // backward: rowsum(dO * O), (B*H, T); the dQ kernel writes it (delta_out),
@@ -75,6 +76,34 @@ constexpr int FW_SMEM = FW_XCHG + 4096 + 1024 + 1024;
 
 // P and dS tiles use the 128B-swizzled layout of TMA and the UMMA descriptors: 16-byte
 // piece c8 (8 keys) of row r of a 64-key block sits at r * 128 + ((c8 ^ (r & 7)) << 4).
+
+// Packed batches: the smallest sample start among a query tile's rows, taken by one warp.  Key tiles
+// that lie wholly before it are masked for every row; what they would add is exactly zero, so the
+// kernels pass over them.  Nothing is assumed about the order of the starts.
+__device__ __forceinline__ int tile_first_start(const uint32_t* seg, int q0, int T, int lane) {
+  uint32_t v = 0x7fffffffu;
+#pragma unroll
+  for (int i = 0; i < FA_T / 32; ++i) {
+    const int q = q0 + i * 32 + lane;
+    if (q < T) v = min(v, seg[q]);
+  }
+  return (int)__reduce_min_sync(0xffffffffu, v);
+}
+constexpr int SEG_ITEMS = 64, SEG_TILES = 32;      // items of a CTA, tiles of a sequence this is done for
+// Reading the starts takes a kernel half a microsecond before its first load.  From three tiles to a
+// sequence on it saves more (2 x 700 tokens, 6 heads, samples of 170: forward 17.5 -> 14.1 us); one or
+// two tiles rarely have one to pass over.
+int skip_tiles(const uint32_t* seg, int nqt) { return seg && nqt > 2 && nqt <= SEG_TILES; }
+
+// What the causal rule and the sample starts leave of a warp's block of nq queries from q0 on and nk keys
+// from k0 on, the starts lying in st_min .. st_max: everything, some of it (tested element by element),
+// or nothing (no arithmetic at all).  Packed batches only: with the causal rule alone, where one tile in
+// several has such blocks, the extra paths measured more than they saved (8 x 1024 x 12, dK / dV: 49 -> 63 us).
+enum : int { BLOCK_ALL, BLOCK_SOME, BLOCK_NONE };
+__device__ __forceinline__ int block_class(int q0, int nq, int k0, int nk, int st_min, int st_max) {
+  if (k0 > q0 + nq - 1 || st_min > k0 + nk - 1) return BLOCK_NONE;
+  return k0 + nk - 1 <= q0 && st_max <= k0 ? BLOCK_ALL : BLOCK_SOME;
+}
 
 // Row maximum over this thread's 64 raw scores of one key tile.  MASK adds the causal /
 // packed-sample test and is compiled only into the tiles that need it.
@@ -400,6 +429,7 @@ constexpr int F1_K = FW_K, F1_V = F1_K + F1_K_STAGES * FA_TILE_BYTES;
 constexpr int F1_OUT = F1_V;          // output staging, once every product has retired
 static_assert(F1_V + F1_V_STAGES * FA_TILE_BYTES <= FW_BAR, "one-pass forward: shared memory");
 
+template <bool PACKED>
 __global__ void __launch_bounds__(FA_THREADS, 2)
 attn_fwd1_kernel(const __grid_constant__ CUtensorMap tm, const AttnParams p) {
   extern __shared__ __align__(1024) uint8_t smem_raw[];
@@ -437,6 +467,16 @@ attn_fwd1_kernel(const __grid_constant__ CUtensorMap tm, const AttnParams p) {
   __syncthreads();
   tcgen05_fence_after();
   pdl_wait();
+  int j0 = 0;                      // first key tile that counts
+  if (PACKED && p.skip_tiles) {
+    volatile int* slot = reinterpret_cast<volatile int*>(gbase + FW_BAR + 144);
+    if (warp == 0) {
+      const int st = tile_first_start(p.seg + row0, q0, p.T, lane);
+      if (lane == 0) *slot = min(st / FA_T, qt);
+    }
+    __syncthreads();
+    j0 = *slot;
+  }
   const uint32_t tmem = *tmem_slot;
   const uint32_t tS = tmem, tO = tmem + 128, tP = tmem + 192;   // P~: 128 keys, two per column
 
@@ -446,7 +486,7 @@ attn_fwd1_kernel(const __grid_constant__ CUtensorMap tm, const AttnParams p) {
       tma_load_2d(base + FW_Q, &tm, B_(0), h * FA_HD, row0 + q0);
       int ks = 0;
       uint32_t kph = 0;
-      for (int j = 0; j < nj; ++j) {
+      for (int j = j0, n = 0; j < nj; ++j, ++n) {
         if (!mbar_wait<true>(B_(12 + ks), kph ^ 1u, abort_flag, p.err, 0x6100u + ks)) break;
         mbar_expect_tx(B_(5 + ks), FA_TILE_BYTES);
         tma_load_2d(base + F1_K + ks * FA_TILE_BYTES, &tm, B_(5 + ks), p.D + h * FA_HD, row0 + j * FA_T);
@@ -454,8 +494,8 @@ attn_fwd1_kernel(const __grid_constant__ CUtensorMap tm, const AttnParams p) {
           ks = 0;
           kph ^= 1u;
         }
-        const int vs = j & 1;
-        if (!mbar_wait<true>(B_(3 + vs), ((j >> 1) & 1) ^ 1u, abort_flag, p.err, 0x6200u + vs)) break;
+        const int vs = n & 1;
+        if (!mbar_wait<true>(B_(3 + vs), ((n >> 1) & 1) ^ 1u, abort_flag, p.err, 0x6200u + vs)) break;
         mbar_expect_tx(B_(1 + vs), FA_TILE_BYTES);
         tma_load_2d(base + F1_V + vs * FA_TILE_BYTES, &tm, B_(1 + vs), 2 * p.D + h * FA_HD, row0 + j * FA_T);
       }
@@ -487,8 +527,8 @@ attn_fwd1_kernel(const __grid_constant__ CUtensorMap tm, const AttnParams p) {
     };
     int n = 0;
     if (ok) ok = issue_s(n++);
-    for (int j = 0; j < nj && ok; ++j) {
-      if (j + 1 < nj) {          // the next scores first: the tensor core works while P(j) forms
+    for (int j = 0; j0 + j < nj && ok; ++j) {
+      if (j0 + j + 1 < nj) {     // the next scores first: the tensor core works while P(j) forms
         ok = issue_s(n++);
         if (!ok) break;
       }
@@ -508,15 +548,20 @@ attn_fwd1_kernel(const __grid_constant__ CUtensorMap tm, const AttnParams p) {
     const int qr = (warp & 3) * 32 + lane;      // row within the tile = TMEM lane
     const int qi = q0 + qr;
     const bool q_ok = qi < p.T;
-    const int st = (p.seg && q_ok) ? (int)p.seg[row0 + qi] : 0;
+    const int st = (PACKED && q_ok) ? (int)p.seg[row0 + qi] : 0;
+    const int st_min = PACKED ? __reduce_min_sync(0xffffffffu, st) : 0;
+    const int st_max = PACKED ? __reduce_max_sync(0xffffffffu, st) : 0;
     const uint32_t t_lane = ((uint32_t)((warp & 3) * 32)) << 16;
     float m_ref = -1e30f, l = 0.f;              // reference maximum (scaled units), row sum
     bool ok = true;
-    for (int j = 0; j < nj && ok; ++j) {
-      ok = mbar_wait_warp<SM_SPIN>(B_(15), j & 1, abort_flag, p.err, 0x8100u);
+    for (int n = 0; j0 + n < nj && ok; ++n) {
+      const int j = j0 + n;
+      ok = mbar_wait_warp<SM_SPIN>(B_(15), n & 1, abort_flag, p.err, 0x8100u);
       if (!ok) break;
       tcgen05_fence_after();
-      const bool need_mask = (j == qt) || (p.seg != nullptr);
+      const int key0 = j * FA_T + half * 64;
+      const int cls = PACKED ? block_class(q0 + (warp & 3) * 32, 32, key0, 64, st_min, st_max)
+                             : j == qt ? BLOCK_SOME : BLOCK_ALL;
       uint32_t r[64];
 #pragma unroll
       for (int c = 0; c < 4; ++c) tmem_ld16(tS + t_lane + half * 64 + c * 16, r + c * 16);
@@ -525,8 +570,9 @@ attn_fwd1_kernel(const __grid_constant__ CUtensorMap tm, const AttnParams p) {
       __syncwarp();
       if (lane == 0) mbar_arrive(B_(8));        // S may be overwritten
       // this half's maximum of the row, then the partner's through its tagged slot
-      float mt = need_mask ? fwd_max_tile<true>(r, j * FA_T + half * 64, qi, st, -1e30f)
-                           : fwd_max_tile<false>(r, 0, 0, 0, -1e30f);
+      float mt = -1e30f;
+      if (cls == BLOCK_SOME) mt = fwd_max_tile<true>(r, key0, qi, st, mt);
+      else if (!PACKED || cls == BLOCK_ALL) mt = fwd_max_tile<false>(r, 0, 0, 0, mt);
       const unsigned long long tag = (unsigned long long)(unsigned)(j + 1) << 32;
       xslot[((j & 1) * 2 + half) * FA_T + qr] = tag | (unsigned long long)__float_as_uint(mt);
       float mo = -1e30f;
@@ -556,9 +602,9 @@ attn_fwd1_kernel(const __grid_constant__ CUtensorMap tm, const AttnParams p) {
       if (!ok) break;
       const float m_row = fmaxf(mt, mo) * p.cscale;
       // the previous P V has retired: the P buffer is free and O~ is quiet
-      ok = mbar_wait_warp<SM_SPIN>(B_(10), (j & 1) ^ 1u, abort_flag, p.err, 0x8200u);
+      ok = mbar_wait_warp<SM_SPIN>(B_(10), (n & 1) ^ 1u, abort_flag, p.err, 0x8200u);
       if (!ok) break;
-      if (j == 0) {
+      if (n == 0) {
         m_ref = m_row;
       } else {
         const bool grow = m_row > m_ref + FW1_LAZY;
@@ -583,8 +629,14 @@ attn_fwd1_kernel(const __grid_constant__ CUtensorMap tm, const AttnParams p) {
       const float nm = -m_ref;
       // P~ packed two keys per register, overwriting the scores they came from, then into
       // this half's 32 columns of the P~ area
-      if (need_mask) l += fwd_p_pack<true>(r, j * FA_T + half * 64, qi, st, p.cscale, nm);
-      else l += fwd_p_pack<false>(r, 0, 0, 0, p.cscale, nm);
+      if (cls == BLOCK_SOME) {
+        l += fwd_p_pack<true>(r, key0, qi, st, p.cscale, nm);
+      } else if (!PACKED || cls == BLOCK_ALL) {
+        l += fwd_p_pack<false>(r, 0, 0, 0, p.cscale, nm);
+      } else {
+#pragma unroll
+        for (int i = 0; i < 32; ++i) r[i] = 0u;
+      }
       tmem_st16(tP + t_lane + half * 32, r);
       tmem_st16(tP + t_lane + half * 32 + 16, r + 16);
       tmem_wait_st();
@@ -744,7 +796,8 @@ constexpr int KV_K = 0,                                        // two buffers of
               KV_OUT = (4 + 2 * KV_STAGES) * FA_TILE_BYTES,    // staging: dV and dK of 32 keys per epilogue warp
               KV_STAT = KV_OUT + BW_EPI_WARPS * 8192,          // (-lse, -delta scale) of 32 queries per softmax warp
               KV_SEG = KV_STAT + BW_SM_WARPS * 256,            // and where their samples start
-              KV_BAR = KV_SEG + BW_SM_WARPS * 128, KV_SMEM = KV_BAR + 256 + 1024;
+              KV_TILES = KV_SEG + BW_SM_WARPS * 128,           // packed: the query tiles of each item that count
+              KV_BAR = KV_TILES + SEG_ITEMS * 4, KV_SMEM = KV_BAR + 256 + 1024;
 static_assert(KV_SMEM <= 227 * 1024, "dK / dV kernel: shared memory");
 constexpr int KV_KV_FULL = 0, KV_KV_FREE = 2, KV_SDP_FULL = 4, KV_SDP_FREE = 5, KV_PDS_FULL = 6, KV_PDS_FREE = 7,
               KV_OUT_FULL = 8, KV_ACC_FREE = 9, KV_QD_FULL = 10, KV_QD_EMPTY = 10 + KV_STAGES,
@@ -763,6 +816,7 @@ __device__ __forceinline__ void bwd_pds_pack(const uint32_t* rs, const uint32_t*
 #pragma unroll
   for (int i = 0; i < 8; ++i) {
     const float4 s2 = stat[i];
+    const int2 sg = MASK == 2 ? reinterpret_cast<const int2*>(seg)[i] : make_int2(0, 0);
     const float nlse[2] = {s2.x, s2.z}, dsc[2] = {s2.y, s2.w};
     float pv[2], dv[2];
 #pragma unroll
@@ -770,7 +824,9 @@ __device__ __forceinline__ void bwd_pds_pack(const uint32_t* rs, const uint32_t*
       const int idx = 2 * i + w;
       float pr = vkg_ex2(fmaf(__uint_as_float(rs[idx]), cscale, nlse[w]));
       if (MASK) {
-        if (key > q0 + idx || (MASK == 2 && key < seg[idx])) pr = 0.f;
+        bool off = key > q0 + idx;
+        if (MASK == 2) off |= key < (w ? sg.y : sg.x);     // not ||, which makes a branch of the load
+        if (off) pr = 0.f;
       }
       pv[w] = pr;
       dv[w] = pr * fmaf(__uint_as_float(rdp[idx]), scale, dsc[w]);
@@ -781,6 +837,15 @@ __device__ __forceinline__ void bwd_pds_pack(const uint32_t* rs, const uint32_t*
   }
 }
 
+// Query tile after `it` (counted from the item's first) that counts; ni past the last one.
+__device__ __forceinline__ int next_tile(bool skip, uint32_t tiles, int it, int ni) {
+  ++it;
+  if (!skip || it >= ni) return it;
+  const uint32_t left = tiles >> it;
+  return left ? it + __ffs((int)left) - 1 : ni;
+}
+
+template <bool PACKED>
 __global__ void __launch_bounds__(BW_THREADS, 1)
 attn_bwd_kv_kernel(const __grid_constant__ CUtensorMap tm, const __grid_constant__ CUtensorMap tmdo,
                    const AttnParams p) {
@@ -810,6 +875,27 @@ attn_bwd_kv_kernel(const __grid_constant__ CUtensorMap tm, const __grid_constant
   __syncthreads();
   tcgen05_fence_after();
   pdl_wait();
+  // packed: bit i of an item's entry says that query tile kt + i has a row whose sample begins before
+  // the end of key tile kt; the diagonal tile always counts
+  const bool skip = PACKED && p.skip_tiles;
+  uint32_t* tiles_s = reinterpret_cast<uint32_t*>(gbase + KV_TILES);
+  if (skip) {
+    if (threadIdx.x < SEG_ITEMS) tiles_s[threadIdx.x] = 1u;
+    __syncthreads();
+    // one (item, query tile) per warp and round: 700 cycles each, the wait for the starts
+    constexpr int WARPS = BW_THREADS / 32;
+    for (int j = 0; j < SEG_ITEMS; ++j) {
+      const int item = snake_item(j, G, (int)blockIdx.x);
+      if (item >= n_items) break;
+      const int kt = item / HB, ni = p.nqt - kt;
+      for (int i = 1 + (warp + 5 * j) % WARPS; i < ni; i += WARPS) {
+        const int st = tile_first_start(p.seg + ((item % HB) / p.H) * p.T, (kt + i) * FA_T, p.T, lane);
+        if (lane == 0 && st < (kt + 1) * FA_T) atomicOr(&tiles_s[j], 1u << i);
+      }
+    }
+    __syncthreads();
+  }
+  auto item_tiles = [&](int j) { return skip && j < SEG_ITEMS ? tiles_s[j] : ~0u; };
   const uint32_t tmem = *tmem_slot;
   const uint32_t tS = tmem, tdP = tmem + 128, tdV = tmem + 256, tdK = tmem + 320, tP = tmem + 384, tdS = tmem + 448;
 
@@ -833,7 +919,8 @@ attn_bwd_kv_kernel(const __grid_constant__ CUtensorMap tm, const __grid_constant
           tma_load_2d(base + KV_K + (2 * kb) * FA_TILE_BYTES, &tm, B_(KV_KV_FULL + kb), p.D + h * FA_HD, row0 + k0);
           tma_load_2d(base + KV_K + (2 * kb + 1) * FA_TILE_BYTES, &tm, B_(KV_KV_FULL + kb), 2 * p.D + h * FA_HD,
                       row0 + k0);
-          for (int it = 0; it < ni; ++it) {
+          const uint32_t tiles = item_tiles(j);
+          for (int it = 0; it < ni; it = next_tile(skip, tiles, it, ni)) {
             if (!mbar_wait<true>(B_(KV_QD_EMPTY + s), ph ^ 1u, abort_flag, p.err, 0x4100u + s)) {
               ok = false;
               break;
@@ -867,7 +954,9 @@ attn_bwd_kv_kernel(const __grid_constant__ CUtensorMap tm, const __grid_constant
         const int kb = j & 1;
         const uint32_t ko = (uint32_t)(2 * kb) * (FA_TILE_BYTES >> 4);
         ok = mbar_wait_warp<true>(B_(KV_KV_FULL + kb), (j >> 1) & 1, abort_flag, p.err, 0x4200u);
-        for (int it = 0; it < ni && ok; ++it) {
+        const uint32_t tiles = item_tiles(j);
+        for (int it = 0, next; it < ni && ok; it = next) {
+          next = next_tile(skip, tiles, it, ni);
           ok = mbar_wait_warp<true>(B_(KV_QD_FULL + s), ph, abort_flag, p.err, 0x4300u + s) &&
                mbar_wait_warp<true>(B_(KV_SDP_FREE), par ^ 1u, abort_flag, p.err, 0x4400u);
           if (!ok) break;
@@ -876,7 +965,7 @@ attn_bwd_kv_kernel(const __grid_constant__ CUtensorMap tm, const __grid_constant
           umma_f16_chain<4>(tS, k_lo + ko, 2, q_lo + so, 2, d_hi, idesc_s, 0u);
           umma_f16_chain<4>(tdP, v_lo + ko, 2, do_lo + so, 2, d_hi, idesc_s, 0u);
           umma_commit_one(B_(KV_SDP_FULL));
-          if (it == ni - 1) umma_commit_one(B_(KV_KV_FREE + kb));    // the item's K / V may be replaced
+          if (next >= ni) umma_commit_one(B_(KV_KV_FREE + kb));    // the item's K / V may be replaced
           par ^= 1u;
           if (++s == KV_STAGES) {
             s = 0;
@@ -897,7 +986,9 @@ attn_bwd_kv_kernel(const __grid_constant__ CUtensorMap tm, const __grid_constant
         const int item = snake_item(j, G, (int)blockIdx.x);
         if (item >= n_items) break;
         const int ni = p.nqt - item / HB;
-        for (int it = 0; it < ni; ++it, ++g) {
+        const uint32_t tiles = item_tiles(j);
+        for (int it = 0, next; it < ni; it = next, ++g) {
+          next = next_tile(skip, tiles, it, ni);
           ok = mbar_wait_warp<true>(B_(KV_PDS_FULL), g & 1, abort_flag, p.err, 0x4500u);     // P / dS written
           if (!ok) break;
           if (it == 0) {                       // the previous item's dV / dK have been read out
@@ -910,7 +1001,7 @@ attn_bwd_kv_kernel(const __grid_constant__ CUtensorMap tm, const __grid_constant
           umma_f16_ts_chain<8>(tdK, tdS, qm_lo + so, 128, d_hi, idesc_g, it ? 1u : 0u);
           umma_commit_one(B_(KV_QD_EMPTY + s));   // Q / dO stage free
           umma_commit_one(B_(KV_PDS_FREE));       // P / dS may be overwritten
-          if (it == ni - 1) umma_commit_one(B_(KV_OUT_FULL));
+          if (next >= ni) umma_commit_one(B_(KV_OUT_FULL));
           if (++s == KV_STAGES) s = 0;
         }
       }
@@ -965,7 +1056,7 @@ attn_bwd_kv_kernel(const __grid_constant__ CUtensorMap tm, const __grid_constant
       // a query past the end of the sequence gets lse = +inf, hence P = 0 and dS = 0
       lse_n = q_ok ? p.lse2[i] : INFINITY;
       dl_n = p.delta[i];
-      if (p.seg) st_n = q_ok ? (int)p.seg[(hb / p.H) * p.T + qi] : 0;
+      if (PACKED) st_n = q_ok ? (int)p.seg[(hb / p.H) * p.T + qi] : 0;
     };
     if ((int)blockIdx.x < n_items) fetch_stat((int)blockIdx.x % HB, (int)blockIdx.x / HB);
     int g = 0, last = -1, last_j = 0;
@@ -979,12 +1070,19 @@ attn_bwd_kv_kernel(const __grid_constant__ CUtensorMap tm, const __grid_constant
       const int key = kt * FA_T + r;
       last = item;
       last_j = j;
-      for (int qt = kt; qt < p.nqt && ok; ++qt, ++g) {
+      const uint32_t tiles = item_tiles(j);
+      for (int qt = kt, next; qt < p.nqt && ok; qt = next, ++g) {
+        next = kt + next_tile(skip, tiles, qt - kt, p.nqt - kt);
         stat[lane] = make_float2(-lse_n, -dl_n * p.scale);
-        if (p.seg) seg_s[lane] = st_n;
+        int cls = qt == kt ? BLOCK_SOME : BLOCK_ALL;
+        if (PACKED) {
+          seg_s[lane] = st_n;
+          cls = block_class(qt * FA_T + part * 32, 32, key - lane, 32, __reduce_min_sync(0xffffffffu, st_n),
+                            __reduce_max_sync(0xffffffffu, st_n));
+        }
         __syncwarp();
-        if (qt + 1 < p.nqt) {
-          fetch_stat(hb, qt + 1);
+        if (next < p.nqt) {
+          fetch_stat(hb, next);
         } else {
           const int nxt = snake_item(j + 1, G, (int)blockIdx.x);
           if (nxt < n_items) fetch_stat(nxt % HB, nxt / HB);
@@ -1004,13 +1102,18 @@ attn_bwd_kv_kernel(const __grid_constant__ CUtensorMap tm, const __grid_constant
         // P and dS, overwriting the scores and products they came from
         const float4* st4 = reinterpret_cast<const float4*>(stat);
         const int q0 = qt * FA_T + part * 32;
-        if (p.seg) bwd_pds_pack<2>(rs, rdp, st4, seg_s, q0, key, p.cscale, p.scale, rs, rdp);
-        else if (qt == kt) bwd_pds_pack<1>(rs, rdp, st4, nullptr, q0, key, p.cscale, p.scale, rs, rdp);
-        else bwd_pds_pack<0>(rs, rdp, st4, nullptr, 0, 0, p.cscale, p.scale, rs, rdp);
+        if (cls == BLOCK_SOME) bwd_pds_pack<PACKED ? 2 : 1>(rs, rdp, st4, seg_s, q0, key, p.cscale, p.scale, rs, rdp);
+        else if (!PACKED || cls == BLOCK_ALL) bwd_pds_pack<0>(rs, rdp, st4, nullptr, 0, 0, p.cscale, p.scale, rs, rdp);
         ready = mbar_test_wait(B_(KV_PDS_FREE), (g & 1) ^ 1u) != 0;
-        if (p.seg) bwd_pds_pack<2>(rs + 16, rdp + 16, st4 + 8, seg_s + 16, q0 + 16, key, p.cscale, p.scale, rs + 8, rdp + 8);
-        else if (qt == kt) bwd_pds_pack<1>(rs + 16, rdp + 16, st4 + 8, nullptr, q0 + 16, key, p.cscale, p.scale, rs + 8, rdp + 8);
-        else bwd_pds_pack<0>(rs + 16, rdp + 16, st4 + 8, nullptr, 0, 0, p.cscale, p.scale, rs + 8, rdp + 8);
+        if (cls == BLOCK_SOME) {
+          bwd_pds_pack<PACKED ? 2 : 1>(rs + 16, rdp + 16, st4 + 8, seg_s + 16, q0 + 16, key, p.cscale, p.scale, rs + 8,
+                                       rdp + 8);
+        } else if (!PACKED || cls == BLOCK_ALL) {
+          bwd_pds_pack<0>(rs + 16, rdp + 16, st4 + 8, nullptr, 0, 0, p.cscale, p.scale, rs + 8, rdp + 8);
+        } else {
+#pragma unroll
+          for (int i = 0; i < 16; ++i) rs[i] = rdp[i] = 0u;
+        }
         // dV / dK of step g - 1 done
         ok = __all_sync(0xffffffffu, ready) ||
              mbar_wait_warp<SM_SPIN>(B_(KV_PDS_FREE), (g & 1) ^ 1u, abort_flag, p.err, 0x4700u);
@@ -1076,7 +1179,8 @@ constexpr int DQ_Q = 0,                                        // two buffers of
               DQ_K = 6 * FA_TILE_BYTES, DQ_V = (6 + DQ_STAGES) * FA_TILE_BYTES,
               DQ_OUT = (6 + 2 * DQ_STAGES) * FA_TILE_BYTES,    // output staging, one tile
               DQ_DELTA = DQ_OUT + FA_TILE_BYTES,               // [2][128] floats
-              DQ_BAR = DQ_DELTA + 1024, DQ_SMEM = DQ_BAR + 256 + 1024;
+              DQ_FIRST = DQ_DELTA + 1024,                      // packed: the first key tile of each item that counts
+              DQ_BAR = DQ_FIRST + SEG_ITEMS * 4, DQ_SMEM = DQ_BAR + 256 + 1024;
 static_assert(DQ_SMEM <= 227 * 1024, "dQ kernel: shared memory");
 constexpr int DQ_QD_FULL = 0, DQ_QD_FREE = 2, DQ_OD_FREE = 4, DQ_DL_FULL = 6, DQ_SDP_FULL = 8, DQ_SDP_FREE = 9,
               DQ_DS_FULL = 10, DQ_DS_FREE = 12, DQ_OUT_FULL = 14, DQ_ACC_FREE = 16, DQ_KV_FULL = 18,
@@ -1106,6 +1210,7 @@ __device__ __forceinline__ void bwd_ds_pack(const uint32_t* rs, const uint32_t* 
   }
 }
 
+template <bool PACKED>
 __global__ void __launch_bounds__(BW_THREADS, 1)
 attn_bwd_q_kernel(const __grid_constant__ CUtensorMap tm, const __grid_constant__ CUtensorMap tmdo,
                   const __grid_constant__ CUtensorMap tmo, const AttnParams p) {
@@ -1139,6 +1244,18 @@ attn_bwd_q_kernel(const __grid_constant__ CUtensorMap tm, const __grid_constant_
   __syncthreads();
   tcgen05_fence_after();
   pdl_wait();
+  int* first_s = reinterpret_cast<int*>(gbase + DQ_FIRST);
+  if (PACKED && p.skip_tiles) {
+    for (int j = warp; j < SEG_ITEMS; j += BW_THREADS / 32) {
+      const int item = snake_item(j, G, (int)blockIdx.x);
+      if (item >= n_items) break;
+      const int qt = p.nqt - 1 - item / HB;
+      const int st = tile_first_start(p.seg + ((item % HB) / p.H) * p.T, qt * FA_T, p.T, lane);
+      if (lane == 0) first_s[j] = min(st / FA_T, qt);
+    }
+    __syncthreads();
+  }
+  auto item_first = [&](int j) { return PACKED && p.skip_tiles && j < SEG_ITEMS ? first_s[j] : 0; };
   const uint32_t tmem = *tmem_slot;
   const uint32_t tS = tmem, tdP = tmem + 128, tdQ = tmem + 256, tdS = tmem + 384;
 
@@ -1166,7 +1283,7 @@ attn_bwd_q_kernel(const __grid_constant__ CUtensorMap tm, const __grid_constant_
           tma_load_2d(qd, &tm, B_(DQ_QD_FULL + qb), h * FA_HD, row0 + q0);
           tma_load_2d(qd + FA_TILE_BYTES, &tmdo, B_(DQ_QD_FULL + qb), h * FA_HD, row0 + q0);
           tma_load_2d(qd + 2 * FA_TILE_BYTES, &tmo, B_(DQ_QD_FULL + qb), h * FA_HD, row0 + q0);
-          for (int kt = 0; kt < nj; ++kt) {
+          for (int kt = item_first(j); kt < nj; ++kt) {
             if (!mbar_wait<true>(B_(DQ_KV_EMPTY + s), ph ^ 1u, abort_flag, p.err, 0x5100u + s)) {
               ok = false;
               break;
@@ -1199,7 +1316,7 @@ attn_bwd_q_kernel(const __grid_constant__ CUtensorMap tm, const __grid_constant_
         const int qb = j & 1;
         const uint32_t qo = (uint32_t)(3 * qb) * (FA_TILE_BYTES >> 4);
         ok = mbar_wait_warp<true>(B_(DQ_QD_FULL + qb), (j >> 1) & 1, abort_flag, p.err, 0x5200u);
-        for (int kt = 0; kt < nj && ok; ++kt) {
+        for (int kt = item_first(j); kt < nj && ok; ++kt) {
           ok = mbar_wait_warp<true>(B_(DQ_KV_FULL + s), ph, abort_flag, p.err, 0x5300u + s) &&
                mbar_wait_warp<true>(B_(DQ_SDP_FREE), par ^ 1u, abort_flag, p.err, 0x5400u);
           if (!ok) break;
@@ -1232,18 +1349,19 @@ attn_bwd_q_kernel(const __grid_constant__ CUtensorMap tm, const __grid_constant_
         if (item >= n_items) break;
         const int nj = p.nqt - item / HB;
         const int ab = j & 1;
-        for (int kt = 0; kt < nj; ++kt, ++g) {
+        const int first = item_first(j);
+        for (int kt = first; kt < nj; ++kt, ++g) {
           const int pb = g & 1;
           ok = mbar_wait_warp<true>(B_(DQ_DS_FULL + pb), (g >> 1) & 1, abort_flag, p.err, 0x5500u);
           if (!ok) break;
-          if (kt == 0) {                        // dQ of the item before last has been read out
+          if (kt == first) {                    // dQ of the item before last has been read out
             ok = mbar_wait_warp<true>(B_(DQ_ACC_FREE + ab), ((j >> 1) & 1) ^ 1u, abort_flag, p.err, 0x5a00u);
             if (!ok) break;
           }
           tcgen05_fence_after();
           // K = 128 keys: dS from tensor memory (8 columns per step), K MN-major
           umma_f16_ts_chain<8>(tdQ + 64 * ab, tdS + 64 * pb, km_lo + (uint32_t)s * (FA_TILE_BYTES >> 4), 128, d_hi,
-                               idesc_q, kt ? 1u : 0u);
+                               idesc_q, kt != first ? 1u : 0u);
           umma_commit_one(B_(DQ_KV_EMPTY + s));   // K / V stage free
           umma_commit_one(B_(DQ_DS_FREE + pb));   // this dS area free
           if (kt == nj - 1) umma_commit_one(B_(DQ_OUT_FULL + ab));
@@ -1326,7 +1444,7 @@ attn_bwd_q_kernel(const __grid_constant__ CUtensorMap tm, const __grid_constant_
       const int qi = qt * FA_T + r;
       const bool q_ok = qi < p.T;
       lse = p.lse2[(size_t)hb * p.T + (q_ok ? qi : 0)];
-      st = (p.seg && q_ok) ? (int)p.seg[(hb / p.H) * p.T + qi] : 0;
+      st = (PACKED && q_ok) ? (int)p.seg[(hb / p.H) * p.T + qi] : 0;
     };
     float lse_f = 0.f;
     int st_f = 0;
@@ -1342,6 +1460,8 @@ attn_bwd_q_kernel(const __grid_constant__ CUtensorMap tm, const __grid_constant_
       // a row past the end of the sequence gets lse = +inf, hence P = 0 and dS = 0
       const float nlse = qi < p.T ? -lse_f : -INFINITY;
       const int st = st_f;
+      const int st_min = PACKED ? __reduce_min_sync(0xffffffffu, st) : 0;
+      const int st_max = PACKED ? __reduce_max_sync(0xffffffffu, st) : 0;
       {
         const int nxt = snake_item(j + 1, G, (int)blockIdx.x);
         if (nxt < n_items) item_stat(nxt, lse_f, st_f);
@@ -1349,7 +1469,7 @@ attn_bwd_q_kernel(const __grid_constant__ CUtensorMap tm, const __grid_constant_
       ok = mbar_wait_warp<SM_SPIN>(B_(DQ_DL_FULL + (j & 1)), (j >> 1) & 1, abort_flag, p.err, 0x5d00u);
       if (!ok) break;
       const float dsc = -delta_s[(j & 1) * FA_T + r] * p.scale;
-      for (int kt = 0; kt < nj && ok; ++kt, ++g) {
+      for (int kt = item_first(j); kt < nj && ok; ++kt, ++g) {
         ok = ready || mbar_wait_warp<SM_SPIN>(B_(DQ_SDP_FULL), g & 1, abort_flag, p.err, 0x5600u);
         if (!ok) break;
         tcgen05_fence_after();
@@ -1364,13 +1484,20 @@ attn_bwd_q_kernel(const __grid_constant__ CUtensorMap tm, const __grid_constant_
         if (lane == 0) mbar_arrive(B_(DQ_SDP_FREE));
         // dS as fp16 pairs, overwriting the scores they came from
         const int key0 = kt * FA_T + part * 32;
-        const bool need_mask = (kt == qt) || (p.seg != nullptr);
-        if (need_mask) bwd_ds_pack<true>(rs, rdp, key0, qi, st, p.cscale, p.scale, nlse, dsc, rs);
-        else bwd_ds_pack<false>(rs, rdp, 0, 0, 0, p.cscale, p.scale, nlse, dsc, rs);
+        const int cls = PACKED ? block_class(qi - lane, 32, key0, 32, st_min, st_max)
+                               : kt == qt ? BLOCK_SOME : BLOCK_ALL;
+        if (cls == BLOCK_SOME) bwd_ds_pack<true>(rs, rdp, key0, qi, st, p.cscale, p.scale, nlse, dsc, rs);
+        else if (!PACKED || cls == BLOCK_ALL) bwd_ds_pack<false>(rs, rdp, 0, 0, 0, p.cscale, p.scale, nlse, dsc, rs);
         const int pb = g & 1;
         ready = mbar_test_wait(B_(DQ_DS_FREE + pb), ((g >> 1) & 1) ^ 1u) != 0;
-        if (need_mask) bwd_ds_pack<true>(rs + 16, rdp + 16, key0 + 16, qi, st, p.cscale, p.scale, nlse, dsc, rs + 8);
-        else bwd_ds_pack<false>(rs + 16, rdp + 16, 0, 0, 0, p.cscale, p.scale, nlse, dsc, rs + 8);
+        if (cls == BLOCK_SOME) {
+          bwd_ds_pack<true>(rs + 16, rdp + 16, key0 + 16, qi, st, p.cscale, p.scale, nlse, dsc, rs + 8);
+        } else if (!PACKED || cls == BLOCK_ALL) {
+          bwd_ds_pack<false>(rs + 16, rdp + 16, 0, 0, 0, p.cscale, p.scale, nlse, dsc, rs + 8);
+        } else {
+#pragma unroll
+          for (int i = 0; i < 16; ++i) rs[i] = 0u;
+        }
         // dQ of step g - 2 has read this dS area
         ok = __all_sync(0xffffffffu, ready) ||
              mbar_wait_warp<SM_SPIN>(B_(DQ_DS_FREE + pb), ((g >> 1) & 1) ^ 1u, abort_flag, p.err, 0x5700u);
@@ -1460,20 +1587,21 @@ extern "C" int vkg_attn_fwd(vkg_device* dev, const void* qkv16, const uint32_t* 
   p.scale = scale;
   p.cscale = scale * LOG2E;
   p.seg = seg;
+  p.skip_tiles = skip_tiles(seg, p.nqt);
   p.out = (__half*)out16;
   p.lse2 = lse2;
   p.err = dev->err_dev;
   if (!dev->attn_fwd_attr_set) {
     VKG_CUDA(cudaFuncSetAttribute(attn_fwd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                   FW_SMEM));
-    VKG_CUDA(cudaFuncSetAttribute(attn_fwd1_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  FW_SMEM));
+    for (auto fn : {attn_fwd1_kernel<false>, attn_fwd1_kernel<true>})
+      VKG_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, FW_SMEM));
     dev->attn_fwd_attr_set = true;
   }
   const long long ctas = (long long)p.nqt * H * B;
   VKG_REQUIRE(ctas < (1ll << 31), "attn_fwd: too many tiles");
   VKG_CUDA(vkg_launch(dev, VKG_K_ATTN_FWD | vkg_short_if(ctas <= 2ll * dev->sm_count),
-                      dev->attn_one_pass ? attn_fwd1_kernel : attn_fwd_kernel,
+                      !dev->attn_one_pass ? attn_fwd_kernel : seg ? attn_fwd1_kernel<true> : attn_fwd1_kernel<false>,
                       dim3((unsigned)ctas), dim3(FA_THREADS), FW_SMEM, 1, tm, p));
   return vkg_check_launch("attn_fwd_kernel");
 }
@@ -1499,6 +1627,7 @@ extern "C" int vkg_attn_bwd(vkg_device* dev, const void* qkv16, const void* dout
   p.scale = scale;
   p.cscale = scale * LOG2E;
   p.seg = seg;
+  p.skip_tiles = skip_tiles(seg, p.nqt);
   p.lse2 = const_cast<float*>(lse2);
   p.delta = delta;
   p.delta_out = delta;
@@ -1507,10 +1636,10 @@ extern "C" int vkg_attn_bwd(vkg_device* dev, const void* qkv16, const void* dout
   VKG_REQUIRE(!dbias || dbias_scratch, "attn_bwd: dbias needs dbias_scratch");
   p.colsum = dbias ? dbias_scratch : nullptr;
   if (!dev->attn_bwd_attr_set) {
-    VKG_CUDA(cudaFuncSetAttribute(attn_bwd_kv_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  KV_SMEM));
-    VKG_CUDA(cudaFuncSetAttribute(attn_bwd_q_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  DQ_SMEM));
+    for (auto fn : {attn_bwd_kv_kernel<false>, attn_bwd_kv_kernel<true>})
+      VKG_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, KV_SMEM));
+    for (auto fn : {attn_bwd_q_kernel<false>, attn_bwd_q_kernel<true>})
+      VKG_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, DQ_SMEM));
     dev->attn_bwd_attr_set = true;
   }
   VKG_REQUIRE((((uintptr_t)dout16 | (uintptr_t)out16) & 15) == 0, "attn_bwd: dO and O must be 16-byte aligned");
@@ -1521,9 +1650,9 @@ extern "C" int vkg_attn_bwd(vkg_device* dev, const void* qkv16, const void* dout
   const int sms = vkg_persistent_ctas(dev);
   const unsigned ctas = (unsigned)(n_items < sms ? n_items : sms);
   const unsigned family = VKG_K_ATTN_BWD | vkg_short_if(n_items <= sms);
-  VKG_CUDA(vkg_launch(dev, family, attn_bwd_q_kernel, dim3(ctas), dim3(BW_THREADS), DQ_SMEM, 1, tm, tmdo, tmo, p));
+  VKG_CUDA(vkg_launch(dev, family, seg ? attn_bwd_q_kernel<true> : attn_bwd_q_kernel<false>, dim3(ctas), dim3(BW_THREADS), DQ_SMEM, 1, tm, tmdo, tmo, p));
   if (vkg_check_launch("attn_bwd_q_kernel")) return 1;
-  VKG_CUDA(vkg_launch(dev, family, attn_bwd_kv_kernel, dim3(ctas), dim3(BW_THREADS), KV_SMEM, 1, tm, tmdo, p));
+  VKG_CUDA(vkg_launch(dev, family, seg ? attn_bwd_kv_kernel<true> : attn_bwd_kv_kernel<false>, dim3(ctas), dim3(BW_THREADS), KV_SMEM, 1, tm, tmdo, p));
   if (vkg_check_launch("attn_bwd_kv_kernel")) return 1;
   if (dbias)
     return vkg_launch_col_sum_final(dev, dbias_scratch, dbias, 3 * D, B * p.nqt * 4, 0);
