@@ -702,6 +702,10 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
   if (threadIdx.x == 0) {
     prefetch_tensormap(&tmA);
     prefetch_tensormap(&tmB);
+    if ((MODE & E_NO_TMA) == 0 && p.tma_store) {
+      prefetch_tensormap(&tmC);
+      if (MODE & E_PRE) prefetch_tensormap(&tmP);
+    }
   }
   CtaCtx cx;
   cta_setup(cx, smem_raw, p.bn, p.stages);
@@ -999,6 +1003,10 @@ gemm_cta_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
   if (threadIdx.x == 0) {
     prefetch_tensormap(&tmA);
     prefetch_tensormap(&tmB);
+    if ((MODE & E_NO_TMA) == 0 && p.tma_store) {
+      prefetch_tensormap(&tmC);
+      if (MODE & E_PRE) prefetch_tensormap(&tmP);
+    }
   }
   CtaCtx cx;
   pair_setup(cx, smem_raw, p.bn, p.b_mn);
