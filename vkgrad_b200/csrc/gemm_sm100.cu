@@ -36,7 +36,7 @@ namespace {
 using namespace tc05;
 
 constexpr int BM = 128;            // rows of C per tile = UMMA M
-constexpr int BK = 64;             // K elements per stage = 128 bytes of f16 = one swizzle row
+constexpr int BK = 64;             // K elements per k-block = 128 bytes of f16 = one swizzle row
 constexpr int UMMA_K = 16;         // K per tcgen05.mma.kind::f16
 constexpr int A_STAGE_BYTES = BM * BK * 2;
 constexpr int MAX_STAGES = 8;
@@ -54,7 +54,10 @@ struct GemmParams {
   int M, N, K;
   int nb0, nb1;
   int tiles_m, tiles_n;
-  int bn, stages, num_kb;
+  int bn, num_kb;
+  int stages, stage_kb, stage_bytes;   // the ring of one CTA: stages, k-blocks and bytes of each
+  int rows_a, rows_b;                  // of the operands' tiles in one CTA
+  int a_wide, b_wide, a_loads, b_loads;   // Feed
   int split_k, kb_per_split;   // split_k > 1: z1 is the K slice, not a batch index
   int causal;                  // 0 none, 1 skip tiles above the diagonal, 2/3 clip the K range
   int a_mn, b_mn;
@@ -432,75 +435,143 @@ struct CtaCtx {
   uint8_t* epi_stage;
 };
 
-// TMA producer (one lane): stream the k-blocks of work unit t's operands into the ring.
-__device__ __forceinline__ bool produce_unit(const CtaCtx& cx, const GemmParams& p,
-                                             const CUtensorMap* tmA, const CUtensorMap* tmB, int t,
-                                             int& stage, uint32_t& phase) {
-  TileCoord tc = tile_coord(p, t);
+// Position in the ring.  A stage's first fill waits for nobody.
+struct Ring {
+  int stage = 0;
+  uint32_t phase = 0;
+  bool wrapped = false;
+  __device__ __forceinline__ void step(int n_stages) {
+    if (++stage == n_stages) {
+      stage = 0;
+      phase ^= 1u;
+      wrapped = true;
+    }
+  }
+};
+
+// How an operand comes into the ring.  What a k-block of a narrow tile costs is neither bytes nor tensor
+// time but the instructions around them: 115 cycles for a wait, 50 to 100 for each load, in the loop of
+// the warp that loads and again in the loop of the warp that multiplies.  With one k-block to a stage
+// and a load for every 64 columns both loops took 383 (NT) to 490 (TN) cycles where the tensor core needs
+// 192.  So a stage holds two k-blocks wherever that leaves three stages, and an operand whose
+// contiguous dimension is whole 64-element pieces is wide: its map splits that dimension in two, and one
+// load brings the stage's pieces, each a tile of its own ([k-block][row][64] of a K-major operand,
+// [64 columns][k][64] of an MN-major one).  Others take a load per piece, into the same places.
+// 1024 x 768 x 3072 (NN, residual): 15.4 -> 11.9 us, 768 x 2304 x 1024 (TN) 9.1 -> 7.6.
+struct Feed {
+  int c0, c1, c2;        // map coordinates; a load per piece moves c0 on by 64
+  int s0, s1, s2;        // their step per stage
+  int loads;
+  uint32_t step;         // shared-memory bytes from one load to the next
+  __device__ __forceinline__ Feed(bool mn, bool wide, int n, int kb0, int at, int rows, int stage_kb) {
+    c0 = wide ? 0 : mn ? at : kb0 * BK;
+    c1 = mn ? kb0 * BK : at;
+    c2 = !wide ? 0 : mn ? at / 64 : kb0;
+    s0 = wide || mn ? 0 : stage_kb * BK;
+    s1 = mn ? stage_kb * BK : 0;
+    s2 = wide && !mn ? stage_kb : 0;
+    loads = n;
+    step = mn ? (uint32_t)stage_kb * 8192u : (uint32_t)rows * 128u;
+  }
+  template <bool PAIR>
+  __device__ __forceinline__ void load(uint32_t dst, const CUtensorMap* map, uint32_t bar, const TileCoord& tc) {
+    int x = c0;
+    for (int i = loads;;) {
+      if (PAIR) tma_load_5d_pair(dst, map, bar, x, c1, c2, tc.z0, tc.z1);
+      else tma_load_5d(dst, map, bar, x, c1, c2, tc.z0, tc.z1);
+      if (--i == 0) break;
+      x += 64;
+      dst += step;
+    }
+    c0 += s0;
+    c1 += s1;
+    c2 += s2;
+  }
+};
+
+// TMA producer (one lane) of a single CTA or of one CTA of a pair: stream the k-blocks of a work unit's
+// operands into the ring.  b_at: the CTA's first column of B.
+template <bool PAIR>
+__device__ __forceinline__ bool produce(const CtaCtx& cx, const GemmParams& p, const CUtensorMap* tmA,
+                                        const CUtensorMap* tmB, TileCoord tc, int b_at, uint32_t rank, Ring& at) {
   int kb0, nkb;
   kb_range(p, tc, kb0, nkb);
   if (p.split_k > 1) tc.z1 = 0;   // operands are not batched along the slice index
-  for (int kb = 0; kb < nkb; ++kb) {
-    if (!mbar_wait(cx.empty0 + 8 * stage, phase ^ 1u, cx.abort_flag, p.err, 0x100u + stage)) return false;
-    const uint32_t fb = cx.full0 + 8 * stage;
-    mbar_expect_tx(fb, cx.stage_bytes);
-    const uint32_t sa = cx.base + stage * cx.stage_bytes;
-    const uint32_t sb = sa + A_STAGE_BYTES;
-    const int k0 = (kb0 + kb) * BK;
-    if (!p.a_mn) {
-      tma_load_4d(sa, tmA, fb, k0, tc.m0, tc.z0, tc.z1);
+  Feed a(p.a_mn != 0, p.a_wide != 0, p.a_loads, kb0, tc.m0, p.rows_a, p.stage_kb);
+  Feed b(p.b_mn != 0, p.b_wide != 0, p.b_loads, kb0, b_at, p.rows_b, p.stage_kb);
+  const uint32_t a_bytes = (uint32_t)(p.stage_kb * p.rows_a) * 128u;
+  for (int kb = 0; kb < nkb; kb += p.stage_kb) {
+    if (at.wrapped && !mbar_wait(cx.empty0 + 8 * at.stage, at.phase ^ 1u, cx.abort_flag, p.err, 0x100u + at.stage))
+      return false;
+    uint32_t fb = cx.full0 + 8 * at.stage;
+    const uint32_t sa = cx.base + at.stage * cx.stage_bytes;
+    if (PAIR) {
+      if (rank == 0) mbar_expect_tx(fb, 2 * cx.stage_bytes);
+      fb = mapa_shared(fb, 0);
     } else {
-      tma_load_4d(sa, tmA, fb, tc.m0, k0, tc.z0, tc.z1);
-      tma_load_4d(sa + 8192, tmA, fb, tc.m0 + 64, k0, tc.z0, tc.z1);
+      mbar_expect_tx(fb, cx.stage_bytes);
     }
-    if (!p.b_mn) {
-      tma_load_4d(sb, tmB, fb, k0, tc.n0, tc.z0, tc.z1);
-    } else {
-      for (int g = 0; g < p.bn / 64; ++g)
-        tma_load_4d(sb + g * 8192, tmB, fb, tc.n0 + 64 * g, k0, tc.z0, tc.z1);
-    }
-    if (++stage == cx.n_stages) {
-      stage = 0;
-      phase ^= 1u;
-    }
+    a.load<PAIR>(sa, tmA, fb, tc);
+    b.load<PAIR>(sa + a_bytes, tmB, fb, tc);
+    at.step(cx.n_stages);
   }
   return true;
 }
 
-// MMA issue (the whole warp, converged; one elected lane issues each instruction): accumulate the
-// k-blocks of work unit t into one of the two TMEM accumulators.
-__device__ __forceinline__ bool mma_unit(const CtaCtx& cx, const GemmParams& p, int t, int& stage,
-                                         uint32_t& phase, int& acc, uint32_t& acc_phase) {
+// MMA issue (the whole warp, converged; one elected lane issues each instruction) of a single CTA, or of
+// the even-ranked CTA for a pair: accumulate a work unit's k-blocks into one of the two TMEM
+// accumulators.  Descriptor halves step along K by 16 elements: 32 bytes further along the 128-byte row
+// for a K-major operand, two 8-row groups (2 x 1024 bytes) further down for an MN-major one, whose 64-column
+// groups lie a stage's k apart.  All in units of 16 bytes.
+template <bool PAIR, int STAGE_KB>
+__device__ __forceinline__ bool multiply(const CtaCtx& cx, const GemmParams& p, uint32_t d_tmem, int nkb, Ring& at) {
+  const uint32_t d_hi = smem_desc_hi(1024);
+  const uint32_t a_lo0 = smem_desc_lo(cx.base, p.a_mn ? STAGE_KB * 8192 : 16);
+  const uint32_t b_lo0 = smem_desc_lo(cx.base + STAGE_KB * p.rows_a * 128, p.b_mn ? STAGE_KB * 8192 : 16);
+  const uint32_t a_step = p.a_mn ? 128u : 2u, b_step = p.b_mn ? 128u : 2u;
+  const uint32_t a_kb = p.a_mn ? 512u : (uint32_t)p.rows_a * 8u, b_kb = p.b_mn ? 512u : (uint32_t)p.rows_b * 8u;
+  const uint32_t stage16 = cx.stage_bytes >> 4;
+  for (int kb = 0; kb < nkb; kb += STAGE_KB) {
+    if (!mbar_wait_warp(cx.full0 + 8 * at.stage, at.phase, cx.abort_flag, p.err, 0x300u + at.stage)) return false;
+    tcgen05_fence_after();
+    const uint32_t a_lo = a_lo0 + (uint32_t)at.stage * stage16, b_lo = b_lo0 + (uint32_t)at.stage * stage16;
+#pragma unroll
+    for (int i = 0; i < STAGE_KB; ++i) {
+      if (i > 0 && kb + i >= nkb) break;       // the last stage may hold one k-block that does not count
+#pragma unroll
+      for (int k = 0; k < BK / UMMA_K; ++k) {
+        const uint64_t ad = smem_desc_pack(a_lo + i * a_kb + k * a_step, d_hi);
+        const uint64_t bd = smem_desc_pack(b_lo + i * b_kb + k * b_step, d_hi);
+        if (elect_one()) {
+          if (PAIR) umma2_f16(d_tmem, ad, bd, p.idesc, (kb | i | k) != 0 ? 1u : 0u);
+          else umma_f16(d_tmem, ad, bd, p.idesc, (kb | i | k) != 0 ? 1u : 0u);
+        }
+      }
+    }
+    if (elect_one()) {                         // frees the stage when these MMAs retire
+      if (PAIR) umma2_commit(cx.empty0 + 8 * at.stage);
+      else umma_commit(cx.empty0 + 8 * at.stage);
+    }
+    at.step(cx.n_stages);
+  }
+  return true;
+}
+
+template <bool PAIR>
+__device__ __forceinline__ bool mma_unit(const CtaCtx& cx, const GemmParams& p, int t, Ring& at, int& acc,
+                                         uint32_t& acc_phase) {
   int kb0, nkb;
-  kb_range(p, tile_coord(p, t), kb0, nkb);
+  kb_range(p, tile_coord(p, t, PAIR ? 2 * BM : BM), kb0, nkb);
   if (nkb <= 0) return true;   // skipped tile: no accumulator, no epilogue
   if (!mbar_wait_warp(cx.tempty0 + 8 * acc, acc_phase ^ 1u, cx.abort_flag, p.err, 0x200u + acc)) return false;
   tcgen05_fence_after();
   const uint32_t d_tmem = cx.tmem_base + (uint32_t)(acc * ACC_COLS);
-  // Descriptor halves of ring stage 0; a K step of 16 elements is 32 bytes further along the
-  // 128-byte row for a K-major operand and two 8-row groups (2 x 1024 bytes) further down for
-  // an MN-major one; a stage is stage_bytes further on.  All in units of 16 bytes.
-  const uint32_t d_hi = smem_desc_hi(1024);
-  const uint32_t a_lo0 = smem_desc_lo(cx.base, p.a_mn ? 8192 : 16);
-  const uint32_t b_lo0 = smem_desc_lo(cx.base + A_STAGE_BYTES, p.b_mn ? 8192 : 16);
-  const uint32_t a_step = p.a_mn ? 128u : 2u, b_step = p.b_mn ? 128u : 2u;
-  const uint32_t stage16 = cx.stage_bytes >> 4;
-  for (int kb = 0; kb < nkb; ++kb) {
-    if (!mbar_wait_warp(cx.full0 + 8 * stage, phase, cx.abort_flag, p.err, 0x300u + stage)) return false;
-    tcgen05_fence_after();
-    const uint32_t a_lo = a_lo0 + (uint32_t)stage * stage16, b_lo = b_lo0 + (uint32_t)stage * stage16;
-#pragma unroll
-    for (int k = 0; k < BK / UMMA_K; ++k)
-      if (elect_one())
-        umma_f16(d_tmem, smem_desc_pack(a_lo + k * a_step, d_hi), smem_desc_pack(b_lo + k * b_step, d_hi),
-                 p.idesc, (kb | k) != 0 ? 1u : 0u);
-    umma_commit_one(cx.empty0 + 8 * stage);  // frees the stage when these MMAs retire
-    if (++stage == cx.n_stages) {
-      stage = 0;
-      phase ^= 1u;
-    }
+  if (!(p.stage_kb == 2 ? multiply<PAIR, 2>(cx, p, d_tmem, nkb, at) : multiply<PAIR, 1>(cx, p, d_tmem, nkb, at)))
+    return false;
+  if (elect_one()) {           // accumulator complete -> epilogue
+    if (PAIR) umma2_commit(cx.tfull0 + 8 * acc);
+    else umma_commit(cx.tfull0 + 8 * acc);
   }
-  umma_commit_one(cx.tfull0 + 8 * acc);  // accumulator complete -> epilogue
   acc ^= 1;
   if (acc == 0) acc_phase ^= 1u;
   return true;
@@ -627,11 +698,11 @@ __device__ __forceinline__ bool epilogue_unit(const CtaCtx& cx, const GemmParams
 // Barriers, TMEM and the role-independent constants of a CTA.
 // (Issuing the first loads here, before tensor memory is allocated, measured 1 us SLOWER per launch:
 // the tensor maps prefetched at the top of the kernel are not there yet.)
-__device__ __forceinline__ void cta_setup(CtaCtx& cx, uint8_t* smem_raw, int bn, int stages) {
+__device__ __forceinline__ void cta_setup(CtaCtx& cx, uint8_t* smem_raw, int stage_bytes, int stages) {
   // 128B-swizzled tiles want 1024-byte alignment.
   cx.base = (smem_u32(smem_raw) + 1023u) & ~1023u;
   uint8_t* gen_base = smem_raw + (cx.base - smem_u32(smem_raw));
-  cx.stage_bytes = A_STAGE_BYTES + (uint32_t)bn * 128u;
+  cx.stage_bytes = (uint32_t)stage_bytes;
   cx.n_stages = stages;
   // Epilogue staging (one swizzled 32x16 fp32 chunk per epilogue warp), then the barrier block.
   cx.epi_stage = gen_base + RING_BYTES;
@@ -708,23 +779,25 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
     }
   }
   CtaCtx cx;
-  cta_setup(cx, smem_raw, p.bn, p.stages);
+  cta_setup(cx, smem_raw, p.stage_bytes, p.stages);
   pdl_wait();      // barriers, TMEM and tensor maps are ready; operands may still be in flight
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
   const int total_tiles = p.tiles_m * p.tiles_n * p.nb0 * (p.split_k > 1 ? p.split_k : p.nb1);
   if (warp == 0) {
     if (lane == 0) {
-      int stage = 0;
-      uint32_t phase = 0;
-      for (int t = blockIdx.x; t < total_tiles; t += gridDim.x)
-        if (!produce_unit(cx, p, &tmA, &tmB, t, stage, phase)) break;
+      Ring at;
+      for (int t = blockIdx.x; t < total_tiles; t += gridDim.x) {
+        const TileCoord tc = tile_coord(p, t);
+        if (!produce<false>(cx, p, &tmA, &tmB, tc, tc.n0, 0, at)) break;
+      }
     }
   } else if (warp == 1) {
-    int stage = 0, acc = 0;
-    uint32_t phase = 0, acc_phase = 0;
+    Ring at;
+    int acc = 0;
+    uint32_t acc_phase = 0;
     for (int t = blockIdx.x; t < total_tiles; t += gridDim.x)
-      if (!mma_unit(cx, p, t, stage, phase, acc, acc_phase)) break;
+      if (!mma_unit<false>(cx, p, t, at, acc, acc_phase)) break;
   } else {
     int acc = 0;
     uint32_t acc_phase = 0;
@@ -763,35 +836,35 @@ __device__ __forceinline__ int group_find(const int* first, int n, int u) {
 }
 
 __global__ void __launch_bounds__(NUM_THREADS, 1)
-gemm_group_kernel(const GroupEntry* __restrict__ table, int n_problems, int total_units, int bn,
-                  int stages) {
+gemm_group_kernel(const GroupEntry* __restrict__ table, int n_problems, int total_units) {
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   __shared__ int first[GROUP_MAX];
   pdl_trigger();
   // the table was written by the host long before this launch, not by the kernel before it
   for (int i = threadIdx.x; i < n_problems; i += blockDim.x) first[i] = table[i].first_unit;
   CtaCtx cx;
-  cta_setup(cx, smem_raw, bn, stages);     // its __syncthreads also publishes first[]
+  cta_setup(cx, smem_raw, table->p.stage_bytes, table->p.stages);   // the same for all; its __syncthreads also publishes first[]
   pdl_wait();
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
   if (warp == 0) {
     if (lane == 0) {
-      int stage = 0;
-      uint32_t phase = 0;
+      Ring at;
       for (int u = blockIdx.x; u < total_units; u += gridDim.x) {
         const int pi = group_find(first, n_problems, u);
         const GemmParams p = table[pi].p;
-        if (!produce_unit(cx, p, &table[pi].tmA, &table[pi].tmB, u - first[pi], stage, phase)) break;
+        const TileCoord tc = tile_coord(p, u - first[pi]);
+        if (!produce<false>(cx, p, &table[pi].tmA, &table[pi].tmB, tc, tc.n0, 0, at)) break;
       }
     }
   } else if (warp == 1) {
-    int stage = 0, acc = 0;
-    uint32_t phase = 0, acc_phase = 0;
+    Ring at;
+    int acc = 0;
+    uint32_t acc_phase = 0;
     for (int u = blockIdx.x; u < total_units; u += gridDim.x) {
       const int pi = group_find(first, n_problems, u);
       const GemmParams p = table[pi].p;
-      if (!mma_unit(cx, p, u - first[pi], stage, phase, acc, acc_phase)) break;
+      if (!mma_unit<false>(cx, p, u - first[pi], at, acc, acc_phase)) break;
     }
   } else {
     int acc = 0;
@@ -817,24 +890,14 @@ gemm_group_kernel(const GroupEntry* __restrict__ table, int n_problems, int tota
 // leader's full[s]; the leader's commits arrive on empty[s] / tmem_full[a] of both CTAs;
 // the epilogue warps of both CTAs arrive on the leader's tmem_empty[a].
 constexpr int PAIR_BN = 256;        // widest pair tile; 192 is the other width (N = 768 shapes)
-// Bytes of one CTA's half of the B tile per k-block: bn / 2 rows of 128 bytes when B is K-major,
-// whole 64-column groups of 64 k-rows when it is MN-major (96 columns load two groups).
-__host__ __device__ inline int pair_b_stage_bytes(int bn, int b_mn) {
-  return b_mn ? ((bn / 2 + 63) / 64) * 8192 : (bn / 2) * 128;
-}
-__host__ __device__ inline int pair_stages(int bn, int b_mn) {
-  const int n = RING_BYTES / (A_STAGE_BYTES + pair_b_stage_bytes(bn, b_mn));
-  return n > MAX_STAGES ? MAX_STAGES : n;
-}
-
 // Barriers, TMEM and constants of one CTA of a pair; ends with a cluster-wide barrier so the
 // peer's mbarriers exist before anything is signalled on them.
-__device__ __forceinline__ void pair_setup(CtaCtx& cx, uint8_t* smem_raw, int bn, int b_mn) {
+__device__ __forceinline__ void pair_setup(CtaCtx& cx, uint8_t* smem_raw, int stage_bytes, int stages) {
   const int warp = threadIdx.x >> 5;
   cx.base = (smem_u32(smem_raw) + 1023u) & ~1023u;
   uint8_t* gen_base = smem_raw + (cx.base - smem_u32(smem_raw));
-  cx.stage_bytes = (uint32_t)(A_STAGE_BYTES + pair_b_stage_bytes(bn, b_mn));
-  cx.n_stages = pair_stages(bn, b_mn);
+  cx.stage_bytes = (uint32_t)stage_bytes;
+  cx.n_stages = stages;
   cx.epi_stage = gen_base + RING_BYTES;
   uint64_t* bars = reinterpret_cast<uint64_t*>(gen_base + RING_BYTES + EPI_WARPS * EPI_STAGE_BYTES);
   const uint32_t bar_base = cx.base + RING_BYTES + EPI_WARPS * EPI_STAGE_BYTES;
@@ -894,76 +957,9 @@ __device__ __forceinline__ void pair_teardown(const CtaCtx& cx) {
   }
 }
 
-// TMA producer of one CTA of the pair: its 128 rows of A and its half of the B tile.
-__device__ __forceinline__ bool pair_produce_unit(const CtaCtx& cx, const GemmParams& p,
-                                                  const CUtensorMap* tmA, const CUtensorMap* tmB,
-                                                  int t, uint32_t rank, int& stage, uint32_t& phase) {
-  TileCoord tc = tile_coord(p, t, 2 * BM, (int)rank * BM);
-  int kb0, nkb;
-  kb_range(p, tc, kb0, nkb);
-  if (p.split_k > 1) tc.z1 = 0;
-  const int nb = tc.n0 + (int)rank * (p.bn / 2);       // this CTA's columns of B
-  for (int kb = 0; kb < nkb; ++kb) {
-    if (!mbar_wait(cx.empty0 + 8 * stage, phase ^ 1u, cx.abort_flag, p.err, 0x500u + stage)) return false;
-    if (rank == 0) mbar_expect_tx(cx.full0 + 8 * stage, 2 * cx.stage_bytes);
-    const uint32_t fb = mapa_shared(cx.full0 + 8 * stage, 0);
-    const uint32_t sa = cx.base + stage * cx.stage_bytes;
-    const uint32_t sb = sa + A_STAGE_BYTES;
-    const int k0 = (kb0 + kb) * BK;
-    if (!p.a_mn) {
-      tma_load_4d_pair(sa, tmA, fb, k0, tc.m0, tc.z0, tc.z1);
-    } else {
-      tma_load_4d_pair(sa, tmA, fb, tc.m0, k0, tc.z0, tc.z1);
-      tma_load_4d_pair(sa + 8192, tmA, fb, tc.m0 + 64, k0, tc.z0, tc.z1);
-    }
-    if (!p.b_mn) {
-      tma_load_4d_pair(sb, tmB, fb, k0, nb, tc.z0, tc.z1);
-    } else {
-      // whole 64-column groups: a 96-column half loads two and uses one and a half
-      tma_load_4d_pair(sb, tmB, fb, nb, k0, tc.z0, tc.z1);
-      if (p.bn > 128) tma_load_4d_pair(sb + 8192, tmB, fb, nb + 64, k0, tc.z0, tc.z1);
-    }
-    if (++stage == cx.n_stages) {
-      stage = 0;
-      phase ^= 1u;
-    }
-  }
-  return true;
-}
-
-// MMA issue for the pair (a converged warp of the even-ranked CTA).
-__device__ __forceinline__ bool pair_mma_unit(const CtaCtx& cx, const GemmParams& p, int t, int& stage,
-                                              uint32_t& phase, int& acc, uint32_t& acc_phase) {
-  int kb0, nkb;
-  kb_range(p, tile_coord(p, t, 2 * BM, 0), kb0, nkb);
-  if (nkb <= 0) return true;
-  if (!mbar_wait_warp(cx.tempty0 + 8 * acc, acc_phase ^ 1u, cx.abort_flag, p.err, 0x600u + acc)) return false;
-  tcgen05_fence_after();
-  const uint32_t d_tmem = cx.tmem_base + (uint32_t)(acc * ACC_COLS);
-  const uint32_t d_hi = smem_desc_hi(1024);       // descriptor halves as in mma_unit
-  const uint32_t a_lo0 = smem_desc_lo(cx.base, p.a_mn ? 8192 : 16);
-  const uint32_t b_lo0 = smem_desc_lo(cx.base + A_STAGE_BYTES, p.b_mn ? 8192 : 16);
-  const uint32_t a_step = p.a_mn ? 128u : 2u, b_step = p.b_mn ? 128u : 2u;
-  for (int kb = 0; kb < nkb; ++kb) {
-    if (!mbar_wait_warp(cx.full0 + 8 * stage, phase, cx.abort_flag, p.err, 0x700u + stage)) return false;
-    tcgen05_fence_after();
-    const uint32_t a_lo = a_lo0 + (uint32_t)stage * (cx.stage_bytes >> 4);
-    const uint32_t b_lo = b_lo0 + (uint32_t)stage * (cx.stage_bytes >> 4);
-#pragma unroll
-    for (int k = 0; k < BK / UMMA_K; ++k)
-      if (elect_one())
-        umma2_f16(d_tmem, smem_desc_pack(a_lo + k * a_step, d_hi), smem_desc_pack(b_lo + k * b_step, d_hi),
-                  p.idesc, (kb | k) != 0 ? 1u : 0u);
-    if (elect_one()) umma2_commit(cx.empty0 + 8 * stage);
-    if (++stage == cx.n_stages) {
-      stage = 0;
-      phase ^= 1u;
-    }
-  }
-  if (elect_one()) umma2_commit(cx.tfull0 + 8 * acc);
-  acc ^= 1;
-  if (acc == 0) acc_phase ^= 1u;
-  return true;
+// Tile t as CTA `rank` of the pair sees it: its 128 rows of A, and its half of the columns of B.
+__device__ __forceinline__ TileCoord pair_coord(const GemmParams& p, int t, uint32_t rank) {
+  return tile_coord(p, t, 2 * BM, (int)rank * BM);
 }
 
 // Epilogue warp of one CTA of the pair: its 128 rows of the 256 x 256 tile.
@@ -972,7 +968,7 @@ __device__ __forceinline__ bool pair_epilogue_unit(const CtaCtx& cx, const GemmP
                                                    const CUtensorMap* tmC, const CUtensorMap* tmP, int t,
                                                    uint32_t rank, int warp, int lane, int& acc,
                                                    uint32_t& acc_phase) {
-  const TileCoord tc = tile_coord(p, t, 2 * BM, (int)rank * BM);
+  const TileCoord tc = pair_coord(p, t, rank);
   {
     int kb0, nkb;
     kb_range(p, tc, kb0, nkb);
@@ -1009,23 +1005,25 @@ gemm_cta_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
     }
   }
   CtaCtx cx;
-  pair_setup(cx, smem_raw, p.bn, p.b_mn);
+  pair_setup(cx, smem_raw, p.stage_bytes, p.stages);
   pdl_wait();
   const int n_pairs = (int)gridDim.x >> 1, pair = (int)blockIdx.x >> 1;
   const int total_tiles = p.tiles_m * p.tiles_n * p.nb0 * (p.split_k > 1 ? p.split_k : p.nb1);
   if (warp == 0) {
     if (lane == 0) {
-      int stage = 0;
-      uint32_t phase = 0;
-      for (int t = pair; t < total_tiles; t += n_pairs)
-        if (!pair_produce_unit(cx, p, &tmA, &tmB, t, rank, stage, phase)) break;
+      Ring at;
+      for (int t = pair; t < total_tiles; t += n_pairs) {
+        const TileCoord tc = pair_coord(p, t, rank);
+        if (!produce<true>(cx, p, &tmA, &tmB, tc, tc.n0 + (int)rank * p.rows_b, rank, at)) break;
+      }
     }
   } else if (warp == 1) {
     if (rank == 0) {
-      int stage = 0, acc = 0;
-      uint32_t phase = 0, acc_phase = 0;
+      Ring at;
+      int acc = 0;
+      uint32_t acc_phase = 0;
       for (int t = pair; t < total_tiles; t += n_pairs)
-        if (!pair_mma_unit(cx, p, t, stage, phase, acc, acc_phase)) break;
+        if (!mma_unit<true>(cx, p, t, at, acc, acc_phase)) break;
     }
   } else {
     int acc = 0;
@@ -1048,28 +1046,28 @@ gemm_group_pair_kernel(const GroupEntry* __restrict__ table, int n_problems, int
   const int lane = threadIdx.x & 31;
   const uint32_t rank = cluster_ctarank();
   CtaCtx cx;
-  pair_setup(cx, smem_raw, PAIR_BN, 1);   // dW problems: both operands MN-major; publishes first[]
+  pair_setup(cx, smem_raw, table->p.stage_bytes, table->p.stages);   // the same for all; publishes first[]
   pdl_wait();
   const int n_pairs = (int)gridDim.x >> 1, pair = (int)blockIdx.x >> 1;
   if (warp == 0) {
     if (lane == 0) {
-      int stage = 0;
-      uint32_t phase = 0;
+      Ring at;
       for (int u = pair; u < total_units; u += n_pairs) {
         const int pi = group_find(first, n_problems, u);
         const GemmParams p = table[pi].p;
-        if (!pair_produce_unit(cx, p, &table[pi].tmA, &table[pi].tmB, u - first[pi], rank, stage, phase))
-          break;
+        const TileCoord tc = pair_coord(p, u - first[pi], rank);
+        if (!produce<true>(cx, p, &table[pi].tmA, &table[pi].tmB, tc, tc.n0 + (int)rank * p.rows_b, rank, at)) break;
       }
     }
   } else if (warp == 1) {
     if (rank == 0) {
-      int stage = 0, acc = 0;
-      uint32_t phase = 0, acc_phase = 0;
+      Ring at;
+      int acc = 0;
+      uint32_t acc_phase = 0;
       for (int u = pair; u < total_units; u += n_pairs) {
         const int pi = group_find(first, n_problems, u);
         const GemmParams p = table[pi].p;
-        if (!pair_mma_unit(cx, p, u - first[pi], stage, phase, acc, acc_phase)) break;
+        if (!mma_unit<true>(cx, p, u - first[pi], at, acc, acc_phase)) break;
       }
     }
   } else {
@@ -1149,17 +1147,19 @@ typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t,
                                   const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle,
                                   CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
 
-// 4-D map {inner, rows, nb0, nb1} over a 16-bit matrix with two batch strides.
+// 5-D map over a 16-bit matrix with two batch strides: {inner, rows, 1, nb0, nb1}, or wide (Feed)
+// {64, rows, inner / 64, nb0, nb1}, with boxes of 64 x box_rows x pieces.
 int make_map(vkg_device* dev, CUtensorMap* map, const void* ptr, int dtype, int64_t inner,
-             int64_t rows, int64_t ld, int nb0, int64_t s0, int nb1, int64_t s1, int box_inner,
-             int box_rows, const char* what) {
-  cuuint64_t dims[4] = {(cuuint64_t)inner, (cuuint64_t)rows, (cuuint64_t)nb0, (cuuint64_t)nb1};
+             int64_t rows, int64_t ld, int nb0, int64_t s0, int nb1, int64_t s1, bool wide, int box_rows,
+             int pieces, const char* what) {
+  cuuint64_t dims[5] = {(cuuint64_t)(wide ? 64 : inner), (cuuint64_t)rows, (cuuint64_t)(wide ? inner / 64 : 1),
+                        (cuuint64_t)nb0, (cuuint64_t)nb1};
   int64_t pitch = ld * 2;
   int64_t st0 = nb0 > 1 ? s0 * 2 : pitch * rows;
   int64_t st1 = nb1 > 1 ? s1 * 2 : (nb0 > 1 ? st0 * nb0 : pitch * rows);
-  cuuint64_t strides[3] = {(cuuint64_t)pitch, (cuuint64_t)st0, (cuuint64_t)st1};
-  cuuint32_t box[4] = {(cuuint32_t)box_inner, (cuuint32_t)box_rows, 1, 1};
-  cuuint32_t estr[4] = {1, 1, 1, 1};
+  cuuint64_t strides[4] = {(cuuint64_t)pitch, (cuuint64_t)(wide ? 128 : pitch * rows), (cuuint64_t)st0, (cuuint64_t)st1};
+  cuuint32_t box[5] = {64, (cuuint32_t)box_rows, (cuuint32_t)pieces, 1, 1};
+  cuuint32_t estr[5] = {1, 1, 1, 1, 1};
   if (((uintptr_t)ptr & 15) || (pitch & 15) || (st0 & 15) || (st1 & 15)) {
     vkg_set_error("gemm operand %s: base address and strides must be multiples of 16 bytes "
                   "(ptr %p, ld %lld, batch strides %lld/%lld elements)",
@@ -1167,7 +1167,7 @@ int make_map(vkg_device* dev, CUtensorMap* map, const void* ptr, int dtype, int6
     return 1;
   }
   CUresult r = ((EncodeTiledFn)dev->encode_tiled)(
-      map, dtype == VKG_BF16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 4,
+      map, dtype == VKG_BF16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 5,
       const_cast<void*>(ptr), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
       CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
       CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
@@ -1432,11 +1432,20 @@ int build_problem(vkg_device* dev, const vkg_gemm_args* a, Problem* out, bool us
   p.tiles_n = (a->N + bn - 1) / bn;
   p.bn = bn;
   p.num_kb = (a->K + BK - 1) / BK;
-  int stage_bytes = A_STAGE_BYTES + bn * 128;
-  p.stages = RING_BYTES / stage_bytes;
-  if (p.stages > MAX_STAGES) p.stages = MAX_STAGES;
   p.a_mn = a->trans_a ? 1 : 0;
   p.b_mn = a->trans_b ? 0 : 1;
+  p.rows_a = BM;
+  p.rows_b = use_pair ? bn / 2 : bn;
+  // the CTA's columns of an MN-major B in whole groups: a 96-column half loads two and uses one and a half
+  const int b_cols = (p.rows_b + 63) / 64 * 64;
+  const int kb_bytes = A_STAGE_BYTES + (p.b_mn ? b_cols : p.rows_b) * 128;
+  p.stage_kb = !(use_pair && bn == PAIR_BN) && RING_BYTES / (2 * kb_bytes) >= 3 ? 2 : 1;
+  p.stage_bytes = p.stage_kb * kb_bytes;
+  p.stages = std::min(RING_BYTES / p.stage_bytes, MAX_STAGES);
+  p.a_wide = (p.a_mn ? a->M : a->K) % 64 == 0;
+  p.b_wide = (p.b_mn ? a->N : a->K) % 64 == 0 && (!p.b_mn || p.rows_b == b_cols);
+  p.a_loads = p.a_wide ? 1 : p.a_mn ? BM / 64 : p.stage_kb;
+  p.b_loads = p.b_wide ? 1 : p.b_mn ? b_cols / 64 : p.stage_kb;
   const uint32_t fmt = a->in_dtype == VKG_BF16 ? 1u : 0u;
   p.idesc = (1u << 4) | (fmt << 7) | (fmt << 10) | ((uint32_t)p.a_mn << 15) |
             ((uint32_t)p.b_mn << 16) | ((uint32_t)(bn >> 3) << 17) | ((uint32_t)(bm >> 4) << 24);
@@ -1481,21 +1490,24 @@ int build_problem(vkg_device* dev, const vkg_gemm_args* a, Problem* out, bool us
   CUtensorMap& tmB = out->tmB;
   if (!a->trans_a) {
     VKG_REQUIRE(a->lda >= a->K, "gemm: lda %lld < K %d", (long long)a->lda, a->K);
-    if (make_map(dev, &tmA, a->A, a->in_dtype, a->K, a->M, a->lda, nb0, a->sA0, nb1, a->sA1, BK, BM, "A"))
+    if (make_map(dev, &tmA, a->A, a->in_dtype, a->K, a->M, a->lda, nb0, a->sA0, nb1, a->sA1, p.a_wide, BM,
+                 p.a_wide ? p.stage_kb : 1, "A"))
       return 1;
   } else {
     VKG_REQUIRE(a->lda >= a->M, "gemm: lda %lld < M %d (A stored K x M)", (long long)a->lda, a->M);
-    if (make_map(dev, &tmA, a->A, a->in_dtype, a->M, a->K, a->lda, nb0, a->sA0, nb1, a->sA1, 64, BK, "A^T"))
+    if (make_map(dev, &tmA, a->A, a->in_dtype, a->M, a->K, a->lda, nb0, a->sA0, nb1, a->sA1, p.a_wide,
+                 p.stage_kb * BK, p.a_wide ? BM / 64 : 1, "A^T"))
       return 1;
   }
   if (a->trans_b) {
     VKG_REQUIRE(a->ldb >= a->K, "gemm: ldb %lld < K %d (B stored N x K)", (long long)a->ldb, a->K);
-    if (make_map(dev, &tmB, a->B, a->in_dtype, a->K, a->N, a->ldb, nb0, a->sB0, nb1, a->sB1, BK,
-                 use_pair ? bn / 2 : bn, "B^T"))
+    if (make_map(dev, &tmB, a->B, a->in_dtype, a->K, a->N, a->ldb, nb0, a->sB0, nb1, a->sB1, p.b_wide,
+                 p.rows_b, p.b_wide ? p.stage_kb : 1, "B^T"))
       return 1;
   } else {
     VKG_REQUIRE(a->ldb >= a->N, "gemm: ldb %lld < N %d", (long long)a->ldb, a->N);
-    if (make_map(dev, &tmB, a->B, a->in_dtype, a->N, a->K, a->ldb, nb0, a->sB0, nb1, a->sB1, 64, BK, "B"))
+    if (make_map(dev, &tmB, a->B, a->in_dtype, a->N, a->K, a->ldb, nb0, a->sB0, nb1, a->sB1, p.b_wide,
+                 p.stage_kb * BK, p.b_wide ? b_cols / 64 : 1, "B"))
       return 1;
   }
 
@@ -1686,14 +1698,11 @@ extern "C" int vkg_gemm_group_launch(vkg_device* dev, const void* table, int n, 
                         SMEM_BYTES, 2, static_cast<const GroupEntry*>(table), n, units));
     return vkg_check_launch("gemm_group_pair_kernel");
   }
-  const int bn = 64 * ((total_units >> GROUP_BN_SHIFT) + 1);
   total_units &= (1 << GROUP_BN_SHIFT) - 1;
   int ctas = vkg_persistent_ctas(dev) < total_units ? vkg_persistent_ctas(dev) : total_units;
-  int stages = RING_BYTES / (A_STAGE_BYTES + bn * 128);
-  if (stages > MAX_STAGES) stages = MAX_STAGES;
   VKG_CUDA(vkg_launch(dev, VKG_K_GEMM_GROUP | vkg_short_if(total_units <= ctas), gemm_group_kernel,
                       dim3((unsigned)ctas), dim3(NUM_THREADS), SMEM_BYTES, 1,
-                      static_cast<const GroupEntry*>(table), n, total_units, bn, stages));
+                      static_cast<const GroupEntry*>(table), n, total_units));
   return vkg_check_launch("gemm_group_kernel");
 }
 
