@@ -54,13 +54,10 @@ struct GemmParams {
   int M, N, K;
   int nb0, nb1;
   int tiles_m, tiles_n;
-  int bn, num_kb;
-  int stages, stage_kb, stage_bytes;   // the ring of one CTA: stages, k-blocks and bytes of each
-  int rows_a, rows_b;                  // of the operands' tiles in one CTA
-  int a_wide, b_wide, a_loads, b_loads;   // Feed
+  int bn, stage_kb, num_kb;
   int split_k, kb_per_split;   // split_k > 1: z1 is the K slice, not a batch index
   int causal;                  // 0 none, 1 skip tiles above the diagonal, 2/3 clip the K range
-  int a_mn, b_mn;
+  int a_mn, b_mn;              // MN-major, and wide (Feed): OP_MN | OP_WIDE
   uint32_t idesc;
   int c_dtype, act, dact, vec_ok;
   long long ldc, sC0, sC1;
@@ -74,6 +71,19 @@ struct GemmParams {
   float alpha;
   int tma_store;               // epilogue stores C (and pre) through tensor maps
   uint32_t* err;
+};
+
+enum : int { OP_MN = 1, OP_WIDE = 2 };
+
+// The ring of one CTA.  rows_b: its rows of a K-major B, or columns of an MN-major one, which are loaded
+// in whole groups of 64 (a 96-column half of a pair's tile loads two and uses one and a half).
+struct RingShape {
+  int rows_b, stage_bytes, stages;
+  __host__ __device__ RingShape(bool pair, int bn, bool b_mn, int stage_kb) {
+    rows_b = pair ? bn / 2 : bn;
+    stage_bytes = stage_kb * (A_STAGE_BYTES + (b_mn ? (rows_b + 63) / 64 * 64 : rows_b) * 128);
+    stages = RING_BYTES / stage_bytes < MAX_STAGES ? RING_BYTES / stage_bytes : MAX_STAGES;
+  }
 };
 
 struct TileCoord {
@@ -463,14 +473,15 @@ struct Feed {
   int s0, s1, s2;        // their step per stage
   int loads;
   uint32_t step;         // shared-memory bytes from one load to the next
-  __device__ __forceinline__ Feed(bool mn, bool wide, int n, int kb0, int at, int rows, int stage_kb) {
+  __device__ __forceinline__ Feed(int kind, int kb0, int at, int rows, int stage_kb) {
+    const bool mn = (kind & OP_MN) != 0, wide = (kind & OP_WIDE) != 0;
     c0 = wide ? 0 : mn ? at : kb0 * BK;
     c1 = mn ? kb0 * BK : at;
     c2 = !wide ? 0 : mn ? at / 64 : kb0;
     s0 = wide || mn ? 0 : stage_kb * BK;
     s1 = mn ? stage_kb * BK : 0;
     s2 = wide && !mn ? stage_kb : 0;
-    loads = n;
+    loads = wide ? 1 : mn ? (rows + 63) / 64 : stage_kb;
     step = mn ? (uint32_t)stage_kb * 8192u : (uint32_t)rows * 128u;
   }
   template <bool PAIR>
@@ -491,16 +502,15 @@ struct Feed {
 
 // TMA producer (one lane) of a single CTA or of one CTA of a pair: stream the k-blocks of a work unit's
 // operands into the ring.  b_at: the CTA's first column of B.
-template <bool PAIR>
+template <bool PAIR, int STAGE_KB>
 __device__ __forceinline__ bool produce(const CtaCtx& cx, const GemmParams& p, const CUtensorMap* tmA,
                                         const CUtensorMap* tmB, TileCoord tc, int b_at, uint32_t rank, Ring& at) {
   int kb0, nkb;
   kb_range(p, tc, kb0, nkb);
   if (p.split_k > 1) tc.z1 = 0;   // operands are not batched along the slice index
-  Feed a(p.a_mn != 0, p.a_wide != 0, p.a_loads, kb0, tc.m0, p.rows_a, p.stage_kb);
-  Feed b(p.b_mn != 0, p.b_wide != 0, p.b_loads, kb0, b_at, p.rows_b, p.stage_kb);
-  const uint32_t a_bytes = (uint32_t)(p.stage_kb * p.rows_a) * 128u;
-  for (int kb = 0; kb < nkb; kb += p.stage_kb) {
+  Feed a(p.a_mn, kb0, tc.m0, BM, STAGE_KB), b(p.b_mn, kb0, b_at, PAIR ? p.bn / 2 : p.bn, STAGE_KB);
+  constexpr uint32_t a_bytes = STAGE_KB * A_STAGE_BYTES;
+  for (int kb = 0; kb < nkb; kb += STAGE_KB) {
     if (at.wrapped && !mbar_wait(cx.empty0 + 8 * at.stage, at.phase ^ 1u, cx.abort_flag, p.err, 0x100u + at.stage))
       return false;
     uint32_t fb = cx.full0 + 8 * at.stage;
@@ -526,10 +536,11 @@ __device__ __forceinline__ bool produce(const CtaCtx& cx, const GemmParams& p, c
 template <bool PAIR, int STAGE_KB>
 __device__ __forceinline__ bool multiply(const CtaCtx& cx, const GemmParams& p, uint32_t d_tmem, int nkb, Ring& at) {
   const uint32_t d_hi = smem_desc_hi(1024);
-  const uint32_t a_lo0 = smem_desc_lo(cx.base, p.a_mn ? STAGE_KB * 8192 : 16);
-  const uint32_t b_lo0 = smem_desc_lo(cx.base + STAGE_KB * p.rows_a * 128, p.b_mn ? STAGE_KB * 8192 : 16);
-  const uint32_t a_step = p.a_mn ? 128u : 2u, b_step = p.b_mn ? 128u : 2u;
-  const uint32_t a_kb = p.a_mn ? 512u : (uint32_t)p.rows_a * 8u, b_kb = p.b_mn ? 512u : (uint32_t)p.rows_b * 8u;
+  const bool a_mn = (p.a_mn & OP_MN) != 0, b_mn = (p.b_mn & OP_MN) != 0;
+  const uint32_t a_lo0 = smem_desc_lo(cx.base, a_mn ? STAGE_KB * 8192 : 16);
+  const uint32_t b_lo0 = smem_desc_lo(cx.base + STAGE_KB * A_STAGE_BYTES, b_mn ? STAGE_KB * 8192 : 16);
+  const uint32_t a_step = a_mn ? 128u : 2u, b_step = b_mn ? 128u : 2u;
+  const uint32_t a_kb = a_mn ? 512u : BM * 8u, b_kb = b_mn ? 512u : (uint32_t)(PAIR ? p.bn / 2 : p.bn) * 8u;
   const uint32_t stage16 = cx.stage_bytes >> 4;
   for (int kb = 0; kb < nkb; kb += STAGE_KB) {
     if (!mbar_wait_warp(cx.full0 + 8 * at.stage, at.phase, cx.abort_flag, p.err, 0x300u + at.stage)) return false;
@@ -557,7 +568,7 @@ __device__ __forceinline__ bool multiply(const CtaCtx& cx, const GemmParams& p, 
   return true;
 }
 
-template <bool PAIR>
+template <bool PAIR, int STAGE_KB>
 __device__ __forceinline__ bool mma_unit(const CtaCtx& cx, const GemmParams& p, int t, Ring& at, int& acc,
                                          uint32_t& acc_phase) {
   int kb0, nkb;
@@ -566,8 +577,7 @@ __device__ __forceinline__ bool mma_unit(const CtaCtx& cx, const GemmParams& p, 
   if (!mbar_wait_warp(cx.tempty0 + 8 * acc, acc_phase ^ 1u, cx.abort_flag, p.err, 0x200u + acc)) return false;
   tcgen05_fence_after();
   const uint32_t d_tmem = cx.tmem_base + (uint32_t)(acc * ACC_COLS);
-  if (!(p.stage_kb == 2 ? multiply<PAIR, 2>(cx, p, d_tmem, nkb, at) : multiply<PAIR, 1>(cx, p, d_tmem, nkb, at)))
-    return false;
+  if (!multiply<PAIR, STAGE_KB>(cx, p, d_tmem, nkb, at)) return false;
   if (elect_one()) {           // accumulator complete -> epilogue
     if (PAIR) umma2_commit(cx.tfull0 + 8 * acc);
     else umma_commit(cx.tfull0 + 8 * acc);
@@ -698,12 +708,12 @@ __device__ __forceinline__ bool epilogue_unit(const CtaCtx& cx, const GemmParams
 // Barriers, TMEM and the role-independent constants of a CTA.
 // (Issuing the first loads here, before tensor memory is allocated, measured 1 us SLOWER per launch:
 // the tensor maps prefetched at the top of the kernel are not there yet.)
-__device__ __forceinline__ void cta_setup(CtaCtx& cx, uint8_t* smem_raw, int stage_bytes, int stages) {
+__device__ __forceinline__ void cta_setup(CtaCtx& cx, uint8_t* smem_raw, const RingShape& ring) {
   // 128B-swizzled tiles want 1024-byte alignment.
   cx.base = (smem_u32(smem_raw) + 1023u) & ~1023u;
   uint8_t* gen_base = smem_raw + (cx.base - smem_u32(smem_raw));
-  cx.stage_bytes = (uint32_t)stage_bytes;
-  cx.n_stages = stages;
+  cx.stage_bytes = (uint32_t)ring.stage_bytes;
+  cx.n_stages = ring.stages;
   // Epilogue staging (one swizzled 32x16 fp32 chunk per epilogue warp), then the barrier block.
   cx.epi_stage = gen_base + RING_BYTES;
   uint64_t* bars = reinterpret_cast<uint64_t*>(gen_base + RING_BYTES + EPI_WARPS * EPI_STAGE_BYTES);
@@ -717,7 +727,7 @@ __device__ __forceinline__ void cta_setup(CtaCtx& cx, uint8_t* smem_raw, int sta
   cx.abort_flag = reinterpret_cast<volatile uint32_t*>(bars + 21);
   const int warp = threadIdx.x >> 5;
   if (threadIdx.x == 0) {
-    for (int s = 0; s < stages; ++s) {
+    for (int s = 0; s < cx.n_stages; ++s) {
       mbar_init(cx.full0 + 8 * s, 1);
       mbar_init(cx.empty0 + 8 * s, 1);
     }
@@ -763,7 +773,7 @@ __device__ __forceinline__ void cta_teardown(const CtaCtx& cx) {
 }
 
 // One GEMM: CTA b takes tiles b, b + gridDim.x, ...
-template <int MODE>
+template <int MODE, int STAGE_KB>
 __global__ void __launch_bounds__(NUM_THREADS, 1)
 gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                     const __grid_constant__ CUtensorMap tmC, const __grid_constant__ CUtensorMap tmP,
@@ -779,7 +789,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
     }
   }
   CtaCtx cx;
-  cta_setup(cx, smem_raw, p.stage_bytes, p.stages);
+  cta_setup(cx, smem_raw, RingShape(false, p.bn, p.b_mn & OP_MN, STAGE_KB));
   pdl_wait();      // barriers, TMEM and tensor maps are ready; operands may still be in flight
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
@@ -789,7 +799,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
       Ring at;
       for (int t = blockIdx.x; t < total_tiles; t += gridDim.x) {
         const TileCoord tc = tile_coord(p, t);
-        if (!produce<false>(cx, p, &tmA, &tmB, tc, tc.n0, 0, at)) break;
+        if (!produce<false, STAGE_KB>(cx, p, &tmA, &tmB, tc, tc.n0, 0, at)) break;
       }
     }
   } else if (warp == 1) {
@@ -797,7 +807,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
     int acc = 0;
     uint32_t acc_phase = 0;
     for (int t = blockIdx.x; t < total_tiles; t += gridDim.x)
-      if (!mma_unit<false>(cx, p, t, at, acc, acc_phase)) break;
+      if (!mma_unit<false, STAGE_KB>(cx, p, t, at, acc, acc_phase)) break;
   } else {
     int acc = 0;
     uint32_t acc_phase = 0;
@@ -835,15 +845,16 @@ __device__ __forceinline__ int group_find(const int* first, int n, int u) {
   return lo;
 }
 
+template <int STAGE_KB>
 __global__ void __launch_bounds__(NUM_THREADS, 1)
-gemm_group_kernel(const GroupEntry* __restrict__ table, int n_problems, int total_units) {
+gemm_group_kernel(const GroupEntry* __restrict__ table, int n_problems, int total_units, int bn) {
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   __shared__ int first[GROUP_MAX];
   pdl_trigger();
   // the table was written by the host long before this launch, not by the kernel before it
   for (int i = threadIdx.x; i < n_problems; i += blockDim.x) first[i] = table[i].first_unit;
   CtaCtx cx;
-  cta_setup(cx, smem_raw, table->p.stage_bytes, table->p.stages);   // the same for all; its __syncthreads also publishes first[]
+  cta_setup(cx, smem_raw, RingShape(false, bn, true, STAGE_KB));   // its __syncthreads also publishes first[]
   pdl_wait();
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
@@ -854,7 +865,7 @@ gemm_group_kernel(const GroupEntry* __restrict__ table, int n_problems, int tota
         const int pi = group_find(first, n_problems, u);
         const GemmParams p = table[pi].p;
         const TileCoord tc = tile_coord(p, u - first[pi]);
-        if (!produce<false>(cx, p, &table[pi].tmA, &table[pi].tmB, tc, tc.n0, 0, at)) break;
+        if (!produce<false, STAGE_KB>(cx, p, &table[pi].tmA, &table[pi].tmB, tc, tc.n0, 0, at)) break;
       }
     }
   } else if (warp == 1) {
@@ -864,7 +875,7 @@ gemm_group_kernel(const GroupEntry* __restrict__ table, int n_problems, int tota
     for (int u = blockIdx.x; u < total_units; u += gridDim.x) {
       const int pi = group_find(first, n_problems, u);
       const GemmParams p = table[pi].p;
-      if (!mma_unit<false>(cx, p, u - first[pi], at, acc, acc_phase)) break;
+      if (!mma_unit<false, STAGE_KB>(cx, p, u - first[pi], at, acc, acc_phase)) break;
     }
   } else {
     int acc = 0;
@@ -892,12 +903,12 @@ gemm_group_kernel(const GroupEntry* __restrict__ table, int n_problems, int tota
 constexpr int PAIR_BN = 256;        // widest pair tile; 192 is the other width (N = 768 shapes)
 // Barriers, TMEM and constants of one CTA of a pair; ends with a cluster-wide barrier so the
 // peer's mbarriers exist before anything is signalled on them.
-__device__ __forceinline__ void pair_setup(CtaCtx& cx, uint8_t* smem_raw, int stage_bytes, int stages) {
+__device__ __forceinline__ void pair_setup(CtaCtx& cx, uint8_t* smem_raw, const RingShape& ring) {
   const int warp = threadIdx.x >> 5;
   cx.base = (smem_u32(smem_raw) + 1023u) & ~1023u;
   uint8_t* gen_base = smem_raw + (cx.base - smem_u32(smem_raw));
-  cx.stage_bytes = (uint32_t)stage_bytes;
-  cx.n_stages = stages;
+  cx.stage_bytes = (uint32_t)ring.stage_bytes;
+  cx.n_stages = ring.stages;
   cx.epi_stage = gen_base + RING_BYTES;
   uint64_t* bars = reinterpret_cast<uint64_t*>(gen_base + RING_BYTES + EPI_WARPS * EPI_STAGE_BYTES);
   const uint32_t bar_base = cx.base + RING_BYTES + EPI_WARPS * EPI_STAGE_BYTES;
@@ -986,7 +997,7 @@ __device__ __forceinline__ bool pair_epilogue_unit(const CtaCtx& cx, const GemmP
   return true;
 }
 
-template <int MODE>
+template <int MODE, int STAGE_KB>
 __global__ void __launch_bounds__(NUM_THREADS, 1)
 gemm_cta_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                      const __grid_constant__ CUtensorMap tmC, const __grid_constant__ CUtensorMap tmP,
@@ -1005,7 +1016,7 @@ gemm_cta_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
     }
   }
   CtaCtx cx;
-  pair_setup(cx, smem_raw, p.stage_bytes, p.stages);
+  pair_setup(cx, smem_raw, RingShape(true, p.bn, p.b_mn & OP_MN, STAGE_KB));
   pdl_wait();
   const int n_pairs = (int)gridDim.x >> 1, pair = (int)blockIdx.x >> 1;
   const int total_tiles = p.tiles_m * p.tiles_n * p.nb0 * (p.split_k > 1 ? p.split_k : p.nb1);
@@ -1014,7 +1025,7 @@ gemm_cta_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
       Ring at;
       for (int t = pair; t < total_tiles; t += n_pairs) {
         const TileCoord tc = pair_coord(p, t, rank);
-        if (!produce<true>(cx, p, &tmA, &tmB, tc, tc.n0 + (int)rank * p.rows_b, rank, at)) break;
+        if (!produce<true, STAGE_KB>(cx, p, &tmA, &tmB, tc, tc.n0 + (int)rank * (p.bn / 2), rank, at)) break;
       }
     }
   } else if (warp == 1) {
@@ -1023,7 +1034,7 @@ gemm_cta_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
       int acc = 0;
       uint32_t acc_phase = 0;
       for (int t = pair; t < total_tiles; t += n_pairs)
-        if (!mma_unit<true>(cx, p, t, at, acc, acc_phase)) break;
+        if (!mma_unit<true, STAGE_KB>(cx, p, t, at, acc, acc_phase)) break;
     }
   } else {
     int acc = 0;
@@ -1046,7 +1057,7 @@ gemm_group_pair_kernel(const GroupEntry* __restrict__ table, int n_problems, int
   const int lane = threadIdx.x & 31;
   const uint32_t rank = cluster_ctarank();
   CtaCtx cx;
-  pair_setup(cx, smem_raw, table->p.stage_bytes, table->p.stages);   // the same for all; publishes first[]
+  pair_setup(cx, smem_raw, RingShape(true, PAIR_BN, true, 1));   // publishes first[]
   pdl_wait();
   const int n_pairs = (int)gridDim.x >> 1, pair = (int)blockIdx.x >> 1;
   if (warp == 0) {
@@ -1056,7 +1067,7 @@ gemm_group_pair_kernel(const GroupEntry* __restrict__ table, int n_problems, int
         const int pi = group_find(first, n_problems, u);
         const GemmParams p = table[pi].p;
         const TileCoord tc = pair_coord(p, u - first[pi], rank);
-        if (!produce<true>(cx, p, &table[pi].tmA, &table[pi].tmB, tc, tc.n0 + (int)rank * p.rows_b, rank, at)) break;
+        if (!produce<true, 1>(cx, p, &table[pi].tmA, &table[pi].tmB, tc, tc.n0 + (int)rank * (p.bn / 2), rank, at)) break;
       }
     }
   } else if (warp == 1) {
@@ -1067,7 +1078,7 @@ gemm_group_pair_kernel(const GroupEntry* __restrict__ table, int n_problems, int
       for (int u = pair; u < total_units; u += n_pairs) {
         const int pi = group_find(first, n_problems, u);
         const GemmParams p = table[pi].p;
-        if (!mma_unit<true>(cx, p, u - first[pi], at, acc, acc_phase)) break;
+        if (!mma_unit<true, 1>(cx, p, u - first[pi], at, acc, acc_phase)) break;
       }
     }
   } else {
@@ -1107,9 +1118,9 @@ typedef void (*GemmKernel)(const CUtensorMap, const CUtensorMap, const CUtensorM
                            const GemmParams);
 struct Specialised {
   int mode;
-  GemmKernel fn;
+  GemmKernel fn[2];      // one and two k-blocks to a stage
 };
-#define VKG_SPEC(m) {(m), gemm_tcgen05_kernel<(m)>}
+#define VKG_SPEC(m) {(m), {gemm_tcgen05_kernel<(m), 1>, gemm_tcgen05_kernel<(m), 2>}}
 // The epilogues the training step uses; anything else runs the generic kernel.
 const Specialised kSpecialised[] = {
     VKG_SPEC(0),                                   // fp32 out: dW, dX into layernorm, scores
@@ -1121,9 +1132,10 @@ const Specialised kSpecialised[] = {
     VKG_SPEC(E_BIAS | E_ACT | E_F16),              // the same without a backward to keep z for
     VKG_SPEC(E_DACT | E_F16),                      // fc2 dX: * GELU'(z), narrow
     VKG_SPEC(E_DACT | E_F16 | E_COLSUM),           // the same + column sums = fc1's bias gradient
+    VKG_SPEC(E_GENERIC),                           // last: whatever is not above
 };
 const int kNumSpecialised = sizeof(kSpecialised) / sizeof(kSpecialised[0]);
-#define VKG_SPEC_CP(m) {(m), gemm_cta_pair_kernel<(m)>}
+#define VKG_SPEC_CP(m) {(m), {gemm_cta_pair_kernel<(m), 1>, gemm_cta_pair_kernel<(m), 2>}}
 // The same epilogues on 256 x 256 tiles computed by CTA pairs.
 const Specialised kCtaPair[] = {
     VKG_SPEC_CP(0),
@@ -1135,12 +1147,13 @@ const Specialised kCtaPair[] = {
     VKG_SPEC_CP(E_BIAS | E_ACT | E_F16),
     VKG_SPEC_CP(E_DACT | E_F16),
     VKG_SPEC_CP(E_DACT | E_F16 | E_COLSUM),
+    VKG_SPEC_CP(E_GENERIC),
 };
 const int kNumCtaPair = sizeof(kCtaPair) / sizeof(kCtaPair[0]);
-GemmKernel pick(const Specialised* t, int n, GemmKernel generic, int mode) {
-  for (int i = 0; i < n; ++i)
-    if (t[i].mode == mode) return t[i].fn;
-  return generic;
+GemmKernel pick(const Specialised* t, int n, int mode, int stage_kb) {
+  int i = 0;
+  while (i + 1 < n && t[i].mode != mode) ++i;
+  return t[i].fn[stage_kb - 1];
 }
 typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*,
                                   const cuuint64_t*, const cuuint64_t*, const cuuint32_t*,
@@ -1417,6 +1430,9 @@ int check_args(const vkg_gemm_args* a) {
   return 0;
 }
 
+// Two k-blocks to a stage where that leaves three stages (the 192-wide pair tile does too).
+int single_stage_kb(int bn) { return RING_BYTES / (2 * (A_STAGE_BYTES + bn * 128)) >= 3 ? 2 : 1; }
+
 // use_pair: 256 x bn tiles for gemm_cta_pair_kernel (the caller has checked the shape).
 int build_problem(vkg_device* dev, const vkg_gemm_args* a, Problem* out, bool use_pair, int bn, int want_split) {
   if (check_args(a)) return 1;
@@ -1432,23 +1448,15 @@ int build_problem(vkg_device* dev, const vkg_gemm_args* a, Problem* out, bool us
   p.tiles_n = (a->N + bn - 1) / bn;
   p.bn = bn;
   p.num_kb = (a->K + BK - 1) / BK;
-  p.a_mn = a->trans_a ? 1 : 0;
-  p.b_mn = a->trans_b ? 0 : 1;
-  p.rows_a = BM;
-  p.rows_b = use_pair ? bn / 2 : bn;
-  // the CTA's columns of an MN-major B in whole groups: a 96-column half loads two and uses one and a half
-  const int b_cols = (p.rows_b + 63) / 64 * 64;
-  const int kb_bytes = A_STAGE_BYTES + (p.b_mn ? b_cols : p.rows_b) * 128;
-  p.stage_kb = !(use_pair && bn == PAIR_BN) && RING_BYTES / (2 * kb_bytes) >= 3 ? 2 : 1;
-  p.stage_bytes = p.stage_kb * kb_bytes;
-  p.stages = std::min(RING_BYTES / p.stage_bytes, MAX_STAGES);
-  p.a_wide = (p.a_mn ? a->M : a->K) % 64 == 0;
-  p.b_wide = (p.b_mn ? a->N : a->K) % 64 == 0 && (!p.b_mn || p.rows_b == b_cols);
-  p.a_loads = p.a_wide ? 1 : p.a_mn ? BM / 64 : p.stage_kb;
-  p.b_loads = p.b_wide ? 1 : p.b_mn ? b_cols / 64 : p.stage_kb;
+  p.stage_kb = use_pair ? (bn == PAIR_BN ? 1 : 2) : single_stage_kb(bn);
+  const int rows_b = use_pair ? bn / 2 : bn, b_groups = (rows_b + 63) / 64;
+  const bool a_wide = (a->trans_a ? a->M : a->K) % 64 == 0;
+  const bool b_wide = (a->trans_b ? a->K : a->N) % 64 == 0 && (a->trans_b || rows_b % 64 == 0);
+  p.a_mn = (a->trans_a ? OP_MN : 0) | (a_wide ? OP_WIDE : 0);
+  p.b_mn = (a->trans_b ? 0 : OP_MN) | (b_wide ? OP_WIDE : 0);
   const uint32_t fmt = a->in_dtype == VKG_BF16 ? 1u : 0u;
-  p.idesc = (1u << 4) | (fmt << 7) | (fmt << 10) | ((uint32_t)p.a_mn << 15) |
-            ((uint32_t)p.b_mn << 16) | ((uint32_t)(bn >> 3) << 17) | ((uint32_t)(bm >> 4) << 24);
+  p.idesc = (1u << 4) | (fmt << 7) | (fmt << 10) | ((uint32_t)(p.a_mn & OP_MN) << 15) |
+            ((uint32_t)(p.b_mn & OP_MN) << 16) | ((uint32_t)(bn >> 3) << 17) | ((uint32_t)(bm >> 4) << 24);
   p.c_dtype = a->c_dtype; p.act = a->act; p.dact = a->dact;
   p.ldc = a->ldc; p.sC0 = a->sC0; p.sC1 = a->sC1;
   p.C = a->C; p.C2 = a->C2; p.bias = a->bias; p.pre = a->pre;
@@ -1490,24 +1498,24 @@ int build_problem(vkg_device* dev, const vkg_gemm_args* a, Problem* out, bool us
   CUtensorMap& tmB = out->tmB;
   if (!a->trans_a) {
     VKG_REQUIRE(a->lda >= a->K, "gemm: lda %lld < K %d", (long long)a->lda, a->K);
-    if (make_map(dev, &tmA, a->A, a->in_dtype, a->K, a->M, a->lda, nb0, a->sA0, nb1, a->sA1, p.a_wide, BM,
-                 p.a_wide ? p.stage_kb : 1, "A"))
+    if (make_map(dev, &tmA, a->A, a->in_dtype, a->K, a->M, a->lda, nb0, a->sA0, nb1, a->sA1, a_wide, BM,
+                 a_wide ? p.stage_kb : 1, "A"))
       return 1;
   } else {
     VKG_REQUIRE(a->lda >= a->M, "gemm: lda %lld < M %d (A stored K x M)", (long long)a->lda, a->M);
-    if (make_map(dev, &tmA, a->A, a->in_dtype, a->M, a->K, a->lda, nb0, a->sA0, nb1, a->sA1, p.a_wide,
-                 p.stage_kb * BK, p.a_wide ? BM / 64 : 1, "A^T"))
+    if (make_map(dev, &tmA, a->A, a->in_dtype, a->M, a->K, a->lda, nb0, a->sA0, nb1, a->sA1, a_wide,
+                 p.stage_kb * BK, a_wide ? BM / 64 : 1, "A^T"))
       return 1;
   }
   if (a->trans_b) {
     VKG_REQUIRE(a->ldb >= a->K, "gemm: ldb %lld < K %d (B stored N x K)", (long long)a->ldb, a->K);
-    if (make_map(dev, &tmB, a->B, a->in_dtype, a->K, a->N, a->ldb, nb0, a->sB0, nb1, a->sB1, p.b_wide,
-                 p.rows_b, p.b_wide ? p.stage_kb : 1, "B^T"))
+    if (make_map(dev, &tmB, a->B, a->in_dtype, a->K, a->N, a->ldb, nb0, a->sB0, nb1, a->sB1, b_wide,
+                 rows_b, b_wide ? p.stage_kb : 1, "B^T"))
       return 1;
   } else {
     VKG_REQUIRE(a->ldb >= a->N, "gemm: ldb %lld < N %d", (long long)a->ldb, a->N);
-    if (make_map(dev, &tmB, a->B, a->in_dtype, a->N, a->K, a->ldb, nb0, a->sB0, nb1, a->sB1, p.b_wide,
-                 p.stage_kb * BK, p.b_wide ? b_cols / 64 : 1, "B"))
+    if (make_map(dev, &tmB, a->B, a->in_dtype, a->N, a->K, a->ldb, nb0, a->sB0, nb1, a->sB1, b_wide,
+                 p.stage_kb * BK, b_wide ? b_groups : 1, "B"))
       return 1;
   }
 
@@ -1542,16 +1550,10 @@ int ensure_attrs(vkg_device* dev) {
   VKG_REQUIRE((size_t)SMEM_BYTES <= dev->gemm_smem_optin,
               "gemm needs %d bytes of shared memory, device offers %zu", SMEM_BYTES,
               dev->gemm_smem_optin);
-  VKG_CUDA(cudaFuncSetAttribute(gemm_tcgen05_kernel<E_GENERIC>,
-                                cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES));
-  for (int i = 0; i < kNumSpecialised; ++i)
-    VKG_CUDA(cudaFuncSetAttribute(kSpecialised[i].fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  SMEM_BYTES));
-  VKG_CUDA(cudaFuncSetAttribute(gemm_cta_pair_kernel<E_GENERIC>,
-                                cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES));
-  for (int i = 0; i < kNumCtaPair; ++i)
-    VKG_CUDA(cudaFuncSetAttribute(kCtaPair[i].fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  SMEM_BYTES));
+  for (const Specialised& k : kSpecialised)
+    for (GemmKernel fn : k.fn) VKG_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES));
+  for (const Specialised& k : kCtaPair)
+    for (GemmKernel fn : k.fn) VKG_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES));
   dev->gemm_attr_set = true;
   return 0;
 }
@@ -1684,8 +1686,8 @@ extern "C" int vkg_gemm_group_launch(vkg_device* dev, const void* table, int n, 
   VKG_REQUIRE(table && n > 0 && n <= GROUP_MAX && total_units != 0, "gemm_group: bad arguments");
   if (ensure_attrs(dev)) return 1;
   if (!dev->group_attr_set) {
-    VKG_CUDA(cudaFuncSetAttribute(gemm_group_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  SMEM_BYTES));
+    for (auto fn : {gemm_group_kernel<1>, gemm_group_kernel<2>})
+      VKG_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES));
     VKG_CUDA(cudaFuncSetAttribute(gemm_group_pair_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                   SMEM_BYTES));
     dev->group_attr_set = true;
@@ -1698,11 +1700,13 @@ extern "C" int vkg_gemm_group_launch(vkg_device* dev, const void* table, int n, 
                         SMEM_BYTES, 2, static_cast<const GroupEntry*>(table), n, units));
     return vkg_check_launch("gemm_group_pair_kernel");
   }
+  const int bn = 64 * ((total_units >> GROUP_BN_SHIFT) + 1);
   total_units &= (1 << GROUP_BN_SHIFT) - 1;
   int ctas = vkg_persistent_ctas(dev) < total_units ? vkg_persistent_ctas(dev) : total_units;
-  VKG_CUDA(vkg_launch(dev, VKG_K_GEMM_GROUP | vkg_short_if(total_units <= ctas), gemm_group_kernel,
+  VKG_CUDA(vkg_launch(dev, VKG_K_GEMM_GROUP | vkg_short_if(total_units <= ctas),
+                      single_stage_kb(bn) == 2 ? gemm_group_kernel<2> : gemm_group_kernel<1>,
                       dim3((unsigned)ctas), dim3(NUM_THREADS), SMEM_BYTES, 1,
-                      static_cast<const GroupEntry*>(table), n, total_units));
+                      static_cast<const GroupEntry*>(table), n, total_units, bn));
   return vkg_check_launch("gemm_group_kernel");
 }
 
@@ -1738,7 +1742,7 @@ int make_plan(vkg_device* dev, const vkg_gemm_args* a, GemmPlan* out) {
   const bool use_pair = t.pair;
   if (build_problem(dev, a, &q, use_pair, t.bn, t.split)) return 1;
   if (use_pair) {
-    out->fn = pick(kCtaPair, kNumCtaPair, gemm_cta_pair_kernel<E_GENERIC>, q.mode);
+    out->fn = pick(kCtaPair, kNumCtaPair, q.mode, q.p.stage_kb);
     long long pairs = vkg_persistent_ctas(dev) / 2;
     if (pairs > q.total_tiles) pairs = q.total_tiles;
     out->family = VKG_K_GEMM_PAIR;
@@ -1746,7 +1750,7 @@ int make_plan(vkg_device* dev, const vkg_gemm_args* a, GemmPlan* out) {
     out->cluster = 2;
     out->tile_rows = 2 * BM;
   } else {
-    out->fn = pick(kSpecialised, kNumSpecialised, gemm_tcgen05_kernel<E_GENERIC>, q.mode);
+    out->fn = pick(kSpecialised, kNumSpecialised, q.mode, q.p.stage_kb);
     long long ctas = a->max_ctas > 0 ? a->max_ctas : vkg_persistent_ctas(dev);
     if (ctas > q.total_tiles) ctas = q.total_tiles;
     out->family = VKG_K_GEMM;
