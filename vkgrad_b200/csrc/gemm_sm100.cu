@@ -1245,6 +1245,7 @@ constexpr KBlockCost KB_TN = {{0.245, 0.300, 0.335, 0.400}, {0.330, 0.375}};
 constexpr double PL_LAUNCH = 3.43;     // launch, set-up, first load, drain
 constexpr double PL_EPI = 0.69, PL_EPI_COL = 0.00658;   // epilogue of a tile, per column at fp32 out
 constexpr double PL_PAIR = 1.29;       // a pair's barriers and its later start
+constexpr double PL_SHORT_US = 12.0;   // a launch that overlaps its predecessor, whatever its waves
 constexpr double PL_IDLE = 0.81;       // k-block cost with one CTA busy, of that with all
 constexpr double PL_WAVE = 0.95;       // per further wave
 constexpr double PL_OVERLAP = 1.42;    // epilogue beside a main loop, of the epilogue alone
@@ -1717,7 +1718,7 @@ struct GemmPlan {
   Problem q;
   GemmKernel fn;
   unsigned family, grid;
-  bool one_wave;      // no CTA works on a second tile
+  bool is_short;      // VKG_SHORT
   int cluster;        // CTAs per thread-block cluster
   int tile_rows;      // rows of C per tile, for the column sums' partial rows
 };
@@ -1758,7 +1759,8 @@ int make_plan(vkg_device* dev, const vkg_gemm_args* a, GemmPlan* out) {
     out->cluster = 1;
     out->tile_rows = BM;
   }
-  out->one_wave = q.total_tiles * out->cluster <= (long long)out->grid;
+  // no CTA works on a second tile, or it is over soon all the same
+  out->is_short = q.total_tiles * out->cluster <= (long long)out->grid || t.us < PL_SHORT_US;
   return 0;
 }
 
@@ -1807,7 +1809,7 @@ int find_plan(vkg_device* dev, const vkg_gemm_args* a, GemmPlan* out) {
 
 int launch_plan(vkg_device* dev, const vkg_gemm_args* a, const GemmPlan& pl) {
   const Problem& q = pl.q;
-  VKG_CUDA(vkg_launch(dev, pl.family | vkg_short_if(pl.one_wave), pl.fn, dim3(pl.grid), dim3(NUM_THREADS),
+  VKG_CUDA(vkg_launch(dev, pl.family | vkg_short_if(pl.is_short), pl.fn, dim3(pl.grid), dim3(NUM_THREADS),
                       SMEM_BYTES, pl.cluster, q.tmA, q.tmB, q.tmC, q.tmP, q.p));
   if (vkg_check_launch("gemm")) return 1;
   if (reduce_slices(dev, a, q.p)) return 1;
