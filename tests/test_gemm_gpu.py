@@ -531,3 +531,55 @@ def test_grouped_dw_launch_equals_separate_launches(dev, pair):
         assert relerr(res[1][j], orc.matmul16(xs[j], dys[j], True, False)) < TOL
     for b in bx + bdy:
         b.destroy()
+
+
+@pytest.mark.parametrize("ta,tb", [(False, False), (False, True), (True, False), (True, True)])
+@pytest.mark.parametrize("m,n,k,split_k", [
+    (128, 64, 64, 1),          # one k-block: half of a two-k-block stage
+    (256, 128, 192, 1),        # three: the last stage is half full
+    (320, 448, 1024, 1),       # every operand wide, a last column group and row block of 64
+    (136, 200, 136, 1),        # none wide, all dimensions end inside a piece
+    (264, 192, 1096, 1),       # B wide where its columns are contiguous, more stages than the ring
+    (192, 264, 576, 3),        # slices of three k-blocks: a stage's second belongs to the next slice
+    (200, 136, 600, 3),
+])
+def test_loads_of_every_tile(dev, m, n, k, split_k, ta, tb):
+    """Operands by one load per stage or one per 64-element piece, one or two k-blocks to a stage:
+    the same bits from every tile, and the oracle's product."""
+    from vkgrad_b200.kernels import gemm
+    rng = np.random.default_rng(m + 3 * n + 7 * k)
+    a = rng.standard_normal((k, m) if ta else (m, k)).astype(np.float16)
+    b = rng.standard_normal((n, k) if tb else (k, n)).astype(np.float16)
+    ba, bb = up(dev, a), up(dev, b)
+    outs = []
+    for pair, tn in ((-1, 64), (-1, 128), (-1, 192), (-1, 256), (1, 192), (1, 256)):
+        bc = up(dev, np.full((m, n), np.nan, np.float32))
+        gemm(dev, ba, bb, bc, m, n, k, trans_a=ta, trans_b=tb, split_k=split_k, cta_pair=pair, tile_n=tn)
+        outs.append(down(dev, bc, np.float32, (m, n)))
+        bc.destroy()
+    # fp32 sums of exact products: 1e-6 per term at most, in another order than numpy's
+    assert relerr(outs[0], orc.matmul16(a, b, ta, tb)) < 5e-5
+    for o in outs[1:]:
+        assert np.array_equal(outs[0], o)
+    for x in (ba, bb):
+        x.destroy()
+
+
+def test_loads_of_a_group(dev):
+    """Problems of one grouped launch whose operands are loaded differently share the ring."""
+    from vkgrad_b200.kernels import gemm_group
+    rng = np.random.default_rng(5)
+    k, sizes = 328, [(128, 256), (200, 136), (64, 72), (320, 64)]
+    made, problems = [], []
+    for m, n in sizes:
+        x, dy = (rng.standard_normal((k, c)).astype(np.float16) for c in (m, n))
+        bx, by, bc = up(dev, x), up(dev, dy), up(dev, np.full((m, n), np.nan, np.float32))
+        made.append((x, dy, bx, by, bc, m, n))
+        problems.append((bx, by, bc, m, n, k, dict(trans_a=True)))
+    for pair in (0, 1):
+        gemm_group(dev, problems, cta_pair=pair)
+        for x, dy, _, _, bc, m, n in made:
+            assert relerr(down(dev, bc, np.float32, (m, n)), orc.matmul16(x, dy, True, False)) < 5e-5
+    for _, _, bx, by, bc, _, _ in made:
+        for t in (bx, by, bc):
+            t.destroy()
