@@ -502,15 +502,15 @@ struct Feed {
 
 // TMA producer (one lane) of a single CTA or of one CTA of a pair: stream the k-blocks of a work unit's
 // operands into the ring.  b_at: the CTA's first column of B.
-template <bool PAIR, int STAGE_KB>
+template <bool PAIR>
 __device__ __forceinline__ bool produce(const CtaCtx& cx, const GemmParams& p, const CUtensorMap* tmA,
                                         const CUtensorMap* tmB, TileCoord tc, int b_at, uint32_t rank, Ring& at) {
   int kb0, nkb;
   kb_range(p, tc, kb0, nkb);
   if (p.split_k > 1) tc.z1 = 0;   // operands are not batched along the slice index
-  Feed a(p.a_mn, kb0, tc.m0, BM, STAGE_KB), b(p.b_mn, kb0, b_at, PAIR ? p.bn / 2 : p.bn, STAGE_KB);
-  constexpr uint32_t a_bytes = STAGE_KB * A_STAGE_BYTES;
-  for (int kb = 0; kb < nkb; kb += STAGE_KB) {
+  Feed a(p.a_mn, kb0, tc.m0, BM, p.stage_kb), b(p.b_mn, kb0, b_at, PAIR ? p.bn / 2 : p.bn, p.stage_kb);
+  const uint32_t a_bytes = (uint32_t)p.stage_kb * A_STAGE_BYTES;
+  for (int kb = 0; kb < nkb; kb += p.stage_kb) {
     if (at.wrapped && !mbar_wait(cx.empty0 + 8 * at.stage, at.phase ^ 1u, cx.abort_flag, p.err, 0x100u + at.stage))
       return false;
     uint32_t fb = cx.full0 + 8 * at.stage;
@@ -568,7 +568,7 @@ __device__ __forceinline__ bool multiply(const CtaCtx& cx, const GemmParams& p, 
   return true;
 }
 
-template <bool PAIR, int STAGE_KB>
+template <bool PAIR>
 __device__ __forceinline__ bool mma_unit(const CtaCtx& cx, const GemmParams& p, int t, Ring& at, int& acc,
                                          uint32_t& acc_phase) {
   int kb0, nkb;
@@ -577,7 +577,10 @@ __device__ __forceinline__ bool mma_unit(const CtaCtx& cx, const GemmParams& p, 
   if (!mbar_wait_warp(cx.tempty0 + 8 * acc, acc_phase ^ 1u, cx.abort_flag, p.err, 0x200u + acc)) return false;
   tcgen05_fence_after();
   const uint32_t d_tmem = cx.tmem_base + (uint32_t)(acc * ACC_COLS);
-  if (!multiply<PAIR, STAGE_KB>(cx, p, d_tmem, nkb, at)) return false;
+  // (a kernel for each of the two loops made steps that use both longer: 259 -> 264 us of a block run
+  // through the op dictionaries, 2385 -> 2412 of four microbatches with heads of 32)
+  if (!(p.stage_kb == 2 ? multiply<PAIR, 2>(cx, p, d_tmem, nkb, at) : multiply<PAIR, 1>(cx, p, d_tmem, nkb, at)))
+    return false;
   if (elect_one()) {           // accumulator complete -> epilogue
     if (PAIR) umma2_commit(cx.tfull0 + 8 * acc);
     else umma_commit(cx.tfull0 + 8 * acc);
@@ -773,7 +776,7 @@ __device__ __forceinline__ void cta_teardown(const CtaCtx& cx) {
 }
 
 // One GEMM: CTA b takes tiles b, b + gridDim.x, ...
-template <int MODE, int STAGE_KB>
+template <int MODE>
 __global__ void __launch_bounds__(NUM_THREADS, 1)
 gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                     const __grid_constant__ CUtensorMap tmC, const __grid_constant__ CUtensorMap tmP,
@@ -789,7 +792,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
     }
   }
   CtaCtx cx;
-  cta_setup(cx, smem_raw, RingShape(false, p.bn, p.b_mn & OP_MN, STAGE_KB));
+  cta_setup(cx, smem_raw, RingShape(false, p.bn, p.b_mn & OP_MN, p.stage_kb));
   pdl_wait();      // barriers, TMEM and tensor maps are ready; operands may still be in flight
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
@@ -799,7 +802,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
       Ring at;
       for (int t = blockIdx.x; t < total_tiles; t += gridDim.x) {
         const TileCoord tc = tile_coord(p, t);
-        if (!produce<false, STAGE_KB>(cx, p, &tmA, &tmB, tc, tc.n0, 0, at)) break;
+        if (!produce<false>(cx, p, &tmA, &tmB, tc, tc.n0, 0, at)) break;
       }
     }
   } else if (warp == 1) {
@@ -807,7 +810,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
     int acc = 0;
     uint32_t acc_phase = 0;
     for (int t = blockIdx.x; t < total_tiles; t += gridDim.x)
-      if (!mma_unit<false, STAGE_KB>(cx, p, t, at, acc, acc_phase)) break;
+      if (!mma_unit<false>(cx, p, t, at, acc, acc_phase)) break;
   } else {
     int acc = 0;
     uint32_t acc_phase = 0;
@@ -845,7 +848,6 @@ __device__ __forceinline__ int group_find(const int* first, int n, int u) {
   return lo;
 }
 
-template <int STAGE_KB>
 __global__ void __launch_bounds__(NUM_THREADS, 1)
 gemm_group_kernel(const GroupEntry* __restrict__ table, int n_problems, int total_units, int bn) {
   extern __shared__ __align__(1024) uint8_t smem_raw[];
@@ -854,7 +856,7 @@ gemm_group_kernel(const GroupEntry* __restrict__ table, int n_problems, int tota
   // the table was written by the host long before this launch, not by the kernel before it
   for (int i = threadIdx.x; i < n_problems; i += blockDim.x) first[i] = table[i].first_unit;
   CtaCtx cx;
-  cta_setup(cx, smem_raw, RingShape(false, bn, true, STAGE_KB));   // its __syncthreads also publishes first[]
+  cta_setup(cx, smem_raw, RingShape(false, bn, true, table->p.stage_kb));   // its __syncthreads also publishes first[]
   pdl_wait();
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
@@ -865,7 +867,7 @@ gemm_group_kernel(const GroupEntry* __restrict__ table, int n_problems, int tota
         const int pi = group_find(first, n_problems, u);
         const GemmParams p = table[pi].p;
         const TileCoord tc = tile_coord(p, u - first[pi]);
-        if (!produce<false, STAGE_KB>(cx, p, &table[pi].tmA, &table[pi].tmB, tc, tc.n0, 0, at)) break;
+        if (!produce<false>(cx, p, &table[pi].tmA, &table[pi].tmB, tc, tc.n0, 0, at)) break;
       }
     }
   } else if (warp == 1) {
@@ -875,7 +877,7 @@ gemm_group_kernel(const GroupEntry* __restrict__ table, int n_problems, int tota
     for (int u = blockIdx.x; u < total_units; u += gridDim.x) {
       const int pi = group_find(first, n_problems, u);
       const GemmParams p = table[pi].p;
-      if (!mma_unit<false, STAGE_KB>(cx, p, u - first[pi], at, acc, acc_phase)) break;
+      if (!mma_unit<false>(cx, p, u - first[pi], at, acc, acc_phase)) break;
     }
   } else {
     int acc = 0;
@@ -997,7 +999,7 @@ __device__ __forceinline__ bool pair_epilogue_unit(const CtaCtx& cx, const GemmP
   return true;
 }
 
-template <int MODE, int STAGE_KB>
+template <int MODE>
 __global__ void __launch_bounds__(NUM_THREADS, 1)
 gemm_cta_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                      const __grid_constant__ CUtensorMap tmC, const __grid_constant__ CUtensorMap tmP,
@@ -1016,7 +1018,7 @@ gemm_cta_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
     }
   }
   CtaCtx cx;
-  pair_setup(cx, smem_raw, RingShape(true, p.bn, p.b_mn & OP_MN, STAGE_KB));
+  pair_setup(cx, smem_raw, RingShape(true, p.bn, p.b_mn & OP_MN, p.stage_kb));
   pdl_wait();
   const int n_pairs = (int)gridDim.x >> 1, pair = (int)blockIdx.x >> 1;
   const int total_tiles = p.tiles_m * p.tiles_n * p.nb0 * (p.split_k > 1 ? p.split_k : p.nb1);
@@ -1025,7 +1027,7 @@ gemm_cta_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
       Ring at;
       for (int t = pair; t < total_tiles; t += n_pairs) {
         const TileCoord tc = pair_coord(p, t, rank);
-        if (!produce<true, STAGE_KB>(cx, p, &tmA, &tmB, tc, tc.n0 + (int)rank * (p.bn / 2), rank, at)) break;
+        if (!produce<true>(cx, p, &tmA, &tmB, tc, tc.n0 + (int)rank * (p.bn / 2), rank, at)) break;
       }
     }
   } else if (warp == 1) {
@@ -1034,7 +1036,7 @@ gemm_cta_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
       int acc = 0;
       uint32_t acc_phase = 0;
       for (int t = pair; t < total_tiles; t += n_pairs)
-        if (!mma_unit<true, STAGE_KB>(cx, p, t, at, acc, acc_phase)) break;
+        if (!mma_unit<true>(cx, p, t, at, acc, acc_phase)) break;
     }
   } else {
     int acc = 0;
@@ -1067,7 +1069,7 @@ gemm_group_pair_kernel(const GroupEntry* __restrict__ table, int n_problems, int
         const int pi = group_find(first, n_problems, u);
         const GemmParams p = table[pi].p;
         const TileCoord tc = pair_coord(p, u - first[pi], rank);
-        if (!produce<true, 1>(cx, p, &table[pi].tmA, &table[pi].tmB, tc, tc.n0 + (int)rank * (p.bn / 2), rank, at)) break;
+        if (!produce<true>(cx, p, &table[pi].tmA, &table[pi].tmB, tc, tc.n0 + (int)rank * (p.bn / 2), rank, at)) break;
       }
     }
   } else if (warp == 1) {
@@ -1078,7 +1080,7 @@ gemm_group_pair_kernel(const GroupEntry* __restrict__ table, int n_problems, int
       for (int u = pair; u < total_units; u += n_pairs) {
         const int pi = group_find(first, n_problems, u);
         const GemmParams p = table[pi].p;
-        if (!mma_unit<true, 1>(cx, p, u - first[pi], at, acc, acc_phase)) break;
+        if (!mma_unit<true>(cx, p, u - first[pi], at, acc, acc_phase)) break;
       }
     }
   } else {
@@ -1118,9 +1120,9 @@ typedef void (*GemmKernel)(const CUtensorMap, const CUtensorMap, const CUtensorM
                            const GemmParams);
 struct Specialised {
   int mode;
-  GemmKernel fn[2];      // one and two k-blocks to a stage
+  GemmKernel fn;
 };
-#define VKG_SPEC(m) {(m), {gemm_tcgen05_kernel<(m), 1>, gemm_tcgen05_kernel<(m), 2>}}
+#define VKG_SPEC(m) {(m), gemm_tcgen05_kernel<(m)>}
 // The epilogues the training step uses; anything else runs the generic kernel.
 const Specialised kSpecialised[] = {
     VKG_SPEC(0),                                   // fp32 out: dW, dX into layernorm, scores
@@ -1135,7 +1137,7 @@ const Specialised kSpecialised[] = {
     VKG_SPEC(E_GENERIC),                           // last: whatever is not above
 };
 const int kNumSpecialised = sizeof(kSpecialised) / sizeof(kSpecialised[0]);
-#define VKG_SPEC_CP(m) {(m), {gemm_cta_pair_kernel<(m), 1>, gemm_cta_pair_kernel<(m), 2>}}
+#define VKG_SPEC_CP(m) {(m), gemm_cta_pair_kernel<(m)>}
 // The same epilogues on 256 x 256 tiles computed by CTA pairs.
 const Specialised kCtaPair[] = {
     VKG_SPEC_CP(0),
@@ -1150,10 +1152,10 @@ const Specialised kCtaPair[] = {
     VKG_SPEC_CP(E_GENERIC),
 };
 const int kNumCtaPair = sizeof(kCtaPair) / sizeof(kCtaPair[0]);
-GemmKernel pick(const Specialised* t, int n, int mode, int stage_kb) {
+GemmKernel pick(const Specialised* t, int n, int mode) {
   int i = 0;
   while (i + 1 < n && t[i].mode != mode) ++i;
-  return t[i].fn[stage_kb - 1];
+  return t[i].fn;
 }
 typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*,
                                   const cuuint64_t*, const cuuint64_t*, const cuuint32_t*,
@@ -1230,9 +1232,11 @@ int make_out_map(vkg_device* dev, CUtensorMap* map, const void* ptr, int dtype, 
 // tiles of a CTA pair, 64 to 256 columns wide.  How many slices K is cut into is not the model's to
 // choose (k_slices): it is part of the result.  Its constants were fitted to 208 shapes (M to 50272,
 // N and K alike, aligned and ragged, the three transpositions, every epilogue of a training step;
-// launches in a graph on B200, operands warm).  Over 180 others (drawn M, N, K up to 16384, and the
-// GEMMs of eight models) the choice takes 0.4 % longer than the best candidate on average, 14 % at
-// worst and more than 5 % for four.
+// launches in a graph on B200, operands warm) when a k-block of a narrow tile still took a load and a wait
+// of its own; since then they are too high there, by a quarter, but the order they give stands: over
+// 380 drawn shapes the choice takes 0.4 % longer than the best candidate on average, more than 5 % for nine.
+// Constants fitted anew, 10 % off the times instead of 18 %, chose no better (0.3 % on shapes held out; a block
+// run through the op dictionaries 261 us against 259).
 //
 // Per k-block (64 of K), microseconds by tile width 64 / 128 / 192 / 256.  A CTA pulls its operands
 // through an L2 port of 64 bytes a cycle; K-major operands go a little faster than MN-major ones.
@@ -1552,9 +1556,9 @@ int ensure_attrs(vkg_device* dev) {
               "gemm needs %d bytes of shared memory, device offers %zu", SMEM_BYTES,
               dev->gemm_smem_optin);
   for (const Specialised& k : kSpecialised)
-    for (GemmKernel fn : k.fn) VKG_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES));
+    VKG_CUDA(cudaFuncSetAttribute(k.fn, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES));
   for (const Specialised& k : kCtaPair)
-    for (GemmKernel fn : k.fn) VKG_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES));
+    VKG_CUDA(cudaFuncSetAttribute(k.fn, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES));
   dev->gemm_attr_set = true;
   return 0;
 }
@@ -1687,8 +1691,7 @@ extern "C" int vkg_gemm_group_launch(vkg_device* dev, const void* table, int n, 
   VKG_REQUIRE(table && n > 0 && n <= GROUP_MAX && total_units != 0, "gemm_group: bad arguments");
   if (ensure_attrs(dev)) return 1;
   if (!dev->group_attr_set) {
-    for (auto fn : {gemm_group_kernel<1>, gemm_group_kernel<2>})
-      VKG_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES));
+    VKG_CUDA(cudaFuncSetAttribute(gemm_group_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES));
     VKG_CUDA(cudaFuncSetAttribute(gemm_group_pair_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                   SMEM_BYTES));
     dev->group_attr_set = true;
@@ -1705,7 +1708,7 @@ extern "C" int vkg_gemm_group_launch(vkg_device* dev, const void* table, int n, 
   total_units &= (1 << GROUP_BN_SHIFT) - 1;
   int ctas = vkg_persistent_ctas(dev) < total_units ? vkg_persistent_ctas(dev) : total_units;
   VKG_CUDA(vkg_launch(dev, VKG_K_GEMM_GROUP | vkg_short_if(total_units <= ctas),
-                      single_stage_kb(bn) == 2 ? gemm_group_kernel<2> : gemm_group_kernel<1>,
+                      gemm_group_kernel,
                       dim3((unsigned)ctas), dim3(NUM_THREADS), SMEM_BYTES, 1,
                       static_cast<const GroupEntry*>(table), n, total_units, bn));
   return vkg_check_launch("gemm_group_kernel");
@@ -1743,7 +1746,7 @@ int make_plan(vkg_device* dev, const vkg_gemm_args* a, GemmPlan* out) {
   const bool use_pair = t.pair;
   if (build_problem(dev, a, &q, use_pair, t.bn, t.split)) return 1;
   if (use_pair) {
-    out->fn = pick(kCtaPair, kNumCtaPair, q.mode, q.p.stage_kb);
+    out->fn = pick(kCtaPair, kNumCtaPair, q.mode);
     long long pairs = vkg_persistent_ctas(dev) / 2;
     if (pairs > q.total_tiles) pairs = q.total_tiles;
     out->family = VKG_K_GEMM_PAIR;
@@ -1751,7 +1754,7 @@ int make_plan(vkg_device* dev, const vkg_gemm_args* a, GemmPlan* out) {
     out->cluster = 2;
     out->tile_rows = 2 * BM;
   } else {
-    out->fn = pick(kSpecialised, kNumSpecialised, q.mode, q.p.stage_kb);
+    out->fn = pick(kSpecialised, kNumSpecialised, q.mode);
     long long ctas = a->max_ctas > 0 ? a->max_ctas : vkg_persistent_ctas(dev);
     if (ctas > q.total_tiles) ctas = q.total_tiles;
     out->family = VKG_K_GEMM;
