@@ -800,8 +800,8 @@ constexpr int KV_K = 0,                                        // two buffers of
               KV_BAR = KV_TILES + SEG_ITEMS * 4, KV_SMEM = KV_BAR + 256 + 1024;
 static_assert(KV_SMEM <= 227 * 1024, "dK / dV kernel: shared memory");
 constexpr int KV_KV_FULL = 0, KV_KV_FREE = 2, KV_SDP_FULL = 4, KV_SDP_FREE = 5, KV_PDS_FULL = 6, KV_PDS_FREE = 7,
-              KV_OUT_FULL = 8, KV_ACC_FREE = 9, KV_QD_FULL = 10, KV_QD_EMPTY = 10 + KV_STAGES,
-              KV_NBAR = 10 + 2 * KV_STAGES;
+              KV_OUT_FULL = 8, KV_ACC_FREE = 10, KV_QD_FULL = 11, KV_QD_EMPTY = 11 + KV_STAGES,
+              KV_NBAR = 11 + 2 * KV_STAGES;
 
 // P and dS = P (dP - delta) scale of one key row against 16 queries, as fp16 pairs (queries 2i, 2i + 1)
 // in pp[i] and pd[i], ready for tcgen05.st.  P is rebuilt from the saved log-sum-exp; stat holds
@@ -1001,7 +1001,7 @@ attn_bwd_kv_kernel(const __grid_constant__ CUtensorMap tm, const __grid_constant
           umma_f16_ts_chain<8>(tdK, tdS, qm_lo + so, 128, d_hi, idesc_g, it ? 1u : 0u);
           umma_commit_one(B_(KV_QD_EMPTY + s));   // Q / dO stage free
           umma_commit_one(B_(KV_PDS_FREE));       // P / dS may be overwritten
-          if (next >= ni) umma_commit_one(B_(KV_OUT_FULL));
+          if (next >= ni) umma_commit_one(B_(KV_OUT_FULL + (j & 1)));
           if (++s == KV_STAGES) s = 0;
         }
       }
@@ -1019,7 +1019,7 @@ attn_bwd_kv_kernel(const __grid_constant__ CUtensorMap tm, const __grid_constant
       if (snake_item(j + 1, G, (int)blockIdx.x) >= n_items) break;   // the last one: see the softmax warps
       const int kt = item / HB, hb = item % HB;
       const int h = hb % p.H, b = hb / p.H;
-      if (!mbar_wait_warp<SM_SPIN>(B_(KV_OUT_FULL), j & 1, abort_flag, p.err, 0x4800u)) break;
+      if (!mbar_wait_warp<SM_SPIN>(B_(KV_OUT_FULL + (j & 1)), (j >> 1) & 1, abort_flag, p.err, 0x4800u)) break;
       tcgen05_fence_after();
       stage_acc<8>(tdV + t_lane, stage, lane);
       stage_acc<8>(tdK + t_lane, stage + 4096, lane);
@@ -1131,7 +1131,15 @@ attn_bwd_kv_kernel(const __grid_constant__ CUtensorMap tm, const __grid_constant
     }
     // The CTA's last item (its only one in a small problem) has nothing to overlap with: all sixteen
     // warps read it out, 32 columns each (dV by parts 0 and 1, dK by 2 and 3), through the idle ring.
-    if (ok && last >= 0 && mbar_wait_warp<SM_SPIN>(B_(KV_OUT_FULL), last_j & 1, abort_flag, p.err, 0x4c00u)) {
+    // They have waited for no other item's KV_OUT_FULL, and a parity wait also passes while its barrier is
+    // a phase behind.  Hence a barrier for even items and one for odd ones: a phase behind is then item
+    // last_j - 2, whose barrier has completed.  The last wait for KV_PDS_FREE was for a step of the last
+    // item or of the one before it (every item has a step), the products of either came after those of
+    // item last_j - 1's first step, and these after KV_ACC_FREE of item last_j - 2, which its readers signal
+    // only once they have seen its KV_OUT_FULL.  With one barrier, a last item of one step could find the
+    // phase of item last_j - 1 still open: its KV_PDS_FREE and KV_OUT_FULL are two commits.
+    if (ok && last >= 0 &&
+        mbar_wait_warp<SM_SPIN>(B_(KV_OUT_FULL + (last_j & 1)), (last_j >> 1) & 1, abort_flag, p.err, 0x4c00u)) {
       tcgen05_fence_after();
       uint8_t* stage = gbase + KV_Q + (warp - BW_SM_WARP) * 2048;
       stage_acc<4>(tdV + t_lane + part * 32, stage, lane);
