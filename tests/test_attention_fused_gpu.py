@@ -57,6 +57,18 @@ def one_pass(dev):
     set_(0)
 
 
+@pytest.fixture
+def sm_limit(dev):
+    """Holds persistent kernels to that many CTAs for the test."""
+    from vkgrad_b200._lib import TUNE_SM_LIMIT
+    from vkgrad_b200.vk import _check
+
+    def set_(n):
+        _check(dev.lib.vkg_set_tuning(dev.handle, TUNE_SM_LIMIT, n), "tune")
+    yield set_
+    set_(0)
+
+
 @pytest.mark.parametrize("B,T,H", [(1, 128, 1), (2, 320, 2), (1, 1024, 3), (3, 72, 1)])
 @pytest.mark.parametrize("packed", [False, True])
 @pytest.mark.parametrize("kernel", ["two_pass", "one_pass", "one_pass_rescaled"])
@@ -154,6 +166,37 @@ def test_backward(dev, B, T, H, packed):
                           ("dv", dv, slice(2 * D, 3 * D))):
         assert relerr(got[:, sl], merge(ref)) < 3e-3, name
     for x in (bq, bdo, bo, bl, bdelta, bdq) + (() if bs is None else (bs,)):
+        x.destroy()
+
+
+# The partial column sums may start at any float of a larger buffer.  One CTA for six items: all but the
+# last are stored, and added up, by the epilogue warps.
+@pytest.mark.parametrize("first", [0, 1, 2, 3])
+def test_dbias_scratch_at_any_float(dev, sm_limit, first):
+    from vkgrad_b200.vk import _check
+    B, T, H = 1, 300, 2
+    D = H * 64
+    rng = np.random.default_rng(first)
+    qkv = rng.standard_normal((B * T, 3 * D)).astype(np.float16)
+    dout = (0.1 * rng.standard_normal((B * T, D))).astype(np.float16)
+    bq, bdo = up(dev, qkv), up(dev, dout)
+    bo, bdq = up(dev, np.zeros((B * T, D), np.float16)), up(dev, np.full((B * T, 3 * D), np.nan, np.float16))
+    bl, bdelta = (up(dev, np.zeros((B * H, T), np.float32)) for _ in range(2))
+    bdb = up(dev, np.full(3 * D, np.nan, np.float32))
+    n = dev.lib.vkg_attn_bwd_dbias_scratch_floats(B, T, H, 64)
+    bsc = up(dev, np.full(n + 8, np.nan, np.float32))
+    sm_limit(1)
+    _check(dev.lib.vkg_attn_fwd(dev.handle, bq.dptr, None, bo.dptr, bl.dptr, B, T, H, 64, 0.125), "attn_fwd")
+    _check(dev.lib.vkg_attn_bwd(dev.handle, bq.dptr, bdo.dptr, bo.dptr, bl.dptr, None, bdq.dptr, bdelta.dptr,
+                                bdb.dptr, bsc.dptr + 4 * first, B, T, H, 64, 0.125), "attn_bwd")
+    dev.sync()
+    want = get(bdq, np.float16, (B * T, 3 * D)).astype(np.float64).sum(0)
+    # fp32 sums of T values in a tree and 4 * 3 partial rows: far below 1e-5 of the largest
+    assert np.abs(get(bdb, np.float32, (3 * D,)) - want).max() <= 1e-5 * max(np.abs(want).max(), 1.0)
+    scratch = get(bsc, np.float32, (n + 8,))
+    assert np.isfinite(scratch[first:first + n]).all()
+    assert np.isnan(scratch[:first]).all() and np.isnan(scratch[first + n:]).all()
+    for x in (bq, bdo, bo, bdq, bl, bdelta, bdb, bsc):
         x.destroy()
 
 

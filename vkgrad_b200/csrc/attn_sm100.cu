@@ -771,8 +771,12 @@ __device__ __forceinline__ void store_staged(const uint8_t* stage, int lane, uin
   auto t4 = [&](int r) { return add(t8(r), t8(r + 4)); };
   auto t2 = [&](int r) { return add(t4(r), t4(r + 2)); };
   const float2 sum = add(t2(0), t2(1));
-  if (NU == 8) *reinterpret_cast<float2*>(sums + 2 * lane) = sum;
-  else sums[lane] = (lane & 1) ? sum.y : sum.x;
+  if (NU == 8) {                   // one by one: the caller's scratch need not start on 8 bytes
+    sums[2 * lane] = sum.x;
+    sums[2 * lane + 1] = sum.y;
+  } else {
+    sums[lane] = (lane & 1) ? sum.y : sum.x;
+  }
 }
 
 // Item number j of persistent CTA c out of G: rows of G items are dealt left to right and right
