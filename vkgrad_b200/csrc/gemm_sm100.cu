@@ -5,7 +5,7 @@
 // bias / activation / activation-derivative / residual / narrowing.
 //
 // One persistent CTA per SM, 576 threads:
-//   warp 0       TMA producer (one lane)
+//   warp 0       TMA producer (one lane; of a CTA pair: converged, one elected lane per stage)
 //   warp 1       TMEM allocation + MMA issue (converged, one elected lane per instruction)
 //   warps 2..17  epilogue; warp w reads TMEM lanes 32*(w%4) .. +31 and takes every
 //                fourth 16-column chunk.  The epilogue is instruction-issue / latency
@@ -494,14 +494,20 @@ struct Feed {
       x += 64;
       dst += step;
     }
+  }
+  __device__ __forceinline__ void next() {
     c0 += s0;
     c1 += s1;
     c2 += s2;
   }
 };
 
-// TMA producer (one lane) of a single CTA or of one CTA of a pair: stream the k-blocks of a work unit's
-// operands into the ring.  b_at: the CTA's first column of B.
+// TMA producer of a single CTA (one lane) or of one CTA of a pair (the whole warp): stream the k-blocks of a
+// work unit's operands into the ring.  b_at: the CTA's first column of B.
+// A load issued from a branch that only lane 0 takes has its operands moved from vector registers one by
+// one.  Where a k-block of a 256-column pair tile comes in four loads, that paces the tile (2544 x 1392 x 3640
+// TN: 26.4 us, 24.0 with an elected lane of a converged warp).  A single CTA's short tiles start 0.05 to 0.1 us
+// later that way (280 x 832 x 264: 7.08 -> 7.21), and gain nothing.
 template <bool PAIR>
 __device__ __forceinline__ bool produce(const CtaCtx& cx, const GemmParams& p, const CUtensorMap* tmA,
                                         const CUtensorMap* tmB, TileCoord tc, int b_at, uint32_t rank, Ring& at) {
@@ -511,18 +517,24 @@ __device__ __forceinline__ bool produce(const CtaCtx& cx, const GemmParams& p, c
   Feed a(p.a_mn, kb0, tc.m0, BM, p.stage_kb), b(p.b_mn, kb0, b_at, PAIR ? p.bn / 2 : p.bn, p.stage_kb);
   const uint32_t a_bytes = (uint32_t)p.stage_kb * A_STAGE_BYTES;
   for (int kb = 0; kb < nkb; kb += p.stage_kb) {
-    if (at.wrapped && !mbar_wait(cx.empty0 + 8 * at.stage, at.phase ^ 1u, cx.abort_flag, p.err, 0x100u + at.stage))
+    const uint32_t empty = cx.empty0 + 8 * at.stage, old = at.phase ^ 1u, where = 0x100u + at.stage;
+    if (at.wrapped && !(PAIR ? mbar_wait_warp(empty, old, cx.abort_flag, p.err, where)
+                             : mbar_wait(empty, old, cx.abort_flag, p.err, where)))
       return false;
     uint32_t fb = cx.full0 + 8 * at.stage;
     const uint32_t sa = cx.base + at.stage * cx.stage_bytes;
-    if (PAIR) {
-      if (rank == 0) mbar_expect_tx(fb, 2 * cx.stage_bytes);
-      fb = mapa_shared(fb, 0);
-    } else {
-      mbar_expect_tx(fb, cx.stage_bytes);
+    if (!PAIR || elect_one()) {
+      if (PAIR) {
+        if (rank == 0) mbar_expect_tx(fb, 2 * cx.stage_bytes);
+        fb = mapa_shared(fb, 0);
+      } else {
+        mbar_expect_tx(fb, cx.stage_bytes);
+      }
+      a.load<PAIR>(sa, tmA, fb, tc);
+      b.load<PAIR>(sa + a_bytes, tmB, fb, tc);
     }
-    a.load<PAIR>(sa, tmA, fb, tc);
-    b.load<PAIR>(sa + a_bytes, tmB, fb, tc);
+    a.next();
+    b.next();
     at.step(cx.n_stages);
   }
   return true;
@@ -1023,12 +1035,10 @@ gemm_cta_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
   const int n_pairs = (int)gridDim.x >> 1, pair = (int)blockIdx.x >> 1;
   const int total_tiles = p.tiles_m * p.tiles_n * p.nb0 * (p.split_k > 1 ? p.split_k : p.nb1);
   if (warp == 0) {
-    if (lane == 0) {
-      Ring at;
-      for (int t = pair; t < total_tiles; t += n_pairs) {
-        const TileCoord tc = pair_coord(p, t, rank);
-        if (!produce<true>(cx, p, &tmA, &tmB, tc, tc.n0 + (int)rank * (p.bn / 2), rank, at)) break;
-      }
+    Ring at;
+    for (int t = pair; t < total_tiles; t += n_pairs) {
+      const TileCoord tc = pair_coord(p, t, rank);
+      if (!produce<true>(cx, p, &tmA, &tmB, tc, tc.n0 + (int)rank * (p.bn / 2), rank, at)) break;
     }
   } else if (warp == 1) {
     if (rank == 0) {
@@ -1063,14 +1073,12 @@ gemm_group_pair_kernel(const GroupEntry* __restrict__ table, int n_problems, int
   pdl_wait();
   const int n_pairs = (int)gridDim.x >> 1, pair = (int)blockIdx.x >> 1;
   if (warp == 0) {
-    if (lane == 0) {
-      Ring at;
-      for (int u = pair; u < total_units; u += n_pairs) {
-        const int pi = group_find(first, n_problems, u);
-        const GemmParams p = table[pi].p;
-        const TileCoord tc = pair_coord(p, u - first[pi], rank);
-        if (!produce<true>(cx, p, &table[pi].tmA, &table[pi].tmB, tc, tc.n0 + (int)rank * (p.bn / 2), rank, at)) break;
-      }
+    Ring at;
+    for (int u = pair; u < total_units; u += n_pairs) {
+      const int pi = group_find(first, n_problems, u);
+      const GemmParams p = table[pi].p;
+      const TileCoord tc = pair_coord(p, u - first[pi], rank);
+      if (!produce<true>(cx, p, &table[pi].tmA, &table[pi].tmB, tc, tc.n0 + (int)rank * (p.bn / 2), rank, at)) break;
     }
   } else if (warp == 1) {
     if (rank == 0) {
