@@ -463,11 +463,11 @@ struct Ring {
 // time but the instructions around them: 115 cycles for a wait, 50 to 100 for each load, in the loop of
 // the warp that loads and again in the loop of the warp that multiplies.  With one k-block to a stage
 // and a load for every 64 columns both loops took 383 (NT) to 490 (TN) cycles where the tensor core needs
-// 192.  So a stage holds two k-blocks wherever that leaves three stages, and an operand whose
+// 192.  So a stage may hold two k-blocks (stage_kb_for), and an operand whose
 // contiguous dimension is whole 64-element pieces is wide: its map splits that dimension in two, and one
 // load brings the stage's pieces, each a tile of its own ([k-block][row][64] of a K-major operand,
 // [64 columns][k][64] of an MN-major one).  Others take a load per piece, into the same places.
-// 1024 x 768 x 3072 (NN, residual): 15.4 -> 11.9 us, 768 x 2304 x 1024 (TN) 9.1 -> 7.6.
+// 1024 x 768 x 3072 (NN, residual): 15.4 -> 11.7 us, 768 x 2304 x 1024 (TN) 9.1 -> 7.6.
 struct Feed {
   int c0, c1, c2;        // map coordinates; a load per piece moves c0 on by 64
   int s0, s1, s2;        // their step per stage
@@ -517,10 +517,15 @@ __device__ __forceinline__ bool produce(const CtaCtx& cx, const GemmParams& p, c
   Feed a(p.a_mn, kb0, tc.m0, BM, p.stage_kb), b(p.b_mn, kb0, b_at, PAIR ? p.bn / 2 : p.bn, p.stage_kb);
   const uint32_t a_bytes = (uint32_t)p.stage_kb * A_STAGE_BYTES;
   for (int kb = 0; kb < nkb; kb += p.stage_kb) {
-    const uint32_t empty = cx.empty0 + 8 * at.stage, old = at.phase ^ 1u, where = 0x100u + at.stage;
-    if (at.wrapped && !(PAIR ? mbar_wait_warp(empty, old, cx.abort_flag, p.err, where)
-                             : mbar_wait(empty, old, cx.abort_flag, p.err, where)))
-      return false;
+    // (one expression for both kinds of wait made a single CTA's launches 0.03 us longer)
+    if (PAIR) {
+      if (at.wrapped &&
+          !mbar_wait_warp(cx.empty0 + 8 * at.stage, at.phase ^ 1u, cx.abort_flag, p.err, 0x100u + at.stage))
+        return false;
+    } else {
+      if (at.wrapped && !mbar_wait(cx.empty0 + 8 * at.stage, at.phase ^ 1u, cx.abort_flag, p.err, 0x100u + at.stage))
+        return false;
+    }
     uint32_t fb = cx.full0 + 8 * at.stage;
     const uint32_t sa = cx.base + at.stage * cx.stage_bytes;
     if (!PAIR || elect_one()) {
@@ -1444,10 +1449,34 @@ int check_args(const vkg_gemm_args* a) {
 }
 
 // Two k-blocks to a stage where that leaves three stages (the 192-wide pair tile does too).
-int single_stage_kb(int bn) { return RING_BYTES / (2 * (A_STAGE_BYTES + bn * 128)) >= 3 ? 2 : 1; }
+int most_stage_kb(bool pair, int bn) {
+  return pair ? (bn == PAIR_BN ? 1 : 2) : RING_BYTES / (2 * (A_STAGE_BYTES + bn * 128)) >= 3 ? 2 : 1;
+}
 
-// use_pair: 256 x bn tiles for gemm_cta_pair_kernel (the caller has checked the shape).
-int build_problem(vkg_device* dev, const vkg_gemm_args* a, Problem* out, bool use_pair, int bn, int want_split) {
+// Whether a launch takes them: kbs k-blocks to a work unit, operands wide (Feed) or in pieces.  Two save a wait
+// and, of all but K-major operands in pieces, loads; but the first products wait for both, 0.1 us later.
+// Against a start with one k-block to a stage, 88 drawn shapes in three transpositions:
+//   - one k-block to a unit: the second is loaded for nothing (2822 x 64 x 400 NN 4.35 us, with two 4.70);
+//   - all in pieces, both K-major: two save no load (1545 x 80 x 264 NT 3.90, with two 4.02);
+//   - all in pieces, single tiles: of the loads saved a tile of 64 columns sees little (837 x 280 x 264 NN 4.92,
+//     with two 5.01; 280 x 832 x 264 TN 7.04, 7.14), wider MN-major ones do, and pairs (1760 x 3304 x 1904 TN
+//     24.2, with two 19.9);
+//   - one in pieces: two pay from five k-blocks on (915 x 736 x 128 NN 5.67, with two 5.34), where a K-major one
+//     is, else from four (248 x 168 x 1344 TN, three: 4.17, with two 4.42).
+// Where the kernel of before those loads was faster (4.53, 3.88, 4.88, 6.99 and 4.18 above) that leaves 0.02 us.
+int stage_kb_for(const vkg_gemm_args* a, bool pair, int bn, int kbs, bool a_wide, bool b_wide) {
+  if (most_stage_kb(pair, bn) == 1 || kbs <= 1) return 1;
+  if (a_wide && b_wide) return 2;
+  const bool k_pieces = (!a->trans_a && !a_wide) || (a->trans_b && !b_wide);
+  if (a_wide || b_wide) return kbs <= (k_pieces ? 4 : 3) ? 1 : 2;
+  if (!a->trans_a && a->trans_b) return 1;
+  return !pair && (k_pieces || bn == 64) ? 1 : 2;
+}
+
+// use_pair: 256 x bn tiles for gemm_cta_pair_kernel (the caller has checked the shape).  grouped: the ring is
+// shared with other problems.
+int build_problem(vkg_device* dev, const vkg_gemm_args* a, Problem* out, bool use_pair, int bn, int want_split,
+                  bool grouped = false) {
   if (check_args(a)) return 1;
   const int nb0 = a->nb0 > 0 ? a->nb0 : 1, nb1 = a->nb1 > 0 ? a->nb1 : 1;
   const int batch = nb0 * nb1;
@@ -1461,10 +1490,11 @@ int build_problem(vkg_device* dev, const vkg_gemm_args* a, Problem* out, bool us
   p.tiles_n = (a->N + bn - 1) / bn;
   p.bn = bn;
   p.num_kb = (a->K + BK - 1) / BK;
-  p.stage_kb = use_pair ? (bn == PAIR_BN ? 1 : 2) : single_stage_kb(bn);
   const int rows_b = use_pair ? bn / 2 : bn, b_groups = (rows_b + 63) / 64;
   const bool a_wide = (a->trans_a ? a->M : a->K) % 64 == 0;
   const bool b_wide = (a->trans_b ? a->K : a->N) % 64 == 0 && (a->trans_b || rows_b % 64 == 0);
+  const int kbs = want_split > 1 ? (p.num_kb + want_split - 1) / want_split : p.num_kb;
+  p.stage_kb = grouped ? most_stage_kb(use_pair, bn) : stage_kb_for(a, use_pair, bn, kbs, a_wide, b_wide);
   p.a_mn = (a->trans_a ? OP_MN : 0) | (a_wide ? OP_WIDE : 0);
   p.b_mn = (a->trans_b ? 0 : OP_MN) | (b_wide ? OP_WIDE : 0);
   const uint32_t fmt = a->in_dtype == VKG_BF16 ? 1u : 0u;
@@ -1676,7 +1706,7 @@ extern "C" int vkg_gemm_group_prepare(vkg_device* dev, const vkg_gemm_args* args
     one.workspace = nullptr;
     one.workspace_bytes = 0;
     Problem q;
-    if (build_problem(dev, &one, &q, use_pair, tiles.bn, 1)) return 1;
+    if (build_problem(dev, &one, &q, use_pair, tiles.bn, 1, true)) return 1;
     VKG_REQUIRE(q.mode == 0, "gemm_group: problem %d needs 16-byte aligned rows", i);
     memset(&host[i], 0, sizeof(GroupEntry));
     host[i].tmA = q.tmA;
