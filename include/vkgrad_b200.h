@@ -362,6 +362,11 @@ int vkg_attn_bwd(vkg_device* dev, const void* qkv16, const void* dout16,
                  void* dqkv16, float* delta, float* dbias, float* dbias_scratch,
                  int B, int T, int H, int hd, float scale);
 int64_t vkg_attn_bwd_dbias_scratch_floats(int B, int T, int H, int hd);
+/* No reference counterpart, no device needed: vkg_attn_bwd's check, before its first launch, of the
+ * registers a thread that its kernels were compiled to.  Their warps share the block's registers out;
+ * one that asks for more than the block was launched with would wait without a limit.  An error where
+ * per_thread is too few. */
+int vkg_selftest_attn_registers(int per_thread);
 /* split_qkv / merge_qkv_grad / merge_heads / split_heads (tkernels.py:195-300). */
 int vkg_split_qkv(vkg_device* dev, const float* qkv, const float* bias, void* q16,
                   void* k16, void* v16, int64_t n, int D, int T, int H, int hd);

@@ -125,6 +125,20 @@ def test_nobody_reads_an_item_that_is_not_finished(items):
     assert not wrong_reads(items, out_barriers())
 
 
+@pytest.mark.parametrize("registers", [0, 72, 79, 80, 85])
+def test_kernels_with_too_few_registers_are_refused(registers):
+    """The softmax warps ask for 96 registers of the 80 a thread that the block is launched with; that
+    request waits without a limit, so fewer must end in an error before the launch."""
+    from vkgrad_b200 import _lib
+    from vkgrad_b200.vk import VkError, _check
+    call = _lib.load().vkg_selftest_attn_registers(registers)
+    if registers >= 80:
+        assert call == 0
+    else:
+        with pytest.raises(VkError, match=f"launched with {registers} registers"):
+            _check(call, "attn_bwd")
+
+
 def test_one_barrier_for_all_items_would_be_read_a_phase_early():
     """What the model is for: the last item of one step, with the item before it not signalled yet."""
     assert wrong_reads([2, 1], 1) and not wrong_reads([2, 1], 2)

@@ -118,6 +118,7 @@ _SIGNATURES = {
     "vkg_attn_fwd": (i32, [vp, vp, vp, vp, vp, i32, i32, i32, i32, f32]),
     "vkg_attn_bwd": (i32, [vp, vp, vp, vp, vp, vp, vp, vp, vp, vp, i32, i32, i32, i32, f32]),
     "vkg_attn_bwd_dbias_scratch_floats": (i64, [i32, i32, i32, i32]),
+    "vkg_selftest_attn_registers": (i32, [i32]),
     "vkg_split_qkv": (i32, [vp, vp, vp, vp, vp, vp, i64, i32, i32, i32, i32]),
     "vkg_merge_qkv_grad": (i32, [vp, vp, vp, vp, vp, i64, i32, i32, i32, i32]),
     "vkg_merge_heads": (i32, [vp, vp, vp, i64, i32, i32, i32, i32]),

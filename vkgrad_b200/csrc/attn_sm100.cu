@@ -27,8 +27,9 @@
 // same relative rounding per product and one division less per score.  The backward kernels
 // rebuild the normalised P from the saved log-sum-exp and round that, as the reference does
 // (tkernels.py:123, 183); O, dQ, dK, dV are stored fp16 as there (tkernels.py:284, 228-230).
-// Every wait is bounded (see tcgen05.cuh); a wait that gives up flags the error word,
-// all roles leave their loops, TMEM is freed and the CTA returns.
+// Every wait on a barrier is bounded (see tcgen05.cuh); a wait that gives up flags the error word,
+// all roles leave their loops, TMEM is freed and the CTA returns.  The backward's request for registers
+// has no limit; the host makes sure that it can be met.
 #include "common.cuh"
 #include "tcgen05.cuh"
 
@@ -702,12 +703,16 @@ attn_fwd1_kernel(const __grid_constant__ CUtensorMap tm, const AttnParams p) {
 // item ends.  Before (single buffers, accumulators read out and delta formed by the softmax warps) an
 // item boundary cost 5000 cycles, 16 to 18 us of each kernel's 50 at 8 x 1024 tokens, 12 heads.
 // Registers: 768 threads are launched with 80 each; the softmax warps, which hold 64 scores and
-// gradients at a time, take 96 of what the other eight warps give back.
+// gradients at a time, take 96 of what the other eight warps give back.  That request is the one wait
+// without a limit: with fewer registers at launch it would never be met, so the host compares the split
+// with what the kernels were compiled to before it launches them (bwd_registers).
 constexpr int BW_EPI_WARP = 4, BW_EPI_WARPS = 4, BW_SM_WARP = 8, BW_SM_WARPS = 16;
 constexpr int BW_THREADS = (BW_SM_WARP + BW_SM_WARPS) * 32;
 constexpr int BW_REGS_ISSUE = 40, BW_REGS_EPI = 56, BW_REGS_SM = 96;
-static_assert(4 * (BW_REGS_ISSUE + BW_REGS_EPI) + BW_SM_WARPS * BW_REGS_SM <= (BW_SM_WARP + BW_SM_WARPS) * 80,
-              "a split above what the block was launched with would wait forever");
+constexpr int BW_REGS_SPLIT = BW_EPI_WARP * BW_REGS_ISSUE + BW_EPI_WARPS * BW_REGS_EPI + BW_SM_WARPS * BW_REGS_SM;
+constexpr int BW_REGS_LAUNCH = BW_REGS_SPLIT / (BW_SM_WARP + BW_SM_WARPS);      // a thread's share
+static_assert(BW_REGS_LAUNCH * (BW_SM_WARP + BW_SM_WARPS) == BW_REGS_SPLIT && BW_REGS_LAUNCH == 80,
+              "the split is 80 registers a thread, which 768 threads leave room for");
 
 template <int N>
 __device__ __forceinline__ void regs_less() {
@@ -1581,7 +1586,26 @@ int make_map_2d(vkg_device* dev, CUtensorMap* map, const void* ptr, int64_t cols
   return 0;
 }
 
+// Refuses a backward kernel that was compiled to fewer registers a thread than its warps share out.
+int bwd_registers(int per_thread) {
+  VKG_REQUIRE(per_thread >= BW_REGS_LAUNCH,
+              "attn_bwd: the kernels are launched with %d registers a thread, their warps' shares need %d",
+              per_thread, BW_REGS_LAUNCH);
+  return 0;
+}
+
+template <typename Kernel>
+int bwd_prepare(Kernel fn, int smem) {
+  cudaFuncAttributes attr;
+  VKG_CUDA(cudaFuncGetAttributes(&attr, fn));
+  if (bwd_registers(attr.numRegs)) return 1;
+  VKG_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+  return 0;
+}
+
 }  // namespace
+
+extern "C" int vkg_selftest_attn_registers(int per_thread) { return bwd_registers(per_thread); }
 
 extern "C" int vkg_attn_fwd(vkg_device* dev, const void* qkv16, const uint32_t* seg, void* out16,
                             float* lse2, int B, int T, int H, int hd, float scale) {
@@ -1649,9 +1673,9 @@ extern "C" int vkg_attn_bwd(vkg_device* dev, const void* qkv16, const void* dout
   p.colsum = dbias ? dbias_scratch : nullptr;
   if (!dev->attn_bwd_attr_set) {
     for (auto fn : {attn_bwd_kv_kernel<false>, attn_bwd_kv_kernel<true>})
-      VKG_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, KV_SMEM));
+      if (bwd_prepare(fn, KV_SMEM)) return 1;
     for (auto fn : {attn_bwd_q_kernel<false>, attn_bwd_q_kernel<true>})
-      VKG_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, DQ_SMEM));
+      if (bwd_prepare(fn, DQ_SMEM)) return 1;
     dev->attn_bwd_attr_set = true;
   }
   VKG_REQUIRE((((uintptr_t)dout16 | (uintptr_t)out16) & 15) == 0, "attn_bwd: dO and O must be 16-byte aligned");
