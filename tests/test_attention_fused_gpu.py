@@ -54,7 +54,7 @@ def one_pass(dev):
     def set_(on):
         _check(dev.lib.vkg_set_tuning(dev.handle, TUNE_ATTN_ONE_PASS, int(on)), "tune")
     yield set_
-    set_(0)
+    set_(1)
 
 
 @pytest.fixture
@@ -203,33 +203,34 @@ def test_dbias_scratch_at_any_float(dev, sm_limit, first):
 # Packed batches pass over tiles that lie before every row's sample: the edges of that rule are tiles with
 # one row left over, starts on tile borders, and starts in no order at all (nothing sorts them).  The
 # last case gives a CTA several items.
-@pytest.mark.parametrize("B,T,H", [(3, 513, 2), (2, 1000, 8), (1, 385, 60)])
-@pytest.mark.parametrize("starts", ["samples", "tiles", "unordered"])
-def test_packed_tiles(dev, B, T, H, starts):
-    from vkgrad_b200._lib import TUNE_ATTN_ONE_PASS
-    from vkgrad_b200.vk import _check
-    hd, D = 64, H * 64
-    rng = np.random.default_rng(T + H)
+def packed_starts(starts, B, T, rng):
     t = np.arange(T)
     if starts == "samples":
         cut = np.sort(rng.integers(0, T, (B, T // 60)), axis=1)
         cut[:, 0] = 0
-        seg = np.stack([c[np.searchsorted(c, t, side="right") - 1] for c in cut])
-    elif starts == "tiles":
-        seg = np.tile(t // 128 * 128, (B, 1))
-    else:
-        seg = rng.integers(0, t + 1, (B, T))
-    seg = seg.astype(np.uint32)
+        return np.stack([c[np.searchsorted(c, t, side="right") - 1] for c in cut]).astype(np.uint32)
+    if starts == "tiles":
+        return np.tile(t // 128 * 128, (B, 1)).astype(np.uint32)
+    return rng.integers(0, t + 1, (B, T)).astype(np.uint32)
+
+
+def check_packed(dev, B, T, H, seg, rng):
+    """Forward, gradients and their column sums of a packed batch against numpy."""
+    from vkgrad_b200._lib import TUNE_ATTN_ONE_PASS
+    from vkgrad_b200.vk import _check
+    hd, D = 64, H * 64
     qkv = rng.standard_normal((B * T, 3 * D)).astype(np.float16)
     dout = (0.1 * rng.standard_normal((B * T, D))).astype(np.float16)
     scale = 1.0 / np.sqrt(hd)
     bq, bdo, bs = up(dev, qkv), up(dev, dout), up(dev, seg)
     bo, bdq = up(dev, np.full((B * T, D), np.nan, np.float16)), up(dev, np.full((B * T, 3 * D), np.nan, np.float16))
     bl, bdelta = (up(dev, np.zeros((B * H, T), np.float32)) for _ in range(2))
+    bdb = up(dev, np.full(3 * D, np.nan, np.float32))
+    bsc = dev.buffer(4 * dev.lib.vkg_attn_bwd_dbias_scratch_floats(B, T, H, hd), "device")
     _check(dev.lib.vkg_set_tuning(dev.handle, TUNE_ATTN_ONE_PASS, 1), "tune")
     _check(dev.lib.vkg_attn_fwd(dev.handle, bq.dptr, bs.dptr, bo.dptr, bl.dptr, B, T, H, hd, scale), "attn_fwd")
     _check(dev.lib.vkg_attn_bwd(dev.handle, bq.dptr, bdo.dptr, bo.dptr, bl.dptr, bs.dptr, bdq.dptr, bdelta.dptr,
-                                None, None, B, T, H, hd, scale), "attn_bwd")
+                                bdb.dptr, bsc.dptr, B, T, H, hd, scale), "attn_bwd")
     dev.sync()
     q, k, v, p, o, lse2, _ = reference_attention(qkv, B, T, H, scale, seg)
     assert relerr(get(bo, np.float16, (B * T, D)).astype(np.float32), o) < 2e-3
@@ -241,5 +242,25 @@ def test_packed_tiles(dev, B, T, H, starts):
     merge = lambda x: x.transpose(0, 2, 1, 3).reshape(B * T, D)
     for i, ref in enumerate((ds @ k, ds.transpose(0, 1, 3, 2) @ q, p.transpose(0, 1, 3, 2) @ dao)):
         assert relerr(got[:, i * D:(i + 1) * D], merge(ref)) < 3e-3, "qkv"[i]
-    for x in (bq, bdo, bs, bo, bdq, bl, bdelta):
+    # the column sums of what is stored
+    want_db = got.astype(np.float64).sum(0)
+    assert np.abs(get(bdb, np.float32, (3 * D,)) - want_db).max() <= 1e-4 * max(np.abs(want_db).max(), 1.0)
+    for x in (bq, bdo, bs, bo, bdq, bl, bdelta, bdb, bsc):
         x.destroy()
+
+
+@pytest.mark.parametrize("B,T,H", [(3, 513, 2), (2, 1000, 8), (1, 385, 60)])
+@pytest.mark.parametrize("starts", ["samples", "tiles", "unordered"])
+def test_packed_tiles(dev, B, T, H, starts):
+    rng = np.random.default_rng(T + H)
+    check_packed(dev, B, T, H, packed_starts(starts, B, T, rng), rng)
+
+
+# Where passing over tiles ends: past a CTA's 64th item (80 and 160 of them on two CTAs and one), and past 32
+# tiles to a sequence (4096 tokens use every bit of an item's list, 4097 do without lists).
+@pytest.mark.parametrize("B,T,H,sms", [(2, 385, 20, 2), (2, 385, 20, 1), (1, 4096, 1, 0), (1, 4096, 3, 1), (1, 4097, 2, 0)])
+@pytest.mark.parametrize("starts", ["samples", "unordered"])
+def test_packed_limits(dev, sm_limit, B, T, H, sms, starts):
+    rng = np.random.default_rng(T + H)
+    sm_limit(sms)
+    check_packed(dev, B, T, H, packed_starts(starts, B, T, rng), rng)

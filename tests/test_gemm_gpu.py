@@ -2,6 +2,7 @@
 (test_kernels.py) against the golden fixture and the CPU oracle, plus ragged,
 batched and fused-epilogue cases the reference cannot express."""
 
+import ctypes
 import os
 import sys
 
@@ -565,21 +566,89 @@ def test_loads_of_every_tile(dev, m, n, k, split_k, ta, tb):
         x.destroy()
 
 
-def test_loads_of_a_group(dev):
+@pytest.mark.parametrize("bf16,batch,pad", [(True, (1, 1), 0), (False, (1, 1), 72), (False, (2, 3), 8), (True, (3, 1), 64)])
+@pytest.mark.parametrize("m,n,k", [(192, 192, 320), (264, 136, 200)])      # every operand wide, none
+@pytest.mark.parametrize("ta,tb", [(False, False), (False, True), (True, False), (True, True)])
+def test_loads_of_batches_and_pitched_rows(dev, ta, tb, m, n, k, bf16, batch, pad):
+    """The operands' five-dimensional maps: rows further apart than they are long, two batch strides and
+    both types, from every tile.  What lies between the rows is NaN."""
+    from vkgrad_b200._lib import BF16, F16
+    from vkgrad_b200.kernels import gemm
+    rng = np.random.default_rng(m + pad)
+    nb0, nb1 = batch
+
+    def make(rows, cols):
+        x = rng.standard_normal((nb1, nb0, rows, cols)).astype(np.float16).astype(np.float32)
+        if bf16:
+            x = (x.view(np.uint32) & 0xffff0000).view(np.float32)
+        full = np.full((nb1, nb0, rows, cols + pad), np.nan, np.float32)
+        full[..., :cols] = x
+        return x, up(dev, (full.view(np.uint32) >> 16).astype(np.uint16) if bf16 else full.astype(np.float16))
+    a, ba = make(*((k, m) if ta else (m, k)))
+    b, bb = make(*((n, k) if tb else (k, n)))
+    lda, ldb = a.shape[-1] + pad, b.shape[-1] + pad
+    strides = dict(sa=(a.shape[2] * lda, nb0 * a.shape[2] * lda), sb=(b.shape[2] * ldb, nb0 * b.shape[2] * ldb),
+                   sc=(m * n, nb0 * m * n))
+    want = (a.swapaxes(2, 3) if ta else a).astype(np.float64) @ (b.swapaxes(2, 3) if tb else b).astype(np.float64)
+    first = None
+    for pair, tn in ((-1, 64), (-1, 128), (-1, 192), (-1, 256), (1, 192), (1, 256)):
+        bc = up(dev, np.full(want.shape, np.nan, np.float32))
+        gemm(dev, ba, bb, bc, m, n, k, trans_a=ta, trans_b=tb, nb0=nb0, nb1=nb1, lda=lda, ldb=ldb, **strides,
+             in_dtype=BF16 if bf16 else F16, split_k=1, cta_pair=pair, tile_n=tn)
+        got = down(dev, bc, np.float32, want.shape)
+        bc.destroy()
+        # fp32 sums of k exact products: k * 2^-24 of their magnitudes' sum at most, 5e-5 of the largest
+        assert relerr(got, want) < 5e-5
+        first = got if first is None else first
+        assert np.array_equal(first, got)
+    for x in (ba, bb):
+        x.destroy()
+
+
+@pytest.mark.parametrize("tn", [64, 128, 256])
+@pytest.mark.parametrize("t", [320, 328, 448])       # five, six and seven k-blocks; wide, in pieces, wide
+def test_loads_under_a_causal_limit(dev, t, tn):
+    """A triangular operand's k-blocks, clipped to an odd number here and there, two to a stage: mode 2 ends
+    the K range at the diagonal, mode 3 starts it there.  The triangle's other half is zero, as the modes ask."""
+    from vkgrad_b200.kernels import gemm
+    rng = np.random.default_rng(t)
+    p = np.tril(rng.standard_normal((t, t))).astype(np.float16)
+    v = rng.standard_normal((t, 64)).astype(np.float16)
+    bp, bv = up(dev, p), up(dev, v)
+    for mode, ta in ((2, False), (3, True)):
+        bc = up(dev, np.full((t, 64), np.nan, np.float32))
+        gemm(dev, bp, bv, bc, t, 64, t, trans_a=ta, causal=mode, split_k=1, cta_pair=-1, tile_n=tn)
+        assert relerr(down(dev, bc, np.float32, (t, 64)), orc.matmul16(p, v, ta, False)) < 5e-5
+        bc.destroy()
+    for x in (bp, bv):
+        x.destroy()
+
+
+@pytest.mark.parametrize("pair,k,sizes", [
+    (0, 328, [(128, 256), (200, 136), (64, 72), (320, 64)]),
+    (0, 328, [(1536, 2048), (1480, 1928), (136, 1024)]),       # 192 columns: one k-block to a stage
+    (1, 1096, [(1792, 2048), (1736, 1928), (136, 1024)]),
+])
+def test_loads_of_a_group(dev, pair, k, sizes):
     """Problems of one grouped launch whose operands are loaded differently share the ring."""
-    from vkgrad_b200.kernels import gemm_group
+    from vkgrad_b200._lib import GemmArgs
+    from vkgrad_b200.kernels import _gemm_args, gemm_group
     rng = np.random.default_rng(5)
-    k, sizes = 328, [(128, 256), (200, 136), (64, 72), (320, 64)]
     made, problems = [], []
     for m, n in sizes:
         x, dy = (rng.standard_normal((k, c)).astype(np.float16) for c in (m, n))
         bx, by, bc = up(dev, x), up(dev, dy), up(dev, np.full((m, n), np.nan, np.float32))
         made.append((x, dy, bx, by, bc, m, n))
         problems.append((bx, by, bc, m, n, k, dict(trans_a=True)))
-    for pair in (0, 1):
-        gemm_group(dev, problems, cta_pair=pair)
-        for x, dy, _, _, bc, m, n in made:
-            assert relerr(down(dev, bc, np.float32, (m, n)), orc.matmul16(x, dy, True, False)) < 5e-5
-    for _, _, bx, by, bc, _, _ in made:
+    # the tiles that the library chooses for this list are those the case is for
+    args = (GemmArgs * len(problems))(*[_gemm_args(dev, *p[:6], **dict(p[6], split_k=1)) for p in problems])
+    table, units = dev.buffer(dev.lib.vkg_gemm_group_table_bytes(len(problems)), "device"), ctypes.c_int32(0)
+    assert dev.lib.vkg_gemm_group_prepare(dev.handle, args, len(problems), table.dptr, pair, ctypes.byref(units)) == 0
+    table.destroy()
+    width = 64 * ((units.value >> 28) + 1)
+    assert units.value < 0 if pair else (width >= 192) == (sizes[0][0] > 1000), (units.value, width)
+    gemm_group(dev, problems, cta_pair=pair)
+    for x, dy, bx, by, bc, m, n in made:
+        assert relerr(down(dev, bc, np.float32, (m, n)), orc.matmul16(x, dy, True, False)) < 5e-5
         for t in (bx, by, bc):
             t.destroy()
