@@ -256,9 +256,10 @@ def test_packed_tiles(dev, B, T, H, starts):
     check_packed(dev, B, T, H, packed_starts(starts, B, T, rng), rng)
 
 
-# Where passing over tiles ends: past a CTA's 64th item (80 and 160 of them on two CTAs and one), and past 32
+# Where passing over tiles ends: past a CTA's 64th item (80 of them on each of two CTAs, 160 and 96 on one), and past 32
 # tiles to a sequence (4096 tokens use every bit of an item's list, 4097 do without lists).
-@pytest.mark.parametrize("B,T,H,sms", [(2, 385, 20, 2), (2, 385, 20, 1), (1, 4096, 1, 0), (1, 4096, 3, 1), (1, 4097, 2, 0)])
+@pytest.mark.parametrize("B,T,H,sms", [(2, 385, 20, 2), (2, 385, 20, 1), (1, 4096, 1, 0), (1, 4096, 3, 1),
+                                       (1, 4097, 2, 0)])
 @pytest.mark.parametrize("starts", ["samples", "unordered"])
 def test_packed_limits(dev, sm_limit, B, T, H, sms, starts):
     rng = np.random.default_rng(T + H)

@@ -566,7 +566,8 @@ def test_loads_of_every_tile(dev, m, n, k, split_k, ta, tb):
         x.destroy()
 
 
-@pytest.mark.parametrize("bf16,batch,pad", [(True, (1, 1), 0), (False, (1, 1), 72), (False, (2, 3), 8), (True, (3, 1), 64)])
+@pytest.mark.parametrize("bf16,batch,pad", [(True, (1, 1), 0), (False, (1, 1), 72), (False, (2, 3), 8),
+                                            (True, (3, 1), 64)])
 @pytest.mark.parametrize("m,n,k", [(192, 192, 320), (264, 136, 200)])      # every operand wide, none
 @pytest.mark.parametrize("ta,tb", [(False, False), (False, True), (True, False), (True, True)])
 def test_loads_of_batches_and_pitched_rows(dev, ta, tb, m, n, k, bf16, batch, pad):

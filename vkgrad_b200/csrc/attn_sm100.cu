@@ -1686,9 +1686,11 @@ extern "C" int vkg_attn_bwd(vkg_device* dev, const void* qkv16, const void* dout
   const int sms = vkg_persistent_ctas(dev);
   const unsigned ctas = (unsigned)(n_items < sms ? n_items : sms);
   const unsigned family = VKG_K_ATTN_BWD | vkg_short_if(n_items <= sms);
-  VKG_CUDA(vkg_launch(dev, family, seg ? attn_bwd_q_kernel<true> : attn_bwd_q_kernel<false>, dim3(ctas), dim3(BW_THREADS), DQ_SMEM, 1, tm, tmdo, tmo, p));
+  VKG_CUDA(vkg_launch(dev, family, seg ? attn_bwd_q_kernel<true> : attn_bwd_q_kernel<false>, dim3(ctas),
+                      dim3(BW_THREADS), DQ_SMEM, 1, tm, tmdo, tmo, p));
   if (vkg_check_launch("attn_bwd_q_kernel")) return 1;
-  VKG_CUDA(vkg_launch(dev, family, seg ? attn_bwd_kv_kernel<true> : attn_bwd_kv_kernel<false>, dim3(ctas), dim3(BW_THREADS), KV_SMEM, 1, tm, tmdo, p));
+  VKG_CUDA(vkg_launch(dev, family, seg ? attn_bwd_kv_kernel<true> : attn_bwd_kv_kernel<false>, dim3(ctas),
+                      dim3(BW_THREADS), KV_SMEM, 1, tm, tmdo, p));
   if (vkg_check_launch("attn_bwd_kv_kernel")) return 1;
   if (dbias)
     return vkg_launch_col_sum_final(dev, dbias_scratch, dbias, 3 * D, B * p.nqt * 4, 0);

@@ -75,12 +75,13 @@ struct GemmParams {
 
 enum : int { OP_MN = 1, OP_WIDE = 2 };
 
-// The ring of one CTA.  rows_b: its rows of a K-major B, or columns of an MN-major one, which are loaded
-// in whole groups of 64 (a 96-column half of a pair's tile loads two and uses one and a half).
+// The ring of one CTA.
 struct RingShape {
-  int rows_b, stage_bytes, stages;
+  int stage_bytes, stages;
   __host__ __device__ RingShape(bool pair, int bn, bool b_mn, int stage_kb) {
-    rows_b = pair ? bn / 2 : bn;
+    // rows of a K-major B, or columns of an MN-major one, which are loaded in whole groups of 64 (a 96-column
+    // half of a pair's tile loads two and uses one and a half)
+    const int rows_b = pair ? bn / 2 : bn;
     stage_bytes = stage_kb * (A_STAGE_BYTES + (b_mn ? (rows_b + 63) / 64 * 64 : rows_b) * 128);
     stages = RING_BYTES / stage_bytes < MAX_STAGES ? RING_BYTES / stage_bytes : MAX_STAGES;
   }
@@ -1185,7 +1186,8 @@ int make_map(vkg_device* dev, CUtensorMap* map, const void* ptr, int dtype, int6
   int64_t pitch = ld * 2;
   int64_t st0 = nb0 > 1 ? s0 * 2 : pitch * rows;
   int64_t st1 = nb1 > 1 ? s1 * 2 : (nb0 > 1 ? st0 * nb0 : pitch * rows);
-  cuuint64_t strides[4] = {(cuuint64_t)pitch, (cuuint64_t)(wide ? 128 : pitch * rows), (cuuint64_t)st0, (cuuint64_t)st1};
+  cuuint64_t strides[4] = {(cuuint64_t)pitch, (cuuint64_t)(wide ? 128 : pitch * rows), (cuuint64_t)st0,
+                           (cuuint64_t)st1};
   cuuint32_t box[5] = {64, (cuuint32_t)box_rows, (cuuint32_t)pieces, 1, 1};
   cuuint32_t estr[5] = {1, 1, 1, 1, 1};
   if (((uintptr_t)ptr & 15) || (pitch & 15) || (st0 & 15) || (st1 & 15)) {
@@ -1247,7 +1249,8 @@ int make_out_map(vkg_device* dev, CUtensorMap* map, const void* ptr, int dtype, 
 // N and K alike, aligned and ragged, the three transpositions, every epilogue of a training step;
 // launches in a graph on B200, operands warm) when a k-block of a narrow tile still took a load and a wait
 // of its own; since then they are too high there, by a quarter, but the order they give stands: over
-// 380 drawn shapes the choice takes 0.4 % longer than the best candidate on average, more than 5 % for nine.
+// 380 drawn shapes the choice takes 0.4 % longer than the best candidate on average, more than 5 % for nine,
+// 1.35 times as long at worst.
 // Constants fitted anew, 10 % off the times instead of 18 %, chose no better (0.3 % on shapes held out; a block
 // run through the op dictionaries 261 us against 259).
 //
@@ -1262,7 +1265,8 @@ constexpr KBlockCost KB_TN = {{0.245, 0.300, 0.335, 0.400}, {0.330, 0.375}};
 constexpr double PL_LAUNCH = 3.43;     // launch, set-up, first load, drain
 constexpr double PL_EPI = 0.69, PL_EPI_COL = 0.00658;   // epilogue of a tile, per column at fp32 out
 constexpr double PL_PAIR = 1.29;       // a pair's barriers and its later start
-constexpr double PL_SHORT_US = 12.0;   // a launch that overlaps its predecessor, whatever its waves
+// A launch that overlaps its predecessor, whatever its waves.  In this model's time: 9 to 10 us measured.
+constexpr double PL_SHORT_US = 12.0;
 constexpr double PL_IDLE = 0.81;       // k-block cost with one CTA busy, of that with all
 constexpr double PL_WAVE = 0.95;       // per further wave
 constexpr double PL_OVERLAP = 1.42;    // epilogue beside a main loop, of the epilogue alone
@@ -1745,8 +1749,7 @@ extern "C" int vkg_gemm_group_launch(vkg_device* dev, const void* table, int n, 
   const int bn = 64 * ((total_units >> GROUP_BN_SHIFT) + 1);
   total_units &= (1 << GROUP_BN_SHIFT) - 1;
   int ctas = vkg_persistent_ctas(dev) < total_units ? vkg_persistent_ctas(dev) : total_units;
-  VKG_CUDA(vkg_launch(dev, VKG_K_GEMM_GROUP | vkg_short_if(total_units <= ctas),
-                      gemm_group_kernel,
+  VKG_CUDA(vkg_launch(dev, VKG_K_GEMM_GROUP | vkg_short_if(total_units <= ctas), gemm_group_kernel,
                       dim3((unsigned)ctas), dim3(NUM_THREADS), SMEM_BYTES, 1,
                       static_cast<const GroupEntry*>(table), n, total_units, bn));
   return vkg_check_launch("gemm_group_kernel");
