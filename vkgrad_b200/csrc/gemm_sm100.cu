@@ -1463,18 +1463,20 @@ int most_stage_kb(bool pair, int bn) {
 //   - one k-block to a unit: the second is loaded for nothing (2822 x 64 x 400 NN 4.35 us, with two 4.70);
 //   - all in pieces, both K-major: two save no load (1545 x 80 x 264 NT 3.90, with two 4.02);
 //   - all in pieces, single tiles: of the loads saved a tile of 64 columns sees little (837 x 280 x 264 NN 4.92,
-//     with two 5.01; 280 x 832 x 264 TN 7.04, 7.14), wider MN-major ones do, and pairs (1760 x 3304 x 1904 TN
+//     with two 5.01; 264 x 1544 x 80 TN 6.03, 6.26), wider MN-major ones do, and pairs (1760 x 3304 x 1904 TN
 //     24.2, with two 19.9);
+//   - both only up to ten k-blocks to a unit: calls one at a time lose beyond (1058 x 816 x 848 NT, thirteen:
+//     7.78, with two 7.62; 600 x 1992 x 3336 NT 18.0, 17.4), though launches in a row gain up to 2 % there;
 //   - one in pieces: two pay from five k-blocks on (915 x 736 x 128 NN 5.67, with two 5.34), where a K-major one
 //     is, else from four (248 x 168 x 1344 TN, three: 4.17, with two 4.42).
-// Where the kernel of before those loads was faster (4.53, 3.88, 4.88, 6.99 and 4.18 above) that leaves 0.02 us.
+// The kernel of before those loads took 4.35, 3.88, 4.91, 5.98 and 24.2 us, 7.78, 17.6, 6.1 and 4.18.
 int stage_kb_for(const vkg_gemm_args* a, bool pair, int bn, int kbs, bool a_wide, bool b_wide) {
   if (most_stage_kb(pair, bn) == 1 || kbs <= 1) return 1;
   if (a_wide && b_wide) return 2;
   const bool k_pieces = (!a->trans_a && !a_wide) || (a->trans_b && !b_wide);
   if (a_wide || b_wide) return kbs <= (k_pieces ? 4 : 3) ? 1 : 2;
-  if (!a->trans_a && a->trans_b) return 1;
-  return !pair && (k_pieces || bn == 64) ? 1 : 2;
+  const bool saves_little = (!a->trans_a && a->trans_b) || (!pair && (k_pieces || bn == 64));
+  return saves_little && kbs <= 10 ? 1 : 2;
 }
 
 // use_pair: 256 x bn tiles for gemm_cta_pair_kernel (the caller has checked the shape).  grouped: the ring is
